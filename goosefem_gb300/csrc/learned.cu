@@ -4,7 +4,7 @@
 // scaled by their RMS, plus the nodal bulk and shear moduli), dilations 1, 2, 4, 1, ReLU after
 // the first three layers. Weights are BF16, biases and every accumulation FP32.
 //
-//  * training kernels (CUDA cores, FP32 accumulate): forward with stored activations, backward
+//  * training kernels (nn_train.cuh; CUDA cores, FP32): forward with stored activations, backward
 //    for the inputs and the weights (per-block partial sums reduced in a fixed order:
 //    deterministic), masked mean-squared error or energy-norm loss, Adam;
 //  * inference: the 32 -> 32 layers on the tensor cores (mma.sync m16n8k16 BF16, FP32
@@ -24,6 +24,7 @@
 
 #include "common.cuh"
 #include "ffpair.cuh"
+#include "nn_train.cuh"
 
 namespace gfgpu {
 namespace nn {
@@ -39,153 +40,6 @@ __host__ __device__ constexpr int w_off(int l)
 __host__ __device__ constexpr int b_off(int l) { return w_off(l) + 9 * cin_of(l) * cout_of(l); }
 constexpr int kParams = b_off(3) + 2;
 static_assert(kParams == 20258, "parameter count");
-
-__device__ __forceinline__ float to_f(float v) { return v; }
-__device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float(v); }
-template <class T>
-__device__ __forceinline__ T from_f(float v);
-template <>
-__device__ __forceinline__ float from_f<float>(float v) { return v; }
-template <>
-__device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-
-// ------------------------------------------------------------------ CUDA-core convolutions
-
-// y[p, co] = b[co] + sum_t sum_ci x[p + dil*off_t, ci] W[t, ci, co]   (zero padding)
-template <int CI, int CO, bool RELU, class TI, class TO>
-__global__ void __launch_bounds__(128)
-k_conv_fwd(const TI* __restrict__ X, const __nv_bfloat16* __restrict__ W,
-           const float* __restrict__ bias, int dil, int B, int H, int Wd, TO* __restrict__ Y)
-{
-    __shared__ float Ws[9 * CI * CO];
-    __shared__ float bs[CO];
-    for (int i = threadIdx.x; i < 9 * CI * CO; i += blockDim.x) Ws[i] = __bfloat162float(W[i]);
-    for (int i = threadIdx.x; i < CO; i += blockDim.x) bs[i] = bias[i];
-    __syncthreads();
-    int64_t npix = static_cast<int64_t>(B) * H * Wd;
-    GF_FOR(p, npix)
-    {
-        int x = static_cast<int>(p % Wd);
-        int y = static_cast<int>((p / Wd) % H);
-        int64_t img = p / (static_cast<int64_t>(H) * Wd);
-        float acc[CO];
-#pragma unroll
-        for (int c = 0; c < CO; ++c) acc[c] = bs[c];
-#pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            int yy = y + dil * (t / 3 - 1), xx = x + dil * (t % 3 - 1);
-            if (yy < 0 || yy >= H || xx < 0 || xx >= Wd) continue;
-            const TI* xp = X + ((img * H + yy) * Wd + xx) * CI;
-#pragma unroll 4
-            for (int ci = 0; ci < CI; ++ci) {
-                float xv = to_f(xp[ci]);
-                const float* w = Ws + (t * CI + ci) * CO;
-#pragma unroll
-                for (int c = 0; c < CO; ++c) acc[c] = fmaf(xv, w[c], acc[c]);
-            }
-        }
-        TO* yp = Y + p * CO;
-#pragma unroll
-        for (int c = 0; c < CO; ++c) yp[c] = from_f<TO>(RELU ? fmaxf(acc[c], 0.0f) : acc[c]);
-    }
-}
-
-// dX[p, ci] = (sum_t sum_co dY[p - dil*off_t, co] W[t, ci, co]) * (act[p, ci] > 0)
-template <int CI, int CO>
-__global__ void __launch_bounds__(128)
-k_conv_bwd_data(const float* __restrict__ dY, const __nv_bfloat16* __restrict__ W, int dil, int B,
-                int H, int Wd, const float* __restrict__ act, float* __restrict__ dX)
-{
-    __shared__ float Ws[9 * CI * CO];
-    for (int i = threadIdx.x; i < 9 * CI * CO; i += blockDim.x) Ws[i] = __bfloat162float(W[i]);
-    __syncthreads();
-    int64_t npix = static_cast<int64_t>(B) * H * Wd;
-    GF_FOR(p, npix)
-    {
-        int x = static_cast<int>(p % Wd);
-        int y = static_cast<int>((p / Wd) % H);
-        int64_t img = p / (static_cast<int64_t>(H) * Wd);
-        float acc[CI];
-#pragma unroll
-        for (int c = 0; c < CI; ++c) acc[c] = 0.0f;
-#pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            int yy = y - dil * (t / 3 - 1), xx = x - dil * (t % 3 - 1);
-            if (yy < 0 || yy >= H || xx < 0 || xx >= Wd) continue;
-            const float* gp = dY + ((img * H + yy) * Wd + xx) * CO;
-#pragma unroll 4
-            for (int co = 0; co < CO; ++co) {
-                float g = gp[co];
-#pragma unroll
-                for (int ci = 0; ci < CI; ++ci) acc[ci] = fmaf(g, Ws[(t * CI + ci) * CO + co], acc[ci]);
-            }
-        }
-        const float* ap = act + p * CI;
-        float* o = dX + p * CI;
-#pragma unroll
-        for (int ci = 0; ci < CI; ++ci) o[ci] = ap[ci] > 0.0f ? acc[ci] : 0.0f;
-    }
-}
-
-// Per-block partial sums of dW[t, ci, co] = sum_p x[p + dil*off_t, ci] dY[p, co] and
-// db[co] = sum_p dY[p, co] over the block's contiguous pixel range. Thread (t, ci) owns the CO
-// weights of its row; threads < CO also own one bias. partial: [gridDim.x][9*CI*CO + CO].
-template <int CI, int CO>
-__global__ void k_conv_bwd_weight(const float* __restrict__ X, const float* __restrict__ dY,
-                                  int dil, int B, int H, int Wd, float* __restrict__ partial)
-{
-    constexpr int TILE = 32;
-    __shared__ float gs[TILE][CO];
-    int64_t npix = static_cast<int64_t>(B) * H * Wd;
-    int64_t per = (npix + gridDim.x - 1) / gridDim.x;
-    int64_t p0 = blockIdx.x * per;
-    int64_t p1 = p0 + per < npix ? p0 + per : npix;
-    int row = threadIdx.x; // (t, ci)
-    int t = row / CI, ci = row % CI;
-    bool owner = row < 9 * CI;
-    int dy = dil * (t / 3 - 1), dx = dil * (t % 3 - 1);
-    float acc[CO];
-#pragma unroll
-    for (int c = 0; c < CO; ++c) acc[c] = 0.0f;
-    float bacc = 0.0f;
-    for (int64_t base = p0; base < p1; base += TILE) {
-        int n = p1 - base < TILE ? static_cast<int>(p1 - base) : TILE;
-        __syncthreads();
-        for (int i = threadIdx.x; i < n * CO; i += blockDim.x) gs[i / CO][i % CO] = dY[(base + i / CO) * CO + i % CO];
-        __syncthreads();
-        if (owner) {
-            for (int k = 0; k < n; ++k) {
-                int64_t p = base + k;
-                int x = static_cast<int>(p % Wd);
-                int y = static_cast<int>((p / Wd) % H);
-                int yy = y + dy, xx = x + dx;
-                if (yy < 0 || yy >= H || xx < 0 || xx >= Wd) continue;
-                int64_t img = p / (static_cast<int64_t>(H) * Wd);
-                float xv = X[((img * H + yy) * Wd + xx) * CI + ci];
-#pragma unroll
-                for (int c = 0; c < CO; ++c) acc[c] = fmaf(xv, gs[k][c], acc[c]);
-            }
-        }
-        if (threadIdx.x < CO)
-            for (int k = 0; k < n; ++k) bacc += gs[k][threadIdx.x];
-    }
-    float* out = partial + static_cast<int64_t>(blockIdx.x) * (9 * CI * CO + CO);
-    if (owner)
-#pragma unroll
-        for (int c = 0; c < CO; ++c) out[row * CO + c] = acc[c];
-    if (threadIdx.x < CO) out[9 * CI * CO + threadIdx.x] = bacc;
-}
-
-// out[i] = sum over blocks of partial[b][i], in block order (deterministic)
-__global__ void k_sum_partials(const float* __restrict__ partial, int nblk, int n,
-                               float* __restrict__ out)
-{
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float s = 0.0f;
-    for (int b = 0; b < nblk; ++b) s += partial[static_cast<int64_t>(b) * n + i];
-    out[i] = s;
-}
 
 // masked MSE over the crop interior [m, S-m)^2: dY = 2 (y - t) / N, per-block loss partials
 __global__ void k_mse(const float* __restrict__ Y, const float* __restrict__ T, int B, int S,
@@ -301,21 +155,36 @@ k_crop_energy(const float* __restrict__ Y, const float* __restrict__ T, const fl
     }
 }
 
-// loss = sum_b num_b / sum_b den_b (block, then crop order); scale = 1 / sum_b den_b
-__global__ void k_energy_reduce(const float* __restrict__ part, int B, int nblk,
-                                float* __restrict__ scale, float* __restrict__ loss)
+// loss = sum_b num_b / sum_b den_b (block, then crop order); scale = 1 / sum_b den_b. One block: a
+// thread per crop sums its blocks (independent loads), the first adds the crops. With one thread
+// for all of them the 2 x 64 x 32 loads took 114 us.
+__global__ void __launch_bounds__(256)
+k_energy_reduce(const float* __restrict__ part, int B, int nblk, float* __restrict__ scale,
+                float* __restrict__ loss)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ float2 sh[256];
     float sn = 0.0f, sd = 0.0f;
-    for (int b = 0; b < B; ++b) {
-        float cn = 0.0f, cd = 0.0f;
-        for (int k = 0; k < nblk; ++k) {
-            cn += part[(static_cast<int64_t>(b) * nblk + k) * 2];
-            cd += part[(static_cast<int64_t>(b) * nblk + k) * 2 + 1];
+    for (int b0 = 0; b0 < B; b0 += 256) {
+        const int b = b0 + threadIdx.x;
+        if (b < B) {
+            const float* p = part + static_cast<int64_t>(b) * nblk * 2;
+            float cn = 0.0f, cd = 0.0f;
+#pragma unroll 16
+            for (int k = 0; k < nblk; ++k) {
+                cn += p[2 * k];
+                cd += p[2 * k + 1];
+            }
+            sh[threadIdx.x] = make_float2(cn, cd);
         }
-        sn += cn;
-        sd += cd;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int k = 0; k < min(256, B - b0); ++k) {
+                sn += sh[k].x;
+                sd += sh[k].y;
+            }
+        __syncthreads();
     }
+    if (threadIdx.x != 0) return;
     bool ok = sd > 0.0f;
     *scale = ok ? 1.0f / sd : 0.0f;
     *loss = ok ? sn / sd : 0.0f;
@@ -1397,18 +1266,12 @@ int gfgpu_internal_coarse_apply(const gfgpu_coarse_desc* g, const int32_t* part,
 namespace gfgpu {
 namespace nn {
 
-constexpr int kWgtBlocks = 256; // fixed partition of the weight-gradient reduction
+constexpr int kWgtBlocks = 152; // weight-gradient partials: a block on each of the 152 SMs
 constexpr int kRed = 1024;      // fixed grid of the FCG reductions
 
 inline int64_t a256(int64_t b)
 {
     return (b + 255) / 256 * 256;
-}
-
-inline unsigned pix_grid(int64_t npix)
-{
-    int64_t g = (npix + 127) / 128;
-    return static_cast<unsigned>(g < 1 ? 1 : (g > 65535 * 4 ? 65535 * 4 : g));
 }
 
 struct TrainWs {
@@ -1417,7 +1280,8 @@ struct TrainWs {
 
 inline TrainWs carve_train(void* ws, int64_t B, int64_t npix)
 {
-    char* c = static_cast<char*>(ws);
+    // the tiles are copied 16 bytes at a time: the buffers start at a multiple of 256 whatever `ws` is
+    char* c = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(ws) + 255) / 256 * 256);
     TrainWs w;
     float** bufs[] = {&w.a1, &w.a2, &w.a3, &w.g2, &w.g1};
     for (auto b : bufs) {
@@ -1446,7 +1310,7 @@ inline int64_t loss_bytes(int64_t B)
 inline int64_t train_bytes(int64_t B, int64_t npix)
 {
     return 5 * a256(npix * 32 * 4) + 2 * a256(npix * 2 * 4) +
-           a256(int64_t(kWgtBlocks) * (9 * 32 * 32 + 32) * 4) + loss_bytes(B);
+           a256(int64_t(kWgtBlocks) * (9 * 32 * 32 + 32) * 4) + loss_bytes(B) + 256;
 }
 
 // Element stiffness of the unit square (2x2 Gauss, plane strain) per unit K and per unit G.
@@ -1507,27 +1371,71 @@ inline const __nv_bfloat16* wb(const void* p, int l)
     return static_cast<const __nv_bfloat16*>(p) + w_off(l);
 }
 
-// forward of the four layers in FP32 on B images of H x W, activations kept for the backward
-inline void forward_f32(const void* wbf, const float* pf, const float* X, int B, int H, int W,
-                        TrainWs& w, cudaStream_t s)
+inline bool is_aligned16(const void* p)
 {
-    int64_t npix = int64_t(B) * H * W;
-    unsigned g = pix_grid(npix);
-    k_conv_fwd<4, 32, true, float, float><<<g, 128, 0, s>>>(X, wb(wbf, 0), pf + b_off(0), dil_of(0), B, H, W, w.a1);
-    k_conv_fwd<32, 32, true, float, float><<<g, 128, 0, s>>>(w.a1, wb(wbf, 1), pf + b_off(1), dil_of(1), B, H, W, w.a2);
-    k_conv_fwd<32, 32, true, float, float><<<g, 128, 0, s>>>(w.a2, wb(wbf, 2), pf + b_off(2), dil_of(2), B, H, W, w.a3);
-    k_conv_fwd<32, 2, false, float, float><<<g, 128, 0, s>>>(w.a3, wb(wbf, 3), pf + b_off(3), dil_of(3), B, H, W, w.y);
+    return (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
+}
+
+// Blocks of a tile kernel: one wave of `per_sm` blocks on each of the 152 SMs (what its shared
+// memory allows) walks the tiles when there are more, so that the weights are staged once per
+// block, else one block per tile.
+inline unsigned tile_blocks(const TrainGrid& g, int per_sm)
+{
+    return static_cast<unsigned>(std::min<int64_t>(g.tiles, int64_t(152) * per_sm));
+}
+
+// dynamic shared memory above 48 KB, granted per device and kernel
+template <class K>
+inline int allow_smem(K kernel, size_t bytes)
+{
+    return check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
+                      "cudaFuncSetAttribute");
+}
+
+inline int prepare_train()
+{
+    GF_TRY(allow_smem(k_conv_tile<32, false>, conv_smem(32, 4)));
+    GF_TRY(allow_smem(k_conv_tile<32, true>, conv_smem(32, 4)));
+    GF_TRY(allow_smem(k_conv_out, conv_out_smem(dil_of(3))));
+    GF_TRY(allow_smem(k_wgrad_tile<4, 32>, wgrad_smem(4, 32, dil_of(0))));
+    GF_TRY(allow_smem(k_wgrad_tile<32, 2>, wgrad_smem(32, 2, dil_of(3))));
+    return allow_smem(k_wgrad_tile<32, 32>, wgrad_smem(32, 32, 4));
+}
+
+// forward of the four layers in FP32 on B images of H x W, activations kept for the backward
+inline int forward_f32(const void* wbf, const float* pf, const float* X, int B, int H, int W, TrainWs& w,
+                       cudaStream_t s)
+{
+    GF_TRY(prepare_train());
+    const TrainGrid g = train_grid(B, H, W);
+    k_conv_tile<4, false><<<tile_blocks(g, 4), 256, conv_smem(4, dil_of(0)), s>>>(X, wb(wbf, 0), pf + b_off(0), dil_of(0), g, nullptr,
+                                                                   is_aligned16(X), w.a1);
+    k_conv_tile<32, false><<<tile_blocks(g, 2), 256, conv_smem(32, dil_of(1)), s>>>(w.a1, wb(wbf, 1), pf + b_off(1), dil_of(1), g,
+                                                                     nullptr, true, w.a2);
+    k_conv_tile<32, false><<<tile_blocks(g, 2), 256, conv_smem(32, dil_of(2)), s>>>(w.a2, wb(wbf, 2), pf + b_off(2), dil_of(2), g,
+                                                                     nullptr, true, w.a3);
+    k_conv_out<<<tile_blocks(g, 4), 256, conv_out_smem(dil_of(3)), s>>>(w.a3, wb(wbf, 3), pf + b_off(3), dil_of(3), g, w.y);
+    return check_launch("nn training forward");
 }
 
 template <int CI, int CO>
-inline void weight_grad(const float* X, const float* dY, int dil, int B, int H, int W, float* partial,
-                        float* grad, cudaStream_t s)
+inline void weight_grad(const float* X, const float* dY, int dil, const TrainGrid& g, float* partial, float* grad,
+                        cudaStream_t s)
 {
-    int threads = (9 * CI + 31) / 32 * 32;
-    if (threads < CO) threads = 32;
-    k_conv_bwd_weight<CI, CO><<<kWgtBlocks, threads, 0, s>>>(X, dY, dil, B, H, W, partial);
-    int n = 9 * CI * CO + CO;
-    k_sum_partials<<<(n + 255) / 256, 256, 0, s>>>(partial, kWgtBlocks, n, grad);
+    const unsigned nb = tile_blocks(g, kWgtBlocks / 152);
+    k_wgrad_tile<CI, CO><<<nb, kWgradThreads, wgrad_smem(CI, CO, dil), s>>>(X, dY, dil, g, is_aligned16(X), partial);
+    const int n = 9 * CI * CO + CO;
+    k_sum_partials<<<(n + 31) / 32, 256, 0, s>>>(partial, static_cast<int>(nb), n, grad);
+}
+
+// gradient for the input of a layer 32 -> CO (act: that input, the output of a ReLU)
+template <int CO>
+inline void data_grad(const float* dY, const void* wbf, int layer, const TrainGrid& g, const float* act, float* dX,
+                      cudaStream_t s)
+{
+    const int dil = dil_of(layer);
+    k_conv_tile<CO, true><<<tile_blocks(g, CO == 2 ? 4 : 2), 256, conv_smem(CO, dil), s>>>(dY, wb(wbf, layer), nullptr, dil, g, act,
+                                                                          true, dX);
 }
 
 // ---------------------------------------------------------------- FCG kernels
@@ -2200,7 +2108,7 @@ int gfgpu_nn_forward(const void* weights_bf16, const float* params_f32, const fl
     GF_REQUIRE(weights_bf16 && params_f32 && X && Y && workspace && B > 0 && H > 0 && W > 0,
                "bad argument");
     TrainWs w = carve_train(workspace, B, int64_t(B) * H * W);
-    forward_f32(weights_bf16, params_f32, X, B, H, W, w, S(stream));
+    GF_TRY(forward_f32(weights_bf16, params_f32, X, B, H, W, w, S(stream)));
     GF_TRY(check_cuda(cudaMemcpyAsync(Y, w.y, int64_t(B) * H * W * 2 * 4, cudaMemcpyDeviceToDevice,
                                       S(stream)),
                       "cudaMemcpyAsync"));
@@ -2218,28 +2126,28 @@ int gfgpu_nn_train_step(const void* weights_bf16, const float* params_f32, const
     cudaStream_t s = S(stream);
     int64_t npix = int64_t(B) * S_ * S_;
     TrainWs w = carve_train(workspace, B, npix);
-    forward_f32(weights_bf16, params_f32, X, B, S_, S_, w, s);
+    GF_TRY(forward_f32(weights_bf16, params_f32, X, B, S_, S_, w, s));
     if (E) {
         GF_TRY(upload_ke());
         k_crop_energy<<<dim3(kEnergyBlocks, B), 256, 0, s>>>(w.y, T, E, F, B, S_, margin, w.g3, w.epart);
-        k_energy_reduce<<<1, 32, 0, s>>>(w.epart, B, kEnergyBlocks, w.escale, loss);
+        k_energy_reduce<<<1, 256, 0, s>>>(w.epart, B, kEnergyBlocks, w.escale, loss);
         k_scale_grad<<<grid_for(npix * 2), kBlock, 0, s>>>(w.escale, npix * 2, w.g3);
     } else {
         k_mse<<<1024, 256, 0, s>>>(w.y, T, B, S_, margin, 2, w.g3, w.lpart);
-        k_sum_partials<<<1, 32, 0, s>>>(w.lpart, 1024, 1, loss);
+        k_sum_partials<<<1, 256, 0, s>>>(w.lpart, 1024, 1, loss);
     }
+    const TrainGrid g = train_grid(B, S_, S_);
     // layer 4 (32 -> 2)
-    weight_grad<32, 2>(w.a3, w.g3, dil_of(3), B, S_, S_, w.partial, grads + w_off(3), s);
-    unsigned g = pix_grid(npix);
-    k_conv_bwd_data<32, 2><<<g, 128, 0, s>>>(w.g3, wb(weights_bf16, 3), dil_of(3), B, S_, S_, w.a3, w.g2);
+    weight_grad<32, 2>(w.a3, w.g3, dil_of(3), g, w.partial, grads + w_off(3), s);
+    data_grad<2>(w.g3, weights_bf16, 3, g, w.a3, w.g2, s);
     // layer 3 (32 -> 32)
-    weight_grad<32, 32>(w.a2, w.g2, dil_of(2), B, S_, S_, w.partial, grads + w_off(2), s);
-    k_conv_bwd_data<32, 32><<<g, 128, 0, s>>>(w.g2, wb(weights_bf16, 2), dil_of(2), B, S_, S_, w.a2, w.g1);
+    weight_grad<32, 32>(w.a2, w.g2, dil_of(2), g, w.partial, grads + w_off(2), s);
+    data_grad<32>(w.g2, weights_bf16, 2, g, w.a2, w.g1, s);
     // layer 2 (32 -> 32): the gradient of its input goes back into g2
-    weight_grad<32, 32>(w.a1, w.g1, dil_of(1), B, S_, S_, w.partial, grads + w_off(1), s);
-    k_conv_bwd_data<32, 32><<<g, 128, 0, s>>>(w.g1, wb(weights_bf16, 1), dil_of(1), B, S_, S_, w.a1, w.g2);
+    weight_grad<32, 32>(w.a1, w.g1, dil_of(1), g, w.partial, grads + w_off(1), s);
+    data_grad<32>(w.g1, weights_bf16, 1, g, w.a1, w.g2, s);
     // layer 1 (4 -> 32)
-    weight_grad<4, 32>(X, w.g2, dil_of(0), B, S_, S_, w.partial, grads + w_off(0), s);
+    weight_grad<4, 32>(X, w.g2, dil_of(0), g, w.partial, grads + w_off(0), s);
     return check_launch("nn_train_step");
 }
 
