@@ -427,14 +427,13 @@ __global__ void k_int_n_scalar_diag(const double* __restrict__ N, const double* 
     }
 }
 
-// Int_gradN_dot_tensor4_dot_gradNT_dV: Element.h:1132-1176. Thread per elemmat entry; the
-// entry (m*nd+j, n*nd+k) accumulates over q, then i, then l as in the reference loop nest.
-// td: tensor dimension of C (td = 3 with nd = 2: QuadraturePlanar, the in-plane indices of a
+// Int_gradN_dot_tensor4_dot_gradNT_dV: Element.h:1132-1176, strict arithmetic. Thread per elemmat
+// entry; the entry (m*nd+j, n*nd+k) accumulates over q, then i, then l as in the reference loop
+// nest. td: tensor dimension of C (td = 3 with nd = 2: QuadraturePlanar, the in-plane indices of a
 // [3,3,3,3] tensor).
-template <bool S>
-__global__ void k_int_tensor4(const double* __restrict__ dNx, const double* __restrict__ vol,
-                              const double* __restrict__ C, int64_t nelem, int nne, int nip,
-                              int nd, int td, double* __restrict__ elemmat)
+__global__ void k_int_tensor4_strict(const double* __restrict__ dNx, const double* __restrict__ vol,
+                                     const double* __restrict__ C, int64_t nelem, int nne, int nip,
+                                     int nd, int td, double* __restrict__ elemmat)
 {
     int K = nne * nd;
     GF_FOR(t, nelem * K * K)
@@ -450,12 +449,111 @@ __global__ void k_int_tensor4(const double* __restrict__ dNx, const double* __re
             double v = vol[e * nip + q];
             for (int i = 0; i < nd; ++i)
                 for (int l = 0; l < nd; ++l)
-                    acc = madd<S>(mul<S>(mul<S>(g[m * nd + i], Cq[((i * td + j) * td + k) * td + l]),
-                                         g[n * nd + l]),
-                                  v, acc);
+                    acc = madd<true>(mul<true>(mul<true>(g[m * nd + i], Cq[((i * td + j) * td + k) * td + l]),
+                                               g[n * nd + l]),
+                                     v, acc);
         }
         elemmat[t] = acc;
     }
+}
+
+// The same, fast arithmetic, in two steps: T[m,j,k,l] = sum_i (v g[m,i]) C[i,j,k,l], then
+// K[(m,j),(n,k)] += sum_l T[m,j,k,l] g[n,l]. FP64 instructions bound it (FP64 issues 2 per SM and
+// clock): 200 (nd = 2) and 2400 (nd = 3) per integration point against 768 and 15552 of the form
+// above, whose three factors are multiplied anew for every (i, l) of every entry. A thread owns the
+// row (m, j) and the columns (n, k) of one k, so that its T never leaves registers; the NNE * ND^2
+// threads of an element read its tensors, gradients and v * gradients from shared memory, filled
+// (and the matrices written back) in address order. EPB elements per block make whole warps
+// (16 x 16 and 72 x 4 threads).
+template <int NNE, int ND>
+struct Tensor4Block {
+    static constexpr int K = NNE * ND, C4 = ND * ND * ND * ND, G = NNE * ND;
+    static constexpr int TPE = NNE * ND * ND;        // threads per element
+    static constexpr int EPB = ND == 2 ? 16 : 4;     // elements per block
+    static constexpr int THREADS = TPE * EPB;
+    static constexpr int QC = NNE;                   // integration points staged at a time
+    static constexpr int SZ = QC * (C4 + 2 * G) + 2; // per element, + 2: elements on other banks
+    static_assert(SZ >= K * K && THREADS % 32 == 0, "shared layout");
+};
+
+template <int NNE, int ND, int TD>
+__global__ void __launch_bounds__(Tensor4Block<NNE, ND>::THREADS)
+k_int_tensor4(const double* __restrict__ dNx, const double* __restrict__ vol,
+              const double* __restrict__ C, int64_t nelem, int nip, double* __restrict__ elemmat)
+{
+    using B = Tensor4Block<NNE, ND>;
+    constexpr int K = B::K, C4 = B::C4, G = B::G, QC = B::QC, SZ = B::SZ, T4 = TD * TD * TD * TD;
+    __shared__ double sm[B::EPB * SZ];
+    const int tid = threadIdx.x;
+    const int el = tid / B::TPE, r = tid - el * B::TPE;
+    const int m = r / (ND * ND), j = (r / ND) % ND, k = r % ND;
+    const int64_t e0 = static_cast<int64_t>(blockIdx.x) * B::EPB;
+    const int ne = static_cast<int>(nelem - e0 < B::EPB ? nelem - e0 : B::EPB);
+    double* se = sm + el * SZ;
+    double acc[NNE];
+#pragma unroll
+    for (int n = 0; n < NNE; ++n) acc[n] = 0.0;
+    for (int q0 = 0; q0 < nip; q0 += QC) {
+        const int nq = nip - q0 < QC ? nip - q0 : QC;
+        // per element: [QC][C4] tensors, [QC][G] gradients, [QC][G] v * gradients
+        for (int i = tid; i < ne * nq * C4; i += B::THREADS) {
+            const int x = i / (nq * C4), y = i - x * nq * C4;
+            if constexpr (TD == ND) {
+                sm[x * SZ + y] = __ldg(C + ((e0 + x) * nip + q0) * T4 + y);
+            }
+            else {
+                // the in-plane entries of [TD]^4 (ND = 2)
+                const int q = y / C4, c = y - q * C4;
+                const int at = (((c >> 3) * TD + ((c >> 2) & 1)) * TD + ((c >> 1) & 1)) * TD + (c & 1);
+                sm[x * SZ + y] = __ldg(C + ((e0 + x) * nip + q0 + q) * T4 + at);
+            }
+        }
+        for (int i = tid; i < ne * nq * G; i += B::THREADS) {
+            const int x = i / (nq * G), y = i - x * nq * G, q = y / G;
+            const double g = __ldg(dNx + ((e0 + x) * nip + q0) * G + y);
+            sm[x * SZ + QC * C4 + y] = g;
+            sm[x * SZ + QC * (C4 + G) + y] = __ldg(vol + (e0 + x) * nip + q0 + q) * g;
+        }
+        __syncthreads();
+        if (el < ne) {
+            for (int q = 0; q < nq; ++q) {
+                const double* c = se + q * C4 + (j * ND + k) * ND;
+                const double* g = se + QC * C4 + q * G;
+                const double* gv = se + QC * (C4 + G) + q * G + m * ND;
+                double t[ND];
+#pragma unroll
+                for (int l = 0; l < ND; ++l) t[l] = gv[0] * c[l];
+#pragma unroll
+                for (int i = 1; i < ND; ++i)
+#pragma unroll
+                    for (int l = 0; l < ND; ++l) t[l] = fma(gv[i], c[i * ND * ND * ND + l], t[l]);
+#pragma unroll
+                for (int n = 0; n < NNE; ++n)
+#pragma unroll
+                    for (int l = 0; l < ND; ++l) acc[n] = fma(t[l], g[n * ND + l], acc[n]);
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int n = 0; n < NNE; ++n) se[(m * ND + j) * K + n * ND + k] = acc[n];
+    __syncthreads();
+    for (int i = tid; i < ne * K * K; i += B::THREADS) {
+        const int x = i / (K * K);
+        elemmat[e0 * K * K + i] = sm[x * SZ + i - x * K * K];
+    }
+}
+
+template <int NNE, int ND, int TD = ND>
+static void launch_int_tensor4(const double* dNx, const double* vol, const double* C, int64_t nelem, int nip,
+                               double* elemmat, cudaStream_t s)
+{
+    using B = Tensor4Block<NNE, ND>;
+    if (strict_mode())
+        k_int_tensor4_strict<<<grid_for(nelem * B::K * B::K), kBlock, 0, s>>>(dNx, vol, C, nelem, NNE, nip, ND, TD,
+                                                                             elemmat);
+    else
+        k_int_tensor4<NNE, ND, TD><<<grid_for(nelem, B::EPB), B::THREADS, 0, s>>>(dNx, vol, C, nelem, nip, elemmat);
 }
 
 // Linear elastic stress (plane strain for nd = 2), same operation order as the oracle.
@@ -679,8 +777,10 @@ int gfgpu_int_grad_n_dot_tensor4_dot_grad_nt_dv(const double* dNx, const double*
     int64_t K = nne * ndim;
     GF_REQUIRE(!too_big(nelem * K * K), "too many elements");
     if (nelem == 0) return GFGPU_OK;
-    DISPATCH_S(k_int_tensor4<kS><<<grid_for(nelem * K * K), kBlock, 0, S(stream)>>>(
-        dNx, vol, qtensor4, nelem, nne, nip, ndim, ndim, elemmat));
+    if (ndim == 2)
+        launch_int_tensor4<4, 2>(dNx, vol, qtensor4, nelem, nip, elemmat, S(stream));
+    else
+        launch_int_tensor4<8, 3>(dNx, vol, qtensor4, nelem, nip, elemmat, S(stream));
     return check_launch("int_grad_n_dot_tensor4_dot_grad_nt_dv");
 }
 
@@ -733,8 +833,7 @@ int gfgpu_int_grad_n_dot_tensor4_dot_grad_nt_dv_planar(const double* dNx, const 
     GF_REQUIRE(dNx && vol && qtensor4 && elemmat && nip > 0, "bad argument");
     GF_REQUIRE(!too_big(nelem * 64) && !too_big(nelem * nip * 81), "too many elements");
     if (nelem == 0) return GFGPU_OK;
-    DISPATCH_S(k_int_tensor4<kS><<<grid_for(nelem * 64), kBlock, 0, S(stream)>>>(
-        dNx, vol, qtensor4, nelem, 4, nip, 2, 3, elemmat));
+    launch_int_tensor4<4, 2, 3>(dNx, vol, qtensor4, nelem, nip, elemmat, S(stream));
     return check_launch("int_grad_n_dot_tensor4_dot_grad_nt_dv_planar");
 }
 
