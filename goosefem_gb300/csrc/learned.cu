@@ -1267,7 +1267,7 @@ namespace gfgpu {
 namespace nn {
 
 constexpr int kWgtBlocks = 152; // weight-gradient partials: a block on each of the 152 SMs
-constexpr int kRed = 1024;      // fixed grid of the FCG reductions
+constexpr int kRed = 1024; // most blocks (and partials per row) of the FCG reductions
 
 inline int64_t a256(int64_t b)
 {
@@ -1467,7 +1467,16 @@ __device__ __forceinline__ double bsum(double v, double* sh)
     return r;
 }
 
-// Last-block reductions: every block of a 1024-block (kRed) partial-sum kernel writes its partial,
+// Blocks of a reduction kernel over `items` entries: one per 256, at most kRed. A block without
+// entries still costs its launch, two block sums and an atomic on the counter: at 63k dofs (246
+// blocks) the dots took 12-19 us and the gather 14 us with 1024 blocks whatever the size. The
+// partials keep their places and order of summation, so the sums keep their bits.
+inline unsigned red_blocks(int64_t items)
+{
+    return static_cast<unsigned>(std::min<int64_t>(kRed, std::max<int64_t>(1, (items + 255) / 256)));
+}
+
+// Last-block reductions: every block of a partial-sum kernel writes its partial,
 // fences and counts itself in; the last block to arrive reduces the partials (fixed order, so the
 // result does not depend on which block is last) and resets the counter for the next launch. This
 // replaces a separate one-block reduction launch.
@@ -1486,11 +1495,11 @@ __device__ __forceinline__ bool last_block(unsigned int* counter)
     return is_last;
 }
 
-// sum of partial[0 .. kRed) by the whole block in a fixed order
+// sum of partial[0 .. gridDim.x) by the whole block in a fixed order
 __device__ __forceinline__ double block_sum_partials(const double* partial, double* sh)
 {
     double v = 0.0;
-    for (int i = threadIdx.x; i < kRed; i += blockDim.x) v += __ldcg(partial + i);
+    for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x) v += __ldcg(partial + i);
     return bsum(v, sh);
 }
 
@@ -1502,7 +1511,7 @@ __device__ __forceinline__ void coef_rows(const double* partial, const SlotList&
     const int nw = blockDim.x >> 5, lane = threadIdx.x & 31;
     for (int k = threadIdx.x >> 5; k < L.n; k += nw) {
         double v = 0.0;
-        for (int i = lane; i < kRed; i += 32) v += __ldcg(partial + k * kRed + i);
+        for (int i = lane; i < gridDim.x; i += 32) v += __ldcg(partial + k * kRed + i);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
         if (lane == 0) {
@@ -1609,13 +1618,13 @@ k_resid1(const double* __restrict__ r, const double* __restrict__ q0, double* __
     }
 }
 
-// sc[dst.s[k]] = sum of partial row k (fixed order)
-__global__ void k_fredv(const double* __restrict__ partial, SlotList dst, double* __restrict__ sc)
+// sc[dst.s[k]] = sum of the nblk partials of row k (fixed order)
+__global__ void k_fredv(const double* __restrict__ partial, int nblk, SlotList dst, double* __restrict__ sc)
 {
     __shared__ double sh[32];
     for (int p = 0; p < dst.n; ++p) {
         double v = 0.0;
-        for (int i = threadIdx.x; i < kRed; i += blockDim.x) v += partial[p * kRed + i];
+        for (int i = threadIdx.x; i < nblk; i += blockDim.x) v += partial[p * kRed + i];
         double t = bsum(v, sh);
         if (threadIdx.x == 0) sc[dst.s[p]] = t;
         __syncthreads();
@@ -2238,7 +2247,7 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
         yc = reinterpret_cast<double*>(c + a256(n * 8) + a256(nc * 8));
     }
     const double nfree = static_cast<double>(d->nnu);
-    const unsigned gb = kRed;
+    const unsigned gb = red_blocks(n);
     double h[F_COUNT];
     auto read_sc = [&]() -> int {
         GF_TRY(check_cuda(cudaMemcpyAsync(h, w.sc, F_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s),
@@ -2280,7 +2289,7 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
                 zin = w.z;
             }
             if (L.n > 0) {
-                with_ns<MdotL>(L.n, gb, st, zin, w.minv, w.r, w.Q, w.ld, L, n, w.partial, w.sc, w.cnt);
+                with_ns<MdotL>(L.n, red_blocks(n / 2), st, zin, w.minv, w.r, w.Q, w.ld, L, n, w.partial, w.sc, w.cnt);
             }
             with_ns<McombineL>(L.n, grid_for(n / 2), st, zin, w.minv, w.r, w.sc, w.P, w.ld, L, snew, n);
             double* Pn = w.P + snew * w.ld;
@@ -2303,12 +2312,12 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
     GF_TRY(gfgpu_internal_element_forces(d, w.P, w.fe, s));
     k_fres<<<gb, 256, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.z,
                               w.partial, reg_grid(d));
-    k_fredv<<<1, 1024, 0, s>>>(w.partial, one(F_BB), w.sc);
+    k_fredv<<<1, 1024, 0, s>>>(w.partial, static_cast<int>(gb), one(F_BB), w.sc);
     // r = -(A x)_u
     GF_TRY(gfgpu_internal_element_forces(d, x, w.fe, s));
     k_fres<<<gb, 256, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.r,
                               w.partial, reg_grid(d));
-    k_fredv<<<1, 1024, 0, s>>>(w.partial, one(F_RR), w.sc);
+    k_fredv<<<1, 1024, 0, s>>>(w.partial, static_cast<int>(gb), one(F_RR), w.sc);
     GF_TRY(read_sc());
     double bnorm = std::sqrt(h[F_BB]);
     if (bnorm == 0.0) bnorm = 1.0;
@@ -2380,7 +2389,7 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
     GF_TRY(gfgpu_internal_element_forces(d, x, w.fe, s));
     k_fres<<<gb, 256, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.r,
                               w.partial, reg_grid(d));
-    k_fredv<<<1, 1024, 0, s>>>(w.partial, one(F_RR), w.sc);
+    k_fredv<<<1, 1024, 0, s>>>(w.partial, static_cast<int>(gb), one(F_RR), w.sc);
     GF_TRY(read_sc());
     *iters = it;
     *relres = std::sqrt(h[F_RR]) / bnorm;
