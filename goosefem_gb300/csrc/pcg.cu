@@ -8,6 +8,7 @@
 // in p, r, z. Dot products use a fixed grid and a fixed reduction tree, so every run gives the
 // same bits. The iteration scalars (alpha, beta) stay on the device; the host reads the residual
 // only every `check_every` iterations.
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -16,37 +17,47 @@
 
 namespace gfgpu {
 
-constexpr int kRedBlocks = 1024; // fixed: determinism of the reductions
+constexpr int kRedBlocks = 4096; // most blocks (and partials per row) of a reduction kernel
 constexpr int kRedThreads = 256;
+constexpr int kReduceThreads = 1024; // the one-block kernels that add the partials (set-up, residual)
+constexpr int kWideThreads = 1024;   // update and direction
+
+// Blocks of a reduction kernel over n entries: one entry per thread up to kRedBlocks blocks. Fixed by
+// n: the same sums on every run.
+inline unsigned red_blocks(int64_t n)
+{
+    return static_cast<unsigned>(std::min<int64_t>(kRedBlocks, std::max<int64_t>(1, (n + kRedThreads - 1) / kRedThreads)));
+}
 
 // scalar slots
+// SC_RZ: r.z of the current direction; SC_RZ_NEW: of the last update (copied by the next gather)
 enum { SC_RZ = 0, SC_RZ_NEW, SC_PQ, SC_RR, SC_BB, SC_ALPHA, SC_BETA, SC_COUNT };
 
+// Sum over the block's threads, a fixed order, valid in thread 0 (sh: blockDim doubles). An FP64
+// instruction of a warp takes 16 clocks of the SM's pipe, so the sum is left to one warp: 8 + 5 of
+// them for 256 threads, where a shuffle tree in every warp takes 8 x 5 + 5.
 __device__ __forceinline__ double block_sum(double v, double* sh)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) sh[w] = v;
+    sh[threadIdx.x] = v;
     __syncthreads();
     double r = 0.0;
-    if (w == 0) {
-        r = lane < (blockDim.x >> 5) ? sh[lane] : 0.0;
+    if (threadIdx.x < 32) {
+        for (int i = threadIdx.x; i < static_cast<int>(blockDim.x); i += 32) r += sh[i];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
     }
     __syncthreads();
-    return r; // valid in thread 0
+    return r;
 }
 
-// Final fixed-order reduction of `nparts` partial rows (kRedBlocks each) into scalars.
-__global__ void k_reduce(const double* __restrict__ partials, int nparts, double* __restrict__ sc,
+// Final fixed-order reduction of `nparts` partial rows (nblk partials each) into scalars.
+__global__ void k_reduce(const double* __restrict__ partials, int nblk, int nparts, double* __restrict__ sc,
                          int slot0)
 {
-    __shared__ double sh[32];
+    __shared__ double sh[kReduceThreads];
     for (int p = 0; p < nparts; ++p) {
         double v = 0.0;
-        for (int i = threadIdx.x; i < kRedBlocks; i += blockDim.x) v += partials[p * kRedBlocks + i];
+        for (int i = threadIdx.x; i < nblk; i += blockDim.x) v += partials[p * kRedBlocks + i];
         double s = block_sum(v, sh);
         if (threadIdx.x == 0) sc[slot0 + p] = s;
         __syncthreads();
@@ -58,9 +69,10 @@ __global__ void __launch_bounds__(kRedThreads)
 k_pcg_gather(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr,
              const int32_t* __restrict__ idx, const int32_t* __restrict__ part, int64_t nnu,
              const double* __restrict__ fe, const double* __restrict__ p, int64_t n,
-             double* __restrict__ q, double* __restrict__ partial, RegGrid reg)
+             double* __restrict__ q, double* __restrict__ partial, double* __restrict__ sc, RegGrid reg)
 {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
+    if (blockIdx.x == 0 && threadIdx.x == 0) sc[SC_RZ] = sc[SC_RZ_NEW];
     double acc = 0.0;
     GF_FOR(t, n)
     {
@@ -75,73 +87,92 @@ k_pcg_gather(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr,
     if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
-// p.q from the gather's partial row, then alpha = r.z / p.q (one launch)
-__global__ void k_reduce_alpha(const double* __restrict__ partials, double* __restrict__ sc)
+// The sum of nblk partials, valid in thread 0. The kernel after a dot product adds its partials
+// itself, in each of its blocks: two blocks of 1024 threads per SM keep that to a load or two per
+// thread and 37 warp instructions in FP64 per block. A one-block launch for the sum took 4-6 us of a
+// 60 us iteration at 64^3; a last block that adds the others' partials, with a fence and an atomic in
+// each, 10 us.
+__device__ __forceinline__ double sum_partials(const double* __restrict__ partial, int nblk, double* sh)
 {
-    __shared__ double sh[32];
     double v = 0.0;
-    for (int i = threadIdx.x; i < kRedBlocks; i += blockDim.x) v += partials[i];
-    double s = block_sum(v, sh);
-    if (threadIdx.x == 0) {
-        sc[SC_PQ] = s;
-        sc[SC_ALPHA] = sc[SC_RZ] / s;
-    }
+    for (int i = threadIdx.x; i < nblk; i += blockDim.x) v += partial[i];
+    return block_sum(v, sh);
 }
 
-// x += alpha p, r -= alpha q, z = M^-1 r (free dofs); partials r.z and r.r.
-__global__ void __launch_bounds__(kRedThreads)
+// thread 0's v in every thread (a division is a dozen FP64 instructions: one warp takes it)
+__device__ __forceinline__ double from_thread0(double v, double* sh)
+{
+    if (threadIdx.x == 0) sh[0] = v;
+    __syncthreads();
+    v = sh[0];
+    __syncthreads();
+    return v;
+}
+
+// alpha = r.z / p.q from the gather's partials (row 0); x += alpha p, r -= alpha q, z = M^-1 r (free
+// dofs); partials r.z and, with RR, r.r in rows 1 and 2. With both that is 5 FP64 instructions per dof,
+// and FP64 issue is 60 % of the kernel's time: r.r is formed in the iterations after which the host
+// reads it.
+template <bool RR>
+__global__ void __launch_bounds__(kWideThreads, 2)
 k_pcg_update(const int32_t* __restrict__ part, int64_t nnu, const double* __restrict__ minv,
              const double* __restrict__ p, const double* __restrict__ q, int64_t n,
-             const double* __restrict__ sc, double* __restrict__ x, double* __restrict__ r,
-             double* __restrict__ z, double* __restrict__ partial)
+             double* __restrict__ sc, double* __restrict__ x, double* __restrict__ r,
+             double* __restrict__ z, const double* __restrict__ pq_part, int nblk, double* __restrict__ partial)
 {
-    __shared__ double sh[32];
-    double alpha = sc[SC_ALPHA];
+    __shared__ double sh[kWideThreads];
+    const double pq = sum_partials(pq_part, nblk, sh);
+    const double alpha = from_thread0(threadIdx.x == 0 ? sc[SC_RZ] / pq : 0.0, sh);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sc[SC_PQ] = pq;
+        sc[SC_ALPHA] = alpha;
+    }
     double rz = 0.0, rr = 0.0;
     GF_FOR(t, n)
     {
-        if (__ldg(part + t) < nnu) {
-            x[t] = fma(alpha, p[t], x[t]);
-            double rv = fma(-alpha, q[t], r[t]);
-            double zv = minv[t] * rv;
-            r[t] = rv;
-            z[t] = zv;
-            rz = fma(rv, zv, rz);
-            rr = fma(rv, rv, rr);
-        }
+        // all loads before the test of the dof
+        const bool fr = __ldg(part + t) < nnu;
+        const double pv = p[t], qv = q[t], xv = x[t], rv = r[t], mv = __ldg(minv + t);
+        if (!fr) continue;
+        x[t] = fma(alpha, pv, xv);
+        const double rn = fma(-alpha, qv, rv), zn = mv * rn;
+        r[t] = rn;
+        z[t] = zn;
+        rz = fma(rn, zn, rz);
+        if (RR) rr = fma(rn, rn, rr);
     }
-    double s1 = block_sum(rz, sh);
-    double s2 = block_sum(rr, sh);
+    const double s1 = block_sum(rz, sh), s2 = RR ? block_sum(rr, sh) : 0.0;
     if (threadIdx.x == 0) {
-        partial[blockIdx.x] = s1;
-        partial[kRedBlocks + blockIdx.x] = s2;
+        partial[kRedBlocks + blockIdx.x] = s1;
+        if (RR) partial[2 * kRedBlocks + blockIdx.x] = s2;
     }
 }
 
-// r.z (new) and r.r from the update's partial rows, then beta = r.z_new / r.z (one launch)
-__global__ void k_reduce_beta(const double* __restrict__ partials, double* __restrict__ sc)
+// beta = r.z_new / r.z from the update's partials; the new r.z becomes the current one in the next
+// iteration's gather, where no block reads either
+__device__ __forceinline__ double direction_beta(const double* __restrict__ partial, int nblk, bool with_rr,
+                                                 double* sc, double* sh)
 {
-    __shared__ double sh[32];
-    double v0 = 0.0, v1 = 0.0;
-    for (int i = threadIdx.x; i < kRedBlocks; i += blockDim.x) {
-        v0 += partials[i];
-        v1 += partials[kRedBlocks + i];
+    const double rz = sum_partials(partial + kRedBlocks, nblk, sh);
+    const double beta = from_thread0(threadIdx.x == 0 ? rz / sc[SC_RZ] : 0.0, sh);
+    if (blockIdx.x == 0) {
+        const double rr = with_rr ? sum_partials(partial + 2 * kRedBlocks, nblk, sh) : 0.0;
+        if (threadIdx.x == 0) {
+            sc[SC_RZ_NEW] = rz;
+            if (with_rr) sc[SC_RR] = rr;
+            sc[SC_BETA] = beta;
+        }
     }
-    double rz = block_sum(v0, sh);
-    double rr = block_sum(v1, sh);
-    if (threadIdx.x == 0) {
-        sc[SC_RZ_NEW] = rz;
-        sc[SC_RR] = rr;
-        sc[SC_BETA] = rz / sc[SC_RZ];
-        sc[SC_RZ] = rz;
-    }
+    return beta;
 }
 
 // p = z + beta p
-__global__ void k_pcg_direction(const double* __restrict__ z, const double* __restrict__ sc,
-                                int64_t n, double* __restrict__ p)
+__global__ void __launch_bounds__(kWideThreads, 2)
+k_pcg_direction(const double* __restrict__ z, const double* __restrict__ partial, int nblk, bool with_rr,
+                double* __restrict__ sc, int64_t n, double* __restrict__ p)
 {
-    double beta = sc[SC_BETA];
+    __shared__ double sh[kWideThreads];
+    const double beta = direction_beta(partial, nblk, with_rr, sc, sh);
     GF_FOR(t, n) p[t] = fma(beta, p[t], z[t]);
 }
 
@@ -154,7 +185,7 @@ k_pcg_residual(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr
                double* __restrict__ z, double* __restrict__ p, double* __restrict__ partial,
                RegGrid reg)
 {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
     double rz = 0.0, rr = 0.0;
     GF_FOR(t, n)
     {
@@ -339,53 +370,62 @@ k_elem_force_hex8_cube_pair(const float2* __restrict__ up, const float4* __restr
 }
 
 // q = A p on free dofs from the pair element forces (the Regular Hex8 gather order of gather_dof,
-// summed as pairs, returned to FP64), 0 on prescribed dofs; partial p.q in FP64.
+// summed as pairs, returned to FP64), 0 on prescribed dofs; partial p.q in FP64. A thread per node:
+// its three components share the index arithmetic (two divisions) and the tests of the eight
+// elements, and their 24 loads are independent (64^3, element forces in L2: 21 -> 15 us against a
+// thread per dof).
 __global__ void __launch_bounds__(kRedThreads)
 k_pcg_gather_pair(const int32_t* __restrict__ part, int64_t nnu, const float2* __restrict__ fe,
-                  const double* __restrict__ p, int64_t n, double* __restrict__ q,
-                  double* __restrict__ partial, RegGrid reg)
+                  const double* __restrict__ p, int64_t nnode, double* __restrict__ q,
+                  double* __restrict__ partial, double* __restrict__ sc, RegGrid reg)
 {
-    __shared__ double sh[32];
+    __shared__ double sh[kRedThreads];
+    if (blockIdx.x == 0 && threadIdx.x == 0) sc[SC_RZ] = sc[SC_RZ_NEW];
     double acc = 0.0;
     const uint32_t nx = static_cast<uint32_t>(reg.nx), ny = static_cast<uint32_t>(reg.ny);
     const uint32_t nz = static_cast<uint32_t>(reg.nz), cs = nx * ny * nz;
     const uint32_t W = nx + 1u, A = W * (ny + 1u);
-    GF_FOR(t, n)
+    GF_FOR(node, nnode)
     {
-        double fv = 0.0;
-        if (__ldg(part + t) < nnu) {
-            const uint32_t tt = static_cast<uint32_t>(t), node = tt / 3u, i = tt - node * 3u;
-            const uint32_t iz = node / A, rem = node - iz * A, iy = rem / W, ix = rem - iy * W;
-            ffv f = ff_make(0.0f, 0.0f);
+        const uint32_t nd = static_cast<uint32_t>(node), iz = nd / A, rem = nd - iz * A, iy = rem / W, ix = rem - iy * W;
+        ffv f[3];
 #pragma unroll
-            for (int dz = 1; dz >= 0; --dz) {
-                if ((dz && iz == 0u) || (!dz && iz >= nz)) continue;
+        for (int i = 0; i < 3; ++i) f[i] = ff_make(0.0f, 0.0f);
 #pragma unroll
-                for (int dy = 1; dy >= 0; --dy) {
-                    if ((dy && iy == 0u) || (!dy && iy >= ny)) continue;
+        for (int dz = 1; dz >= 0; --dz)
 #pragma unroll
-                    for (int dx = 1; dx >= 0; --dx) {
-                        if ((dx && ix == 0u) || (!dx && ix >= nx)) continue;
-                        const int m = 4 * dz + (dy ? (dx ? 2 : 3) : (dx ? 1 : 0));
-                        const uint32_t e = ((iz - dz) * ny + (iy - dy)) * nx + (ix - dx);
-                        f = ff_add(f, pfl(__ldg(fe + e + (m * 3u + i) * cs)));
-                    }
+            for (int dy = 1; dy >= 0; --dy)
+#pragma unroll
+                for (int dx = 1; dx >= 0; --dx) {
+                    const bool in = (dz ? iz > 0u : iz < nz) && (dy ? iy > 0u : iy < ny) && (dx ? ix > 0u : ix < nx);
+                    if (!in) continue;
+                    const int m = 4 * dz + (dy ? (dx ? 2 : 3) : (dx ? 1 : 0));
+                    const uint32_t e = ((iz - dz) * ny + (iy - dy)) * nx + (ix - dx);
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) f[i] = ff_add(f[i], pfl(__ldg(fe + e + (m * 3u + i) * cs)));
                 }
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const int64_t t = node * 3 + i;
+            double fv = 0.0;
+            if (__ldg(part + t) < nnu) {
+                fv = ff_to_double(f[i]);
+                acc = fma(p[t], fv, acc);
             }
-            fv = ff_to_double(f);
-            acc = fma(p[t], fv, acc);
+            q[t] = fv;
         }
-        q[t] = fv;
     }
     double s = block_sum(acc, sh);
     if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 
 // p = z + beta p, and p as pairs
-__global__ void k_pcg_direction_pair(const double* __restrict__ z, const double* __restrict__ sc,
-                                     int64_t n, double* __restrict__ p, float2* __restrict__ pp)
+__global__ void __launch_bounds__(kWideThreads, 2)
+k_pcg_direction_pair(const double* __restrict__ z, const double* __restrict__ partial, int nblk, bool with_rr,
+                     double* __restrict__ sc, int64_t n, double* __restrict__ p, float2* __restrict__ pp)
 {
-    double beta = sc[SC_BETA];
+    __shared__ double sh[kWideThreads];
+    const double beta = direction_beta(partial, nblk, with_rr, sc, sh);
     GF_FOR(t, n)
     {
         const double v = fma(beta, p[t], z[t]);
@@ -479,7 +519,7 @@ static PcgWs carve(const gfgpu_verlet_desc* d, void* ws)
         c += align256(n * 8);
     }
     w.partial = reinterpret_cast<double*>(c);
-    c += align256(2 * kRedBlocks * 8);
+    c += align256(3 * kRedBlocks * 8);
     w.sc = reinterpret_cast<double*>(c);
     c += align256(SC_COUNT * 8 + 64);
     w.pp = reinterpret_cast<float2*>(c);
@@ -490,7 +530,7 @@ static int64_t pcg_bytes(const gfgpu_verlet_desc* d)
 {
     int64_t n = d->nnode * d->ndim;
     return align256(d->nelem * d->nne * d->ndim * 8) + 6 * align256(n * 8) +
-           align256(2 * kRedBlocks * 8) + align256(SC_COUNT * 8 + 64) + align256(n * 8);
+           align256(3 * kRedBlocks * 8) + align256(SC_COUNT * 8 + 64) + align256(n * 8);
 }
 
 } // namespace gfgpu
@@ -584,34 +624,41 @@ static CubePair cube_pair(const gfgpu_verlet_desc* d)
     return c;
 }
 
-// One Jacobi-PCG iteration: 6 launches (element forces, gather, alpha, update, beta, direction);
+// One Jacobi-PCG iteration: 4 launches (element forces, gather, update, direction);
 // with d->pcg_pair the element forces and the gather run on pairs and the direction update also
-// writes the pair copy of p that the next iteration's element kernel reads.
-static int pcg_iteration(const gfgpu_verlet_desc* d, const PcgWs& w, double* x, int64_t n,
+// writes the pair copy of p that the next iteration's element kernel reads. rr: r.r as well (the last
+// iteration before it is read).
+static int pcg_iteration(const gfgpu_verlet_desc* d, const PcgWs& w, double* x, int64_t n, bool rr,
                          cudaStream_t s)
 {
-    const unsigned gb = kRedBlocks;
     const bool pair = d->pcg_pair != nullptr && d->nne == 8;
+    unsigned gg; // blocks and partials of the gather
     if (pair) {
         k_elem_force_hex8_cube_pair<<<grid_for(d->nelem, 128), 128, 0, s>>>(
             w.pp, reinterpret_cast<const float4*>(d->pcg_pair), cube_pair(d), d->nelem,
             reinterpret_cast<float2*>(w.fe));
-        k_pcg_gather_pair<<<gb, kRedThreads, 0, s>>>(d->part, d->nnu, reinterpret_cast<const float2*>(w.fe),
-                                                      w.p, n, w.q, w.partial, reg_grid(d));
+        gg = red_blocks(d->nnode);
+        k_pcg_gather_pair<<<gg, kRedThreads, 0, s>>>(d->part, d->nnu, reinterpret_cast<const float2*>(w.fe),
+                                                      w.p, d->nnode, w.q, w.partial, w.sc, reg_grid(d));
     }
     else {
         GF_TRY(gfgpu_internal_iteration_element_forces(d, w.p, w.fe, s));
-        k_pcg_gather<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
-                                                 w.p, n, w.q, w.partial, reg_grid(d));
+        gg = red_blocks(n);
+        k_pcg_gather<<<gg, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
+                                                 w.p, n, w.q, w.partial, w.sc, reg_grid(d));
     }
-    k_reduce_alpha<<<1, 1024, 0, s>>>(w.partial, w.sc);
-    k_pcg_update<<<gb, kRedThreads, 0, s>>>(d->part, d->nnu, w.minv, w.p, w.q, n, w.sc, x, w.r, w.z,
-                                             w.partial);
-    k_reduce_beta<<<1, 1024, 0, s>>>(w.partial, w.sc);
-    if (pair)
-        k_pcg_direction_pair<<<grid_for(n), kBlock, 0, s>>>(w.z, w.sc, n, w.p, w.pp);
+    // two wide blocks per SM, less where the dofs are fewer
+    const unsigned gu = std::min<unsigned>(2 * 152, grid_for(n, kWideThreads));
+    if (rr)
+        k_pcg_update<true><<<gu, kWideThreads, 0, s>>>(d->part, d->nnu, w.minv, w.p, w.q, n, w.sc, x, w.r, w.z,
+                                                       w.partial, static_cast<int>(gg), w.partial);
     else
-        k_pcg_direction<<<grid_for(n), kBlock, 0, s>>>(w.z, w.sc, n, w.p);
+        k_pcg_update<false><<<gu, kWideThreads, 0, s>>>(d->part, d->nnu, w.minv, w.p, w.q, n, w.sc, x, w.r, w.z,
+                                                        w.partial, static_cast<int>(gg), w.partial);
+    if (pair)
+        k_pcg_direction_pair<<<gu, kWideThreads, 0, s>>>(w.z, w.partial, static_cast<int>(gu), rr, w.sc, n, w.p, w.pp);
+    else
+        k_pcg_direction<<<gu, kWideThreads, 0, s>>>(w.z, w.partial, static_cast<int>(gu), rr, w.sc, n, w.p);
     return GFGPU_OK;
 }
 
@@ -637,7 +684,7 @@ int gfgpu_pcg_solve(const gfgpu_verlet_desc* d, const double* diag, double* x, d
     cudaStream_t s = S(stream);
     PcgWs w = carve(d, workspace);
     int64_t n = d->nnode * d->ndim;
-    const unsigned gb = kRedBlocks;
+    const unsigned gb = red_blocks(n);
     double* hsc = nullptr;
     GF_TRY(check_cuda(cudaMallocHost(&hsc, SC_COUNT * sizeof(double)), "cudaMallocHost"));
     int rc = GFGPU_OK;
@@ -651,18 +698,19 @@ int gfgpu_pcg_solve(const gfgpu_verlet_desc* d, const double* diag, double* x, d
     if ((rc = gfgpu_internal_element_forces(d, w.p, w.fe, s)) != GFGPU_OK) return fail_out(rc);
     k_pcg_residual<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
                                                nullptr, w.minv, n, w.bvec, w.z, nullptr, w.partial, reg_grid(d));
-    k_reduce<<<1, 1024, 0, s>>>(w.partial + kRedBlocks, 1, w.sc, SC_BB);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), 1, w.sc, SC_BB);
     // r = b - A x, z = M^-1 r, p = z
     if ((rc = gfgpu_internal_element_forces(d, x, w.fe, s)) != GFGPU_OK) return fail_out(rc);
     k_pcg_residual<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
                                                nullptr, w.minv, n, w.r, w.z, w.p, w.partial, reg_grid(d));
-    k_reduce<<<1, 1024, 0, s>>>(w.partial, 2, w.sc, SC_RZ); // SC_RZ, SC_RZ_NEW(=rr, overwritten)
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial, static_cast<int>(gb), 1, w.sc, SC_RZ_NEW);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), 1, w.sc, SC_RR);
     if (d->pcg_pair && d->nne == 8) k_pcg_split<<<grid_for(n), kBlock, 0, s>>>(w.p, n, w.pp);
     if ((rc = check_launch("pcg set-up")) != GFGPU_OK) return fail_out(rc);
     cudaMemcpyAsync(hsc, w.sc, SC_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s);
     if ((rc = check_cuda(cudaStreamSynchronize(s), "pcg set-up")) != GFGPU_OK) return fail_out(rc);
     double bb = hsc[SC_BB];
-    double rr = hsc[SC_RZ_NEW];
+    double rr = hsc[SC_RR];
     double bnorm = std::sqrt(bb);
     if (bnorm == 0.0) bnorm = 1.0;
     int64_t it = 0;
@@ -686,7 +734,7 @@ int gfgpu_pcg_solve(const gfgpu_verlet_desc* d, const double* diag, double* x, d
                 rc = check_cuda(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "capture");
             if (rc == GFGPU_OK) {
                 int crc = GFGPU_OK;
-                for (int64_t k = 0; k < nb && crc == GFGPU_OK; ++k) crc = pcg_iteration(d, w, x, n, cs);
+                for (int64_t k = 0; k < nb && crc == GFGPU_OK; ++k) crc = pcg_iteration(d, w, x, n, k == nb - 1, cs);
                 cudaError_t e = cudaStreamEndCapture(cs, &graph);
                 rc = crc != GFGPU_OK ? crc : check_cuda(e, "cudaStreamEndCapture");
                 if (rc == GFGPU_OK)
@@ -702,7 +750,7 @@ int gfgpu_pcg_solve(const gfgpu_verlet_desc* d, const double* diag, double* x, d
             rc = check_cuda(cudaGraphLaunch(exec, s), "cudaGraphLaunch");
         }
         else {
-            for (int64_t k = 0; k < nb && rc == GFGPU_OK; ++k) rc = pcg_iteration(d, w, x, n, s);
+            for (int64_t k = 0; k < nb && rc == GFGPU_OK; ++k) rc = pcg_iteration(d, w, x, n, k == nb - 1, s);
         }
         if (rc != GFGPU_OK) {
             release();
@@ -732,7 +780,7 @@ int gfgpu_pcg_solve(const gfgpu_verlet_desc* d, const double* diag, double* x, d
     if ((rc = gfgpu_internal_element_forces(d, x, w.fe, s)) != GFGPU_OK) return fail_out(rc);
     k_pcg_residual<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
                                                nullptr, w.minv, n, w.r, w.z, nullptr, w.partial, reg_grid(d));
-    k_reduce<<<1, 1024, 0, s>>>(w.partial + kRedBlocks, 1, w.sc, SC_RR);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), 1, w.sc, SC_RR);
     cudaMemcpyAsync(hsc, w.sc, SC_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s);
     if ((rc = check_cuda(cudaStreamSynchronize(s), "pcg final residual")) != GFGPU_OK)
         return fail_out(rc);
@@ -753,20 +801,20 @@ int gfgpu_pcg_begin(const gfgpu_verlet_desc* d, const double* diag, const double
     cudaStream_t s = S(stream);
     PcgWs w = carve(d, workspace);
     int64_t n = d->nnode * d->ndim;
-    const unsigned gb = kRedBlocks;
+    const unsigned gb = red_blocks(n);
     k_inv_free<<<grid_for(n), kBlock, 0, s>>>(d->part, d->nnu, diag, n, w.minv);
     // b = rhs_u - (A x_p)_u
     k_keep_prescribed<<<grid_for(n), kBlock, 0, s>>>(d->part, d->nnu, x, n, w.p);
     GF_TRY(gfgpu_internal_element_forces(d, w.p, w.fe, s));
     k_pcg_residual<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
                                                rhs, w.minv, n, w.bvec, w.z, nullptr, w.partial, reg_grid(d));
-    k_reduce<<<1, 1024, 0, s>>>(w.partial + kRedBlocks, 1, w.sc, SC_BB);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), 1, w.sc, SC_BB);
     // r = rhs_u - (A x)_u, z = M^-1 r, p = z
     GF_TRY(gfgpu_internal_element_forces(d, x, w.fe, s));
     k_pcg_residual<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
                                                rhs, w.minv, n, w.r, w.z, w.p, w.partial, reg_grid(d));
-    k_reduce<<<1, 1024, 0, s>>>(w.partial, 2, w.sc, SC_RZ); // SC_RZ = r.z, SC_RZ_NEW = r.r
-    k_reduce<<<1, 1024, 0, s>>>(w.partial + kRedBlocks, 1, w.sc, SC_RR);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial, static_cast<int>(gb), 1, w.sc, SC_RZ_NEW);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), 1, w.sc, SC_RR);
     if (d->pcg_pair && d->nne == 8) k_pcg_split<<<grid_for(n), kBlock, 0, s>>>(w.p, n, w.pp);
     return check_launch("pcg_begin");
 }
@@ -779,7 +827,7 @@ int gfgpu_pcg_iterate(const gfgpu_verlet_desc* d, int64_t niter, double* x, void
     cudaStream_t s = S(stream);
     PcgWs w = carve(d, workspace);
     int64_t n = d->nnode * d->ndim;
-    for (int64_t k = 0; k < niter; ++k) GF_TRY(pcg_iteration(d, w, x, n, s));
+    for (int64_t k = 0; k < niter; ++k) GF_TRY(pcg_iteration(d, w, x, n, k == niter - 1, s));
     return check_launch("pcg_iterate");
 }
 
