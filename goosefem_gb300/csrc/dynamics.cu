@@ -134,11 +134,12 @@ k_elem_force_general_strict(const int32_t* __restrict__ conn, const double* __re
 // distorted Hex8 elements 345 -> 265 us.
 template <int NNE, int ND>
 __global__ void __launch_bounds__(128)
-k_elem_force_general(const int32_t* __restrict__ conn, const double* __restrict__ u,
+k_elem_force_general(const int32_t* __restrict__ conn, const double* u,
                      const double* __restrict__ dNx, const double* __restrict__ vol,
                      const double* __restrict__ Km, const double* __restrict__ Gm, int64_t nelem,
                      int nip, double* __restrict__ fe)
 {
+    pdl_wait();
     GF_FOR(e, nelem)
     {
         double ue[NNE * ND];
@@ -146,7 +147,7 @@ k_elem_force_general(const int32_t* __restrict__ conn, const double* __restrict_
         for (int m = 0; m < NNE; ++m) {
             const int64_t n = __ldg(conn + e * NNE + m);
 #pragma unroll
-            for (int i = 0; i < ND; ++i) ue[m * ND + i] = __ldg(u + n * ND + i);
+            for (int i = 0; i < ND; ++i) ue[m * ND + i] = u[n * ND + i];
         }
         const double G = __ldg(Gm + e), G2 = G + G, lam = fma(-2.0 / 3.0, G, __ldg(Km + e));
         double f[NNE * ND];
@@ -215,17 +216,17 @@ struct Quad4Uniform {
 //   H_0 = (hx2 (lam + 2G) + hy2 G) A3_x,  H_1 = (hx2 G + hy2 (lam + 2G)) A3_y,
 // sigma_bar the plane-strain stress of the mean strain, lam = K - 2G/3.
 __device__ __forceinline__ void quad4_uniform_elem(int64_t e, const int32_t* __restrict__ conn,
-                                                   const double* __restrict__ u,
+                                                   const double* u,
                                                    const double* __restrict__ Km,
                                                    const double* __restrict__ Gm,
                                                    const Quad4Uniform& c, double* __restrict__ fe)
 {
     {
         int4 cn = __ldg(reinterpret_cast<const int4*>(conn) + e);
-        double2 u0 = __ldg(reinterpret_cast<const double2*>(u) + cn.x);
-        double2 u1 = __ldg(reinterpret_cast<const double2*>(u) + cn.y);
-        double2 u2 = __ldg(reinterpret_cast<const double2*>(u) + cn.z);
-        double2 u3 = __ldg(reinterpret_cast<const double2*>(u) + cn.w);
+        double2 u0 = reinterpret_cast<const double2*>(u)[cn.x];
+        double2 u1 = reinterpret_cast<const double2*>(u)[cn.y];
+        double2 u2 = reinterpret_cast<const double2*>(u)[cn.z];
+        double2 u3 = reinterpret_cast<const double2*>(u)[cn.w];
         double K = __ldg(Km + e), G = __ldg(Gm + e);
         // Walsh combinations
         double px = u2.x - u0.x, qx = u1.x - u3.x;
@@ -256,10 +257,11 @@ __device__ __forceinline__ void quad4_uniform_elem(int64_t e, const int32_t* __r
 }
 
 __global__ void __launch_bounds__(256)
-k_elem_force_quad4_uniform(const int32_t* __restrict__ conn, const double* __restrict__ u,
+k_elem_force_quad4_uniform(const int32_t* __restrict__ conn, const double* u,
                            const double* __restrict__ Km, const double* __restrict__ Gm,
                            int64_t nelem, Quad4Uniform c, double* __restrict__ fe)
 {
+    pdl_wait();
     GF_FOR(e, nelem) quad4_uniform_elem(e, conn, u, Km, Gm, c, fe);
 }
 
@@ -286,7 +288,7 @@ template <bool CG>
 __device__ __forceinline__ double2 ld2(const double2* p)
 {
     if constexpr (CG) return __ldcg(p);
-    else return __ldg(p);
+    else return *p;
 }
 
 template <bool CG>
@@ -318,9 +320,10 @@ __device__ __forceinline__ void quad4_square_elem(int64_t e, const int32_t* __re
 }
 
 __global__ void __launch_bounds__(256, 4)
-k_elem_force_quad4_square(const int32_t* __restrict__ conn, const double* __restrict__ u,
+k_elem_force_quad4_square(const int32_t* __restrict__ conn, const double* u,
                           const double* __restrict__ coef, int64_t nelem, double* __restrict__ fe)
 {
+    pdl_wait();
     GF_FOR(e, nelem) quad4_square_elem<false>(e, conn, u, coef, fe);
 }
 
@@ -376,12 +379,13 @@ __device__ __forceinline__ void fwht8(double (&v)[8])
 }
 
 __global__ void __launch_bounds__(128)
-k_elem_force_hex8_uniform(const int32_t* __restrict__ conn, const double* __restrict__ u,
+k_elem_force_hex8_uniform(const int32_t* __restrict__ conn, const double* u,
                           const double* __restrict__ Km, const double* __restrict__ Gm,
                           int64_t nelem, Hex8Uniform c, double* __restrict__ fe)
 {
     // GooseFEM node m -> binary position
     constexpr int pos[8] = {0, 1, 3, 2, 4, 5, 7, 6};
+    pdl_wait();
     GF_FOR(e, nelem)
     {
         double H[3][8];
@@ -391,9 +395,9 @@ k_elem_force_hex8_uniform(const int32_t* __restrict__ conn, const double* __rest
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
             const double* un = u + static_cast<int64_t>(nodes[m]) * 3;
-            H[0][pos[m]] = __ldg(un);
-            H[1][pos[m]] = __ldg(un + 1);
-            H[2][pos[m]] = __ldg(un + 2);
+            H[0][pos[m]] = un[0];
+            H[1][pos[m]] = un[1];
+            H[2][pos[m]] = un[2];
         }
         fwht8(H[0]);
         fwht8(H[1]);
@@ -533,10 +537,11 @@ __device__ __forceinline__ void fwht8_nomean(double (&v)[8])
 // solvers' Regular-mesh gather reads it so); else fe[e * 24 + m * 3 + j].
 template <bool SOA>
 __global__ void __launch_bounds__(128)
-k_elem_force_hex8_cube(const int32_t* __restrict__ conn, const double* __restrict__ u,
+k_elem_force_hex8_cube(const int32_t* __restrict__ conn, const double* u,
                        const double* __restrict__ coef, int64_t nelem, double* __restrict__ fe)
 {
     constexpr int pos[8] = {0, 1, 3, 2, 4, 5, 7, 6};
+    pdl_wait();
     GF_FOR(e, nelem)
     {
         double H[3][8];
@@ -546,9 +551,9 @@ k_elem_force_hex8_cube(const int32_t* __restrict__ conn, const double* __restric
 #pragma unroll
         for (int m = 0; m < 8; ++m) {
             const double* un = u + static_cast<int64_t>(nodes[m]) * 3;
-            H[0][pos[m]] = __ldg(un);
-            H[1][pos[m]] = __ldg(un + 1);
-            H[2][pos[m]] = __ldg(un + 2);
+            H[0][pos[m]] = un[0];
+            H[1][pos[m]] = un[1];
+            H[2][pos[m]] = un[2];
         }
         fwht8_nomean(H[0]);
         fwht8_nomean(H[1]);
@@ -689,7 +694,7 @@ template <bool CG>
 __device__ __forceinline__ double ld1(const double* p)
 {
     if constexpr (CG) return __ldcg(p);
-    else return __ldg(p);
+    else return *p;
 }
 
 // Fast node update (reassociated, not bit-exact with the reference order): the solve
@@ -735,10 +740,11 @@ verlet_node_fast_one(int64_t t, const int32_t* __restrict__ dofs, const int32_t*
 __global__ void __launch_bounds__(256)
 k_verlet_node_fast(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr,
                    const int32_t* __restrict__ idx, const int32_t* __restrict__ part, int64_t nnu,
-                   const double* __restrict__ inv, const double* __restrict__ fe,
+                   const double* __restrict__ inv, const double* fe,
                    const double* __restrict__ fext, int64_t n, VerletCoef k, int advance,
                    double* __restrict__ u, double* __restrict__ v, double* __restrict__ a)
 {
+    pdl_wait();
     GF_FOR(t, n)
     verlet_node_fast_one<false>(t, dofs, ptr, idx, part, nnu, inv, fe, fext, k, advance, u, v, a);
 }
@@ -796,7 +802,7 @@ struct MassClassTab {
 __global__ void __launch_bounds__(256)
 k_verlet_node_cls(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr,
                   const int32_t* __restrict__ idx, const int4* __restrict__ ell, const uint8_t* __restrict__ mclass,
-                  MassClassTab tab, const double* __restrict__ fe, const double* __restrict__ fext,
+                  MassClassTab tab, const double* fe, const double* __restrict__ fext,
                   int64_t n, VerletCoef k, int advance, double* __restrict__ u,
                   double* __restrict__ v, double* __restrict__ a)
 {
@@ -809,6 +815,7 @@ k_verlet_node_cls(const int32_t* __restrict__ dofs, const int32_t* __restrict__ 
         sm[3][c] = tab.c2[c];
         sm[4][c] = tab.c3[c];
     }
+    pdl_wait();
     __syncthreads();
     GF_FOR(t, n)
     {
@@ -816,16 +823,16 @@ k_verlet_node_cls(const int32_t* __restrict__ dofs, const int32_t* __restrict__ 
         if (ell) {
             // the same entries in the same order, one 16-byte load instead of dofs -> ptr -> idx
             const int4 q = __ldg(ell + t);
-            fint = q.x >= 0 ? __ldg(fe + q.x) : 0.0;
-            if (q.y >= 0) fint += __ldg(fe + q.y);
-            if (q.z >= 0) fint += __ldg(fe + q.z);
-            if (q.w >= 0) fint += __ldg(fe + q.w);
+            fint = q.x >= 0 ? fe[q.x] : 0.0;
+            if (q.y >= 0) fint += fe[q.y];
+            if (q.z >= 0) fint += fe[q.z];
+            if (q.w >= 0) fint += fe[q.w];
         }
         else {
             int32_t d = __ldg(dofs + t);
             int32_t b = __ldg(ptr + d), en = __ldg(ptr + d + 1);
-            fint = en > b ? __ldg(fe + __ldg(idx + b)) : 0.0;
-            for (int32_t j = b + 1; j < en; ++j) fint += __ldg(fe + __ldg(idx + j));
+            fint = en > b ? fe[__ldg(idx + b)] : 0.0;
+            for (int32_t j = b + 1; j < en; ++j) fint += fe[__ldg(idx + j)];
         }
         int c = __ldg(mclass + t);
         double vn = v[t], an = a[t];
@@ -852,7 +859,7 @@ k_verlet_node_cls(const int32_t* __restrict__ dofs, const int32_t* __restrict__ 
 // that order: ascending element index, the order of the dof CSR.
 __global__ void __launch_bounds__(256)
 k_verlet_node_cls_regular(int64_t nx, int64_t ny, const uint8_t* __restrict__ mclass,
-                          MassClassTab tab, const double* __restrict__ fe,
+                          MassClassTab tab, const double* fe,
                           const double* __restrict__ fext, VerletCoef k, int advance,
                           double* __restrict__ u, double* __restrict__ v, double* __restrict__ a)
 {
@@ -865,6 +872,7 @@ k_verlet_node_cls_regular(int64_t nx, int64_t ny, const uint8_t* __restrict__ mc
         sm[3][c] = tab.c2[c];
         sm[4][c] = tab.c3[c];
     }
+    pdl_wait();
     __syncthreads();
     const int64_t W = nx + 1, nnode = W * (ny + 1);
     const double2* f2 = reinterpret_cast<const double2*>(fe);
@@ -875,7 +883,7 @@ k_verlet_node_cls_regular(int64_t nx, int64_t ny, const uint8_t* __restrict__ mc
         bool first = true;
         auto take = [&](int64_t ey, int64_t ex, int m) {
             if (ey < 0 || ey >= ny || ex < 0 || ex >= nx) return;
-            double2 g = __ldg(f2 + (ey * nx + ex) * 4 + m);
+            double2 g = f2[(ey * nx + ex) * 4 + m];
             if (first) {
                 fx = g.x;
                 fy = g.y;
@@ -963,7 +971,7 @@ template <bool S>
 __global__ void __launch_bounds__(256)
 k_verlet_node(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr,
               const int32_t* __restrict__ idx, const int32_t* __restrict__ part, int64_t nnu,
-              const double* __restrict__ inv, const double* __restrict__ fe,
+              const double* __restrict__ inv, const double* fe,
               const double* __restrict__ fext, int64_t n, VerletCoef k, int advance,
               double* __restrict__ u, double* __restrict__ v, double* __restrict__ a)
 {
@@ -1153,51 +1161,38 @@ static VerletCoef verlet_coefficients(const gfgpu_verlet_desc* d)
     return k;
 }
 
-static int launch_elem(const gfgpu_verlet_desc* d, const double* u, double* fe, cudaStream_t s)
+// dependent: launched as a dependent of the kernel before it (pdl_wait's rule), for the increments
+static int launch_elem(const gfgpu_verlet_desc* d, const double* u, double* fe, cudaStream_t s, bool dependent = false)
 {
     if (d->nelem == 0) return GFGPU_OK;
+    const Shape l = spread(d->nelem, 256), h = spread(d->nelem, 128);
+    auto run = [&](auto kernel, const Shape& shape, auto... args) -> int {
+        if (dependent) return launch_dependent(kernel, shape, s, args...);
+        kernel<<<shape.grid, shape.block, 0, s>>>(args...);
+        return check_launch("verlet element kernel");
+    };
     if (d->uniform && d->nne == 4 && d->coef) {
-        if (variant_elem() == 1)
+        if (variant_elem() == 1) {
             k_elem_force_quad4_square_x2<<<grid_for((d->nelem + 1) / 2), 256, 0, s>>>(
                 d->conn, u, d->coef, d->nelem, fe);
-        else
-            k_elem_force_quad4_square<<<grid_for(d->nelem), 256, 0, s>>>(d->conn, u, d->coef,
-                                                                         d->nelem, fe);
-    }
-    else if (d->uniform && d->nne == 4) {
-        Quad4Uniform c = quad4_uniform_constants(d);
-        k_elem_force_quad4_uniform<<<grid_for(d->nelem), 256, 0, s>>>(d->conn, u, d->K, d->G,
-                                                                      d->nelem, c, fe);
-    }
-    else if (d->uniform && d->coef) {
-        k_elem_force_hex8_cube<false><<<grid_for(d->nelem, 128), 128, 0, s>>>(d->conn, u, d->coef,
-                                                                              d->nelem, fe);
-    }
-    else if (d->uniform) {
-        Hex8Uniform c = hex8_uniform_constants(d);
-        k_elem_force_hex8_uniform<<<grid_for(d->nelem, 128), 128, 0, s>>>(d->conn, u, d->K, d->G,
-                                                                          d->nelem, c, fe);
-    }
-    else {
-        unsigned g = grid_for(d->nelem, 128);
-        if (d->nne == 4) {
-            if (strict_mode())
-                k_elem_force_general_strict<4, 2><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
-                                                                   d->G, d->nelem, d->nip, fe);
-            else
-                k_elem_force_general<4, 2><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
-                                                                    d->G, d->nelem, d->nip, fe);
+            return check_launch("verlet element kernel");
         }
-        else {
-            if (strict_mode())
-                k_elem_force_general_strict<8, 3><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
-                                                                   d->G, d->nelem, d->nip, fe);
-            else
-                k_elem_force_general<8, 3><<<g, 128, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K,
-                                                                    d->G, d->nelem, d->nip, fe);
-        }
+        return run(k_elem_force_quad4_square, l, d->conn, u, d->coef, d->nelem, fe);
     }
-    return check_launch("verlet element kernel");
+    if (d->uniform && d->nne == 4)
+        return run(k_elem_force_quad4_uniform, l, d->conn, u, d->K, d->G, d->nelem, quad4_uniform_constants(d), fe);
+    if (d->uniform && d->coef) return run(k_elem_force_hex8_cube<false>, h, d->conn, u, d->coef, d->nelem, fe);
+    if (d->uniform)
+        return run(k_elem_force_hex8_uniform, h, d->conn, u, d->K, d->G, d->nelem, hex8_uniform_constants(d), fe);
+    if (strict_mode()) {
+        auto strict = [&](auto kernel) {
+            kernel<<<h.grid, h.block, 0, s>>>(d->conn, u, d->dNx, d->vol, d->K, d->G, d->nelem, d->nip, fe);
+            return check_launch("verlet element kernel");
+        };
+        return d->nne == 4 ? strict(k_elem_force_general_strict<4, 2>) : strict(k_elem_force_general_strict<8, 3>);
+    }
+    return d->nne == 4 ? run(k_elem_force_general<4, 2>, h, d->conn, u, d->dNx, d->vol, d->K, d->G, d->nelem, d->nip, fe)
+                       : run(k_elem_force_general<8, 3>, h, d->conn, u, d->dNx, d->vol, d->K, d->G, d->nelem, d->nip, fe);
 }
 
 // the square Quad4 element forces in pair arithmetic, FP64 in and out (verlet_pair.cu)
@@ -1220,7 +1215,7 @@ static bool mixed_arithmetic(const gfgpu_verlet_desc* d)
 static int launch_elem_step(const gfgpu_verlet_desc* d, const double* u, double* fe, cudaStream_t s)
 {
     if (mixed_arithmetic(d)) return gfgpu_internal_pair_element_forces_f64(d, u, fe, s);
-    return launch_elem(d, u, fe, s);
+    return launch_elem(d, u, fe, s, true);
 }
 
 // float-float path of the Regular square Quad4 mesh (verlet_pair.cu)
@@ -1245,8 +1240,8 @@ int gfgpu_internal_element_forces(const gfgpu_verlet_desc* d, const double* u, d
 {
     GF_TRY(check_operator(d));
     if (reg_grid(d).soa && d->nelem > 0) {
-        k_elem_force_hex8_cube<true><<<grid_for(d->nelem, 128), 128, 0, s>>>(d->conn, u, d->coef,
-                                                                             d->nelem, fe);
+        const Shape h = spread(d->nelem, 128);
+        k_elem_force_hex8_cube<true><<<h.grid, h.block, 0, s>>>(d->conn, u, d->coef, d->nelem, fe);
         return check_launch("cube element kernel");
     }
     return launch_elem(d, u, fe, s);
@@ -1277,24 +1272,25 @@ static int launch_node(const gfgpu_verlet_desc* d, const MassClassTab& tab, cons
                        const double* fe, int adv, double* u, double* v, double* a, cudaStream_t s)
 {
     const int64_t n = d->nnode * d->ndim;
-    const unsigned gn = grid_for(n);
+    const Shape l = spread(n);
     const bool cls = d->mclass && d->mclass_inv && d->ncls > 0;
     if (strict_mode())
-        k_verlet_node<true><<<gn, kBlock, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu,
+        k_verlet_node<true><<<l.grid, l.block, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu,
                                                   d->inv, fe, d->fext, n, k, adv, u, v, a);
-    else if (cls && d->reg_nx > 0 && d->reg_nz == 0 && d->nne == 4)
-        k_verlet_node_cls_regular<<<grid_for(d->nnode), kBlock, 0, s>>>(
-            d->reg_nx, d->reg_ny, d->mclass, tab, fe, d->fext, k, adv, u, v, a);
+    else if (cls && d->reg_nx > 0 && d->reg_nz == 0 && d->nne == 4) {
+        return launch_dependent(k_verlet_node_cls_regular, spread(d->nnode), s, d->reg_nx, d->reg_ny, d->mclass, tab,
+                                fe, d->fext, k, adv, u, v, a);
+    }
     else if (cls)
-        k_verlet_node_cls<<<gn, kBlock, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx,
-                                                reinterpret_cast<const int4*>(d->ell), d->mclass, tab,
-                                                fe, d->fext, n, k, adv, u, v, a);
+        return launch_dependent(k_verlet_node_cls, l, s, d->dofs, d->csr_ptr, d->csr_idx,
+                                reinterpret_cast<const int4*>(d->ell), d->mclass, tab, fe, d->fext, n, k, adv, u, v,
+                                a);
     else if (variant_node() == 1)
         k_verlet_node_fast_x2<<<grid_for((n + 1) / 2), kBlock, 0, s>>>(
             d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, d->inv, fe, d->fext, n, k, adv, u, v, a);
     else
-        k_verlet_node_fast<<<gn, kBlock, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu,
-                                                 d->inv, fe, d->fext, n, k, adv, u, v, a);
+        return launch_dependent(k_verlet_node_fast, l, s, d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, d->inv, fe,
+                                d->fext, n, k, adv, u, v, a);
     return check_launch("verlet node kernel");
 }
 
@@ -1306,13 +1302,13 @@ static int run_increments(const gfgpu_verlet_desc* d, double* u, double* v, doub
 {
     const VerletCoef k = verlet_coefficients(d);
     const int64_t n = d->nnode * d->ndim;
-    const unsigned gn = grid_for(n);
+    const Shape l = spread(n);
     MassClassTab tab;
     GF_TRY(mass_class_tab(d, k, &tab));
     if (strict_mode())
-        k_predict<true><<<gn, kBlock, 0, s>>>(u, v, a, n, k);
+        k_predict<true><<<l.grid, l.block, 0, s>>>(u, v, a, n, k);
     else
-        k_predict<false><<<gn, kBlock, 0, s>>>(u, v, a, n, k);
+        k_predict<false><<<l.grid, l.block, 0, s>>>(u, v, a, n, k);
     GF_TRY(check_launch("verlet predict"));
     // mixed arithmetic with lumped-mass classes: the element forces stay pairs and the node kernel
     // takes the velocity estimates on pairs (4 FP64 instructions per free dof instead of 10)

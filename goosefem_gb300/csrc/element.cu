@@ -704,13 +704,13 @@ static int grad(const double* dNx, const double* elemvec, int64_t nelem, int32_t
     GF_REQUIRE(!too_big(nelem * nip * 24), "too many elements");
     GF_REQUIRE(aligned16(dNx) && aligned16(elemvec), "dNx and elemvec must be 16-byte aligned");
     if (nelem == 0) return GFGPU_OK;
-    unsigned g = grid_for(nelem * nip);
+    const Shape l = spread(nelem * nip);
     if (planar)
-        DISPATCH_S(k_grad<kS, 4, 2, MODE, 3><<<g, kBlock, 0, S(stream)>>>(dNx, elemvec, nelem, nip, qtensor));
+        DISPATCH_S(k_grad<kS, 4, 2, MODE, 3><<<l.grid, l.block, 0, S(stream)>>>(dNx, elemvec, nelem, nip, qtensor));
     else if (nd == 2)
-        DISPATCH_S(k_grad<kS, 4, 2, MODE><<<g, kBlock, 0, S(stream)>>>(dNx, elemvec, nelem, nip, qtensor));
+        DISPATCH_S(k_grad<kS, 4, 2, MODE><<<l.grid, l.block, 0, S(stream)>>>(dNx, elemvec, nelem, nip, qtensor));
     else
-        DISPATCH_S(k_grad<kS, 8, 3, MODE><<<g, kBlock, 0, S(stream)>>>(dNx, elemvec, nelem, nip, qtensor));
+        DISPATCH_S(k_grad<kS, 8, 3, MODE><<<l.grid, l.block, 0, S(stream)>>>(dNx, elemvec, nelem, nip, qtensor));
     return check_launch("grad_n_vector");
 }
 
@@ -846,13 +846,13 @@ int gfgpu_int_grad_n_dot_tensor2_dv(const double* dNx, const double* vol, const 
     GF_REQUIRE(!too_big(nelem * nip * 24), "too many elements");
     GF_REQUIRE(aligned16(dNx) && aligned16(qtensor), "dNx and qtensor must be 16-byte aligned");
     if (nelem == 0) return GFGPU_OK;
-    unsigned g = grid_for(nelem, 128);
+    const Shape l = spread(nelem, 128);
     if (ndim == 2)
-        DISPATCH_S(k_int_grad_tensor2<kS, 4, 2><<<g, 128, 0, S(stream)>>>(dNx, vol, qtensor, nelem,
-                                                                          nip, elemvec));
+        DISPATCH_S(k_int_grad_tensor2<kS, 4, 2><<<l.grid, l.block, 0, S(stream)>>>(dNx, vol, qtensor, nelem,
+                                                                                   nip, elemvec));
     else
-        DISPATCH_S(k_int_grad_tensor2<kS, 8, 3><<<g, 128, 0, S(stream)>>>(dNx, vol, qtensor, nelem,
-                                                                          nip, elemvec));
+        DISPATCH_S(k_int_grad_tensor2<kS, 8, 3><<<l.grid, l.block, 0, S(stream)>>>(dNx, vol, qtensor, nelem,
+                                                                                   nip, elemvec));
     return check_launch("int_grad_n_dot_tensor2_dv");
 }
 

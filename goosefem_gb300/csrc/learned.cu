@@ -325,16 +325,6 @@ __global__ void k_nn_wprep_first(const __nv_bfloat16* __restrict__ W, __nv_bfloa
 // and weight load then overlap this layer's tail) and waits for the previous layer's grid to
 // complete before it touches the previous layer's output or writes anything. Both are no-ops for
 // a kernel launched without the attribute.
-__device__ __forceinline__ void pdl_launch_dependents()
-{
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-}
-
-__device__ __forceinline__ void pdl_wait()
-{
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-}
-
 // Channel-planar activations of the tcgen05 layers: [4][H][Wp][8] BF16, pixel (y, x) stored at
 // row position x + kPlanarPad, Wp = planar_row(W) (a multiple of 8 pixels); the pad pixels are
 // zero. Rows of 128-byte groups of 8 pixels make a halo tile one TMA box per plane with

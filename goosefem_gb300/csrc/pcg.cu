@@ -634,7 +634,8 @@ static int pcg_iteration(const gfgpu_verlet_desc* d, const PcgWs& w, double* x, 
     const bool pair = d->pcg_pair != nullptr && d->nne == 8;
     unsigned gg; // blocks and partials of the gather
     if (pair) {
-        k_elem_force_hex8_cube_pair<<<grid_for(d->nelem, 128), 128, 0, s>>>(
+        const Shape h = spread(d->nelem, 128);
+        k_elem_force_hex8_cube_pair<<<h.grid, h.block, 0, s>>>(
             w.pp, reinterpret_cast<const float4*>(d->pcg_pair), cube_pair(d), d->nelem,
             reinterpret_cast<float2*>(w.fe));
         gg = red_blocks(d->nnode);

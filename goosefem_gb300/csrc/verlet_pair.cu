@@ -70,14 +70,14 @@ __device__ __forceinline__ float4 ppack(ffv x, ffv y) { return make_float4(x.h, 
 
 // pair sum of a nodevec entry's element forces through the gather table (the CSR's entries and
 // order; -1 pads): the first term assigned, the others added, as the CSR loop does
-__device__ __forceinline__ ffv gather_ell_pair(const int4* __restrict__ ell, const float2* __restrict__ fe,
+__device__ __forceinline__ ffv gather_ell_pair(const int4* __restrict__ ell, const float2* fe,
                                                int64_t t)
 {
     const int4 q = __ldg(ell + t);
-    ffv f = q.x >= 0 ? pf(__ldg(fe + q.x)) : ff_make(0.f, 0.f);
-    if (q.y >= 0) f = ff_add(f, pf(__ldg(fe + q.y)));
-    if (q.z >= 0) f = ff_add(f, pf(__ldg(fe + q.z)));
-    if (q.w >= 0) f = ff_add(f, pf(__ldg(fe + q.w)));
+    ffv f = q.x >= 0 ? pf(fe[q.x]) : ff_make(0.f, 0.f);
+    if (q.y >= 0) f = ff_add(f, pf(fe[q.y]));
+    if (q.z >= 0) f = ff_add(f, pf(fe[q.z]));
+    if (q.w >= 0) f = ff_add(f, pf(fe[q.w]));
     return f;
 }
 
@@ -629,14 +629,15 @@ __global__ void k_pair_join(const float2* __restrict__ in, int64_t n, double* __
 }
 
 __global__ void __launch_bounds__(256)
-k_pair_elem_square(const int32_t* __restrict__ conn, const float4* __restrict__ u, const float4* __restrict__ cLN,
+k_pair_elem_square(const int32_t* __restrict__ conn, const float4* u, const float4* __restrict__ cLN,
                    const float2* __restrict__ cH, int64_t nelem, float4* __restrict__ fe)
 {
+    pdl_wait();
     GF_FOR(e, nelem)
     {
         const int4 cn = __ldg(reinterpret_cast<const int4*>(conn) + e);
         float4 S, D, H;
-        const float4 q0 = __ldg(u + cn.x), q1 = __ldg(u + cn.y), q2 = __ldg(u + cn.z), q3 = __ldg(u + cn.w);
+        const float4 q0 = u[cn.x], q1 = u[cn.y], q2 = u[cn.z], q3 = u[cn.w];
         const float4 cln = __ldg(cLN + e);
         pair_element(lo2(q0), hi2(q0), lo2(q1), hi2(q1), lo2(q2), hi2(q2), lo2(q3), hi2(q3), lo2(cln), hi2(cln),
                      pf(__ldg(cH + e)), S, D, H);
@@ -660,14 +661,15 @@ k_pair_elem_square(const int32_t* __restrict__ conn, const float4* __restrict__ 
 // per value like the FP64 layout; the mixed node kernel gathers them).
 template <bool PAIR_OUT>
 __global__ void __launch_bounds__(256)
-k_pair_elem_square_f64(const int32_t* __restrict__ conn, const double2* __restrict__ u,
+k_pair_elem_square_f64(const int32_t* __restrict__ conn, const double2* u,
                        const float4* __restrict__ cLN, const float2* __restrict__ cH, int64_t nelem,
                        double2* __restrict__ fe)
 {
+    pdl_wait();
     GF_FOR(e, nelem)
     {
         const int4 cn = __ldg(reinterpret_cast<const int4*>(conn) + e);
-        const double2 q0 = __ldg(u + cn.x), q1 = __ldg(u + cn.y), q2 = __ldg(u + cn.z), q3 = __ldg(u + cn.w);
+        const double2 q0 = u[cn.x], q1 = u[cn.y], q2 = u[cn.z], q3 = u[cn.w];
         const float4 cln = __ldg(cLN + e);
         float4 S, D, H;
         pair_element_diff(ff_from_double(q2.x - q0.x), ff_from_double(q2.y - q0.y), ff_from_double(q1.x - q3.x),
@@ -721,6 +723,7 @@ k_mixed_node(const MixedNodeStep p, const __grid_constant__ PairClassTab tab)
         sc2[c] = tab.c2[c];
         sc3[c] = tab.c3[c];
     }
+    pdl_wait();
     __syncthreads();
     GF_FOR(t, p.n)
     {
@@ -731,7 +734,7 @@ k_mixed_node(const MixedNodeStep p, const __grid_constant__ PairClassTab tab)
             const uint32_t iy = node / W, ix = node - iy * W;
             bool first = true;
             auto add = [&](uint32_t e, uint32_t m) {
-                const ffv g = pf(__ldg(p.fe + (e * 4u + m) * 2u + i));
+                const ffv g = pf(p.fe[(e * 4u + m) * 2u + i]);
                 f = first ? g : ff_add(f, g);
                 first = false;
             };
@@ -747,7 +750,7 @@ k_mixed_node(const MixedNodeStep p, const __grid_constant__ PairClassTab tab)
             const int32_t d = __ldg(p.dofs + t);
             const int32_t b = __ldg(p.ptr + d), en = __ldg(p.ptr + d + 1);
             for (int32_t j = b; j < en; ++j) {
-                const ffv g = pf(__ldg(p.fe + __ldg(p.idx + j)));
+                const ffv g = pf(p.fe[__ldg(p.idx + j)]);
                 f = j == b ? g : ff_add(f, g);
             }
         }
@@ -775,13 +778,14 @@ k_mixed_node(const MixedNodeStep p, const __grid_constant__ PairClassTab tab)
 }
 
 __global__ void __launch_bounds__(128)
-k_pair_elem_stiff(const int32_t* __restrict__ conn, const float4* __restrict__ u, const float2* __restrict__ Ke,
+k_pair_elem_stiff(const int32_t* __restrict__ conn, const float4* u, const float2* __restrict__ Ke,
                   int64_t nelem, float4* __restrict__ fe)
 {
+    pdl_wait();
     GF_FOR(e, nelem)
     {
         const int4 cn = __ldg(reinterpret_cast<const int4*>(conn) + e);
-        const float4 q[4] = {__ldg(u + cn.x), __ldg(u + cn.y), __ldg(u + cn.z), __ldg(u + cn.w)};
+        const float4 q[4] = {u[cn.x], u[cn.y], u[cn.z], u[cn.w]};
         ffv f[8];
         bool first[8];
 #pragma unroll
@@ -842,6 +846,7 @@ k_pair_node_csr(const PairCsrStep p, const __grid_constant__ PairClassTab tab)
         sc2[c] = tab.c2[c];
         sc3[c] = tab.c3[c];
     }
+    pdl_wait();
     __syncthreads();
     const ffv dt = pf(p.dt), h = pf(p.h), cc = pf(p.cc);
     GF_FOR(t, p.n)
@@ -855,7 +860,7 @@ k_pair_node_csr(const PairCsrStep p, const __grid_constant__ PairClassTab tab)
             const uint32_t iy = node / W, ix = node - iy * W;
             bool first = true;
             auto add = [&](uint32_t e, uint32_t m) {
-                const ffv g = pf(__ldg(p.fe + (e * 4u + m) * 2u + i));
+                const ffv g = pf(p.fe[(e * 4u + m) * 2u + i]);
                 f = first ? g : ff_add(f, g);
                 first = false;
             };
@@ -871,12 +876,12 @@ k_pair_node_csr(const PairCsrStep p, const __grid_constant__ PairClassTab tab)
             const int32_t d = __ldg(p.dofs + t);
             const int32_t b = __ldg(p.ptr + d), en = __ldg(p.ptr + d + 1);
             for (int32_t j = b; j < en; ++j) {
-                const ffv g = pf(__ldg(p.fe + __ldg(p.idx + j)));
+                const ffv g = pf(p.fe[__ldg(p.idx + j)]);
                 f = j == b ? g : ff_add(f, g);
             }
         }
         f = ff_norm(f);
-        const ffv fx = p.fext ? pf(__ldg(p.fext + t)) : ff_make(0.f, 0.f);
+        const ffv fx = p.fext ? pf(p.fext[t]) : ff_make(0.f, 0.f);
         const ffv vn = pf(p.v[t]), an = pf(p.a[t]);
         ffv vv, aa;
         if (p.mclass) {
@@ -1209,18 +1214,17 @@ static int pair_increments(const gfgpu_verlet_desc* d, int64_t first, int64_t co
         q.h = split_host(h);
         q.cc = split_host(c);
         q.eta = split_host(d->eta);
+        const Shape l = spread(d->nelem, 256), h = spread(d->nelem, 128), r = spread(q.n, 256);
         for (int64_t it = first; it < first + count; ++it) {
             if (d->pair_mode == 2)
-                k_pair_elem_square<<<grid_for(d->nelem), 256, 0, s>>>(
-                    d->conn, ub[0], reinterpret_cast<const float4*>(d->coef_pair),
-                    reinterpret_cast<const float2*>(d->coef_pair + 4 * d->nelem), d->nelem, fe);
+                GF_TRY(launch_dependent(k_pair_elem_square, l, s, d->conn, ub[0],
+                                        reinterpret_cast<const float4*>(d->coef_pair),
+                                        reinterpret_cast<const float2*>(d->coef_pair + 4 * d->nelem), d->nelem, fe));
             else
-                k_pair_elem_stiff<<<grid_for(d->nelem, 128), 128, 0, s>>>(
-                    d->conn, ub[0], reinterpret_cast<const float2*>(d->coef_pair), d->nelem, fe);
-            GF_TRY(check_launch("pair element kernel"));
+                GF_TRY(launch_dependent(k_pair_elem_stiff, h, s, d->conn, ub[0],
+                                        reinterpret_cast<const float2*>(d->coef_pair), d->nelem, fe));
             q.advance = (it + 1 < first + count || advance_last) ? 1 : 0;
-            k_pair_node_csr<<<grid_for(q.n), 256, 0, s>>>(q, tab);
-            GF_TRY(check_launch("pair node kernel"));
+            GF_TRY(launch_dependent(k_pair_node_csr, r, s, q, tab));
         }
         return GFGPU_OK;
     }
@@ -1312,7 +1316,8 @@ int gfgpu_internal_pair_element_forces_f64(const gfgpu_verlet_desc* d, const dou
 {
     if (d->nelem == 0) return GFGPU_OK;
     const float* c = d->pcg_pair;
-    k_pair_elem_square_f64<false><<<grid_for(d->nelem), 256, 0, s>>>(
+    const Shape l = spread(d->nelem, 256);
+    k_pair_elem_square_f64<false><<<l.grid, l.block, 0, s>>>(
         d->conn, reinterpret_cast<const double2*>(u), reinterpret_cast<const float4*>(c),
         reinterpret_cast<const float2*>(c + 4 * d->nelem), d->nelem, reinterpret_cast<double2*>(fe));
     return check_launch("pair element kernel (static operator)");
@@ -1324,10 +1329,10 @@ int gfgpu_internal_mixed_increment(const gfgpu_verlet_desc* d, double* fe, int a
                                    double* a, cudaStream_t s)
 {
     const float* c = d->pcg_pair;
-    k_pair_elem_square_f64<true><<<grid_for(d->nelem), 256, 0, s>>>(
-        d->conn, reinterpret_cast<const double2*>(u), reinterpret_cast<const float4*>(c),
-        reinterpret_cast<const float2*>(c + 4 * d->nelem), d->nelem, reinterpret_cast<double2*>(fe));
-    GF_TRY(check_launch("pair element kernel (mixed)"));
+    GF_TRY(launch_dependent(k_pair_elem_square_f64<true>, spread(d->nelem, 256), s, d->conn,
+                            reinterpret_cast<const double2*>(u), reinterpret_cast<const float4*>(c),
+                            reinterpret_cast<const float2*>(c + 4 * d->nelem), d->nelem,
+                            reinterpret_cast<double2*>(fe)));
     MixedNodeStep q;
     q.dofs = d->dofs;
     q.ptr = d->csr_ptr;
@@ -1346,8 +1351,7 @@ int gfgpu_internal_mixed_increment(const gfgpu_verlet_desc* d, double* fe, int a
     q.h = 0.5 * d->dt;
     q.c = 0.5 * std::pow(d->dt, 2.0);
     q.advance = advance;
-    k_mixed_node<<<grid_for(q.n), 256, 0, s>>>(q, pair_class_tab(d));
-    return check_launch("mixed node kernel");
+    return launch_dependent(k_mixed_node, spread(q.n, 256), s, q, pair_class_tab(d));
 }
 
 // {L, N} [nelem] interleaved pairs, then kH [nelem] (6 floats per element) of a uniform square Quad4
