@@ -79,11 +79,12 @@ __device__ __forceinline__ void pdl_launch_dependents()
 }
 
 template <class... P, class... A>
-inline int launch_dependent(void (*kernel)(P...), Shape shape, cudaStream_t s, A... args)
+inline int launch_dependent(void (*kernel)(P...), Shape shape, cudaStream_t s, size_t smem, const A&... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(shape.grid);
     cfg.blockDim = dim3(static_cast<unsigned>(shape.block));
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -1167,7 +1167,7 @@ static int launch_elem(const gfgpu_verlet_desc* d, const double* u, double* fe, 
     if (d->nelem == 0) return GFGPU_OK;
     const Shape l = spread(d->nelem, 256), h = spread(d->nelem, 128);
     auto run = [&](auto kernel, const Shape& shape, auto... args) -> int {
-        if (dependent) return launch_dependent(kernel, shape, s, args...);
+        if (dependent) return launch_dependent(kernel, shape, s, 0, args...);
         kernel<<<shape.grid, shape.block, 0, s>>>(args...);
         return check_launch("verlet element kernel");
     };
@@ -1278,18 +1278,18 @@ static int launch_node(const gfgpu_verlet_desc* d, const MassClassTab& tab, cons
         k_verlet_node<true><<<l.grid, l.block, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu,
                                                   d->inv, fe, d->fext, n, k, adv, u, v, a);
     else if (cls && d->reg_nx > 0 && d->reg_nz == 0 && d->nne == 4) {
-        return launch_dependent(k_verlet_node_cls_regular, spread(d->nnode), s, d->reg_nx, d->reg_ny, d->mclass, tab,
+        return launch_dependent(k_verlet_node_cls_regular, spread(d->nnode), s, 0, d->reg_nx, d->reg_ny, d->mclass, tab,
                                 fe, d->fext, k, adv, u, v, a);
     }
     else if (cls)
-        return launch_dependent(k_verlet_node_cls, l, s, d->dofs, d->csr_ptr, d->csr_idx,
+        return launch_dependent(k_verlet_node_cls, l, s, 0, d->dofs, d->csr_ptr, d->csr_idx,
                                 reinterpret_cast<const int4*>(d->ell), d->mclass, tab, fe, d->fext, n, k, adv, u, v,
                                 a);
     else if (variant_node() == 1)
         k_verlet_node_fast_x2<<<grid_for((n + 1) / 2), kBlock, 0, s>>>(
             d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, d->inv, fe, d->fext, n, k, adv, u, v, a);
     else
-        return launch_dependent(k_verlet_node_fast, l, s, d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, d->inv, fe,
+        return launch_dependent(k_verlet_node_fast, l, s, 0, d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, d->inv, fe,
                                 d->fext, n, k, adv, u, v, a);
     return check_launch("verlet node kernel");
 }

@@ -389,6 +389,11 @@ k_verlet_pair_tma(const __grid_constant__ CUtensorMap mu, const __grid_constant_
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&ma)) : "memory");
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&ml)) : "memory");
         asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<uint64_t>(&mh)) : "memory");
+    }
+    pdl_wait(); // the barriers and tables above are set up while the previous increment ends
+    if (tid == 0) {
+        // what that kernel stored is now visible to this thread: also to the copies it issues
+        asm volatile("fence.proxy.async;\n" ::: "memory");
         if (static_cast<int>(blockIdx.x) < p.ntiles) issue(blockIdx.x, 0);
     }
     const int nx = p.nx, ny = p.ny, W = nx + 1;
@@ -419,7 +424,7 @@ k_verlet_pair_tma(const __grid_constant__ CUtensorMap mu, const __grid_constant_
         float4 fq = make_float4(0.f, 0.f, 0.f, 0.f);
         if (own) {
             cl = __ldg(p.mcls + node);
-            if (hf) fq = __ldg(p.fext + node);
+            if (hf) fq = p.fext[node];
         }
         const bool ok = pair_wait(s_bar + 8u * st, (i >> 1) & 1);
         const unsigned char* sg = base + st * kStageBytes;
@@ -1125,8 +1130,8 @@ static int launch_tma(PairTmaStep p, const CUtensorMap* mu, const CUtensorMap& m
     for (int64_t it = first; it < first + count; ++it) {
         p.uout = ub[(it + 1) & 1];
         p.advance = (it + 1 < first + count || advance_last) ? 1 : 0;
-        k_verlet_pair_tma<TY><<<grid, Gm::threads, Gm::Smem, s>>>(mu[it & 1], mv, ma, ml, mh, p, tab);
-        GF_TRY(check_launch("verlet pair kernel (TMA)"));
+        GF_TRY(launch_dependent(k_verlet_pair_tma<TY>, Shape{static_cast<unsigned>(grid), Gm::threads}, s, Gm::Smem,
+                                mu[it & 1], mv, ma, ml, mh, p, tab));
     }
     return GFGPU_OK;
 }
@@ -1217,14 +1222,14 @@ static int pair_increments(const gfgpu_verlet_desc* d, int64_t first, int64_t co
         const Shape l = spread(d->nelem, 256), h = spread(d->nelem, 128), r = spread(q.n, 256);
         for (int64_t it = first; it < first + count; ++it) {
             if (d->pair_mode == 2)
-                GF_TRY(launch_dependent(k_pair_elem_square, l, s, d->conn, ub[0],
+                GF_TRY(launch_dependent(k_pair_elem_square, l, s, 0, d->conn, ub[0],
                                         reinterpret_cast<const float4*>(d->coef_pair),
                                         reinterpret_cast<const float2*>(d->coef_pair + 4 * d->nelem), d->nelem, fe));
             else
-                GF_TRY(launch_dependent(k_pair_elem_stiff, h, s, d->conn, ub[0],
+                GF_TRY(launch_dependent(k_pair_elem_stiff, h, s, 0, d->conn, ub[0],
                                         reinterpret_cast<const float2*>(d->coef_pair), d->nelem, fe));
             q.advance = (it + 1 < first + count || advance_last) ? 1 : 0;
-            GF_TRY(launch_dependent(k_pair_node_csr, r, s, q, tab));
+            GF_TRY(launch_dependent(k_pair_node_csr, r, s, 0, q, tab));
         }
         return GFGPU_OK;
     }
@@ -1329,7 +1334,7 @@ int gfgpu_internal_mixed_increment(const gfgpu_verlet_desc* d, double* fe, int a
                                    double* a, cudaStream_t s)
 {
     const float* c = d->pcg_pair;
-    GF_TRY(launch_dependent(k_pair_elem_square_f64<true>, spread(d->nelem, 256), s, d->conn,
+    GF_TRY(launch_dependent(k_pair_elem_square_f64<true>, spread(d->nelem, 256), s, 0, d->conn,
                             reinterpret_cast<const double2*>(u), reinterpret_cast<const float4*>(c),
                             reinterpret_cast<const float2*>(c + 4 * d->nelem), d->nelem,
                             reinterpret_cast<double2*>(fe)));
@@ -1351,7 +1356,7 @@ int gfgpu_internal_mixed_increment(const gfgpu_verlet_desc* d, double* fe, int a
     q.h = 0.5 * d->dt;
     q.c = 0.5 * std::pow(d->dt, 2.0);
     q.advance = advance;
-    return launch_dependent(k_mixed_node, spread(q.n, 256), s, q, pair_class_tab(d));
+    return launch_dependent(k_mixed_node, spread(q.n, 256), s, 0, q, pair_class_tab(d));
 }
 
 // {L, N} [nelem] interleaved pairs, then kH [nelem] (6 floats per element) of a uniform square Quad4
