@@ -13,19 +13,37 @@ f64 = torch.float64
 i32 = torch.int32
 
 
+# An operator on a small mesh takes a few microseconds on the GPU, so the Python around it is kept to
+# the same scale: torch.device objects are made once per GPU, the current stream is read as the raw
+# handle, and a tensor that is already what an entry point needs is passed through untouched (the
+# five-call operator chain of a 33 x 29 mesh: 112 -> 48 us).
+_devices = {}
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def device():
-    if not torch.cuda.is_available():
+    """The current CUDA device; raises without one."""
+    if not _devices and not torch.cuda.is_available():
         raise RuntimeError("goosefem_gb300 needs a CUDA device (GB300, sm_103a)")
-    return torch.device("cuda", torch.cuda.current_device())
+    k = torch.cuda.current_device()
+    d = _devices.get(k)
+    if d is None:
+        d = _devices[k] = torch.device("cuda", k)
+    return d
 
 
 def stream():
-    return torch.cuda.current_stream().cuda_stream
+    """Handle of the current stream of the current device."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def dev_f64(a):
     """float64 contiguous device tensor (copies numpy / host / other dtypes)."""
     if isinstance(a, torch.Tensor):
+        if a.dtype is f64 and a.is_cuda and a.get_device() == torch.cuda.current_device() and a.is_contiguous():
+            return a
         t = a.to(device=device(), dtype=f64)
     else:
         t = torch.as_tensor(np.ascontiguousarray(a, dtype=np.float64), device=device())
@@ -59,11 +77,11 @@ def ptr(t):
 
 
 def empty(shape, dtype=f64):
-    return torch.empty(tuple(int(s) for s in shape), dtype=dtype, device=device())
+    return torch.empty(tuple(map(int, shape)), dtype=dtype, device=device())
 
 
 def check_shape(t, shape, name):
-    if tuple(t.shape) != tuple(int(s) for s in shape):
+    if t.shape != shape and tuple(t.shape) != tuple(int(s) for s in shape):
         raise ValueError(f"{name}: shape {tuple(t.shape)} != expected {tuple(shape)}")
 
 

@@ -112,19 +112,26 @@ def last_error():
     return lib().gfgpu_last_error().decode()
 
 
+_funcs = {}  # name -> (ctypes function, number of arguments, whether it returns a status)
+
+
 def call(name, *args):
     """Call an int-returning entry point; raise GFGPUError on a non-zero status.
 
     Only entry points whose prototype was read from include/gfgpu.h are callable: without
     argtypes ctypes would pass 64-bit pointers and sizes as 32-bit ints."""
-    L = lib()
-    if name not in _protos:
-        raise KeyError(f"{name} is not declared in {HEADER}")
-    if len(args) != len(_protos[name][1]):
-        raise TypeError(f"{name} takes {len(_protos[name][1])} arguments, got {len(args)}")
-    f = getattr(L, name)
-    rc = f(*args)
-    if f.restype is C.c_int and rc != 0:
+    f = _funcs.get(name)
+    if f is None:
+        L = lib()
+        if name not in _protos:
+            raise KeyError(f"{name} is not declared in {HEADER}")
+        fn = getattr(L, name)
+        f = _funcs[name] = (fn, len(_protos[name][1]), fn.restype is C.c_int)
+    fn, nargs, status = f
+    if len(args) != nargs:
+        raise TypeError(f"{name} takes {nargs} arguments, got {len(args)}")
+    rc = fn(*args)
+    if status and rc != 0:
         raise GFGPUError(name, rc, last_error())
     return rc
 
