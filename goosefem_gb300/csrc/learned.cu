@@ -366,7 +366,8 @@ k_conv_mma(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict_
                              : X + gp * 32 + ch);
         cp_async16(halo + pix * kPadC + ch, src, in);
     }
-    if (LAST && threadIdx.x == 0) s_sigma = z ? sqrt(sc[rr_slot] / nfree) : 1.0;
+    // (volatile: the first layer of the same chain may have written it)
+    if (LAST && threadIdx.x == 0) s_sigma = z ? sqrt(*static_cast<const volatile double*>(sc + rr_slot) / nfree) : 1.0;
     cp_async_wait_all();
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -447,8 +448,8 @@ k_conv_mma(const __nv_bfloat16* __restrict__ X, const __nv_bfloat16* __restrict_
 // [H, W, 32]. Same tile and warp layout as k_conv_mma.
 template <bool PLANAR_OUT = false>
 __global__ void __launch_bounds__(kMmaThreads, 4)
-k_first_mma(const double* __restrict__ r, const double* __restrict__ sc, int rr_slot, double nfree,
-            const float* __restrict__ mat, const float* __restrict__ X0,
+k_first_mma(const double* __restrict__ r, double* sc, int rr_slot, const double* __restrict__ rr_part, int rr_nblk,
+            double nfree, const float* __restrict__ mat, const float* __restrict__ X0,
             const __nv_bfloat16* __restrict__ WF, const float* __restrict__ bias, int H, int Wd,
             __nv_bfloat16* __restrict__ Y)
 {
@@ -459,9 +460,19 @@ k_first_mma(const double* __restrict__ r, const double* __restrict__ sc, int rr_
     if (PLANAR_OUT) pdl_launch_dependents(); // the tcgen05 layer that follows may launch
     const int y0 = blockIdx.y * kTileY, x0 = blockIdx.x * kTileX;
     for (int i = threadIdx.x; i < 3 * 32 * kPadF / 8; i += blockDim.x) cp_async16(wf + i * 8, WF + i * 8, true);
-    if (threadIdx.x == 0) {
-        double sigma = r ? sqrt(sc[rr_slot] / nfree) : 1.0;
-        s_inv = sigma > 0.0 ? static_cast<float>(1.0 / sigma) : 0.0f;
+    if (threadIdx.x < 32) {
+        // r.r: the scalar, or the sum of the partials of the kernel before (kept for the last layer)
+        double rr = 0.0;
+        if (rr_part) {
+            for (int i = threadIdx.x; i < rr_nblk; i += 32) rr += rr_part[i];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) rr += __shfl_down_sync(0xffffffffu, rr, o);
+        }
+        if (threadIdx.x == 0) {
+            if (rr_part && blockIdx.x == 0 && blockIdx.y == 0) sc[rr_slot] = rr;
+            const double sigma = r ? sqrt((rr_part ? rr : sc[rr_slot]) / nfree) : 1.0;
+            s_inv = sigma > 0.0 ? static_cast<float>(1.0 / sigma) : 0.0f;
+        }
     }
     __syncthreads();
     const float inv = s_inv;
@@ -1257,7 +1268,7 @@ namespace gfgpu {
 namespace nn {
 
 constexpr int kWgtBlocks = 152; // weight-gradient partials: a block on each of the 152 SMs
-constexpr int kRed = 1024; // most blocks (and partials per row) of the FCG reductions
+constexpr int kRed = 304; // most blocks (and partials per row) of the FCG reductions: two per SM
 
 inline int64_t a256(int64_t b)
 {
@@ -1436,20 +1447,20 @@ struct SlotList {
     int n;
     int s[kMaxSlots];
 };
-// device scalars: r.r, b.b, step length per new direction, P.Q per slot, orthogonalisation
-// coefficient per basis entry
-enum { F_RR = 0, F_BB, F_A0, F_A1, F_PQ, F_C = F_PQ + kMaxSlots, F_R1 = F_C + kMaxSlots, F_COUNT };
+// device scalars: r.r, b.b, step length per new direction, P.Q per slot, r1.r1
+enum { F_RR = 0, F_BB, F_A0, F_A1, F_PQ, F_R1 = F_PQ + kMaxSlots, F_COUNT };
 
+constexpr int kWide = 1024; // most threads of a reduction block
+
+// Sum over the block in a fixed order, valid in thread 0 (sh: blockDim doubles). One warp adds: an
+// FP64 instruction of a warp takes 16 clocks of the SM, a shuffle tree in every warp five of them.
 __device__ __forceinline__ double bsum(double v, double* sh)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    if (lane == 0) sh[wi] = v;
+    sh[threadIdx.x] = v;
     __syncthreads();
     double r = 0.0;
-    if (wi == 0) {
-        r = lane < (blockDim.x >> 5) ? sh[lane] : 0.0;
+    if (threadIdx.x < 32) {
+        for (int i = threadIdx.x; i < static_cast<int>(blockDim.x); i += 32) r += sh[i];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) r += __shfl_down_sync(0xffffffffu, r, o);
     }
@@ -1457,59 +1468,82 @@ __device__ __forceinline__ double bsum(double v, double* sh)
     return r;
 }
 
-// Blocks of a reduction kernel over `items` entries: one per 256, at most kRed. A block without
-// entries still costs its launch, two block sums and an atomic on the counter: at 63k dofs (246
-// blocks) the dots took 12-19 us and the gather 14 us with 1024 blocks whatever the size. The
-// partials keep their places and order of summation, so the sums keep their bits.
-inline unsigned red_blocks(int64_t items)
+// Launch shape of a reduction kernel over `items` entries: at most kRed blocks, as many of them as
+// blocks of 256 threads make, else wider blocks, else a grid-stride loop. Fixed by the size, so the
+// sums are the same on every run. With 1024 blocks whatever the size, 63k dofs paid for 778 blocks
+// without entries (two block sums and an atomic each: dots 12-19 us, gather 14 us).
+inline Shape red_shape(int64_t items, int widest = kWide)
 {
-    return static_cast<unsigned>(std::min<int64_t>(kRed, std::max<int64_t>(1, (items + 255) / 256)));
+    int block = 256;
+    while (block < widest && (items + block - 1) / block > kRed) block *= 2;
+    return Shape{static_cast<unsigned>(std::min<int64_t>(kRed, std::max<int64_t>(1, (items + block - 1) / block))), block};
 }
 
-// Last-block reductions: every block of a partial-sum kernel writes its partial,
-// fences and counts itself in; the last block to arrive reduces the partials (fixed order, so the
-// result does not depend on which block is last) and resets the counter for the next launch. This
-// replaces a separate one-block reduction launch.
-__device__ __forceinline__ bool last_block(unsigned int* counter)
-{
-    __shared__ bool is_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned int prev = atomicAdd(counter, 1u);
-        is_last = prev == gridDim.x - 1;
-        if (is_last) *counter = 0u;
-    }
-    __syncthreads();
-    if (is_last) __threadfence();
-    return is_last;
-}
+// Rows of `partial`: the dots of the orthogonalisation in 0 .. kMaxSlots - 1, then P.Q and r.P of the
+// last gather, r1.r1 and r.r.
+enum { ROW_PQ = kMaxSlots, ROW_RP, ROW_R1, ROW_RR, ROW_COUNT };
 
-// sum of partial[0 .. gridDim.x) by the whole block in a fixed order
-__device__ __forceinline__ double block_sum_partials(const double* partial, double* sh)
+// A kernel that needs a sum over the dofs adds the partials of the kernel that formed them in each of
+// its blocks (at most kRed of them, a load or two per thread). The last block of the first kernel did
+// it before: the fence and the atomic in every block cost 4-6 us of each of six kernels an iteration.
+__device__ __forceinline__ double sum_row(const double* partial, int row, int nblk, double* sh)
 {
     double v = 0.0;
-    for (int i = threadIdx.x; i < gridDim.x; i += blockDim.x) v += __ldcg(partial + i);
+    for (int i = threadIdx.x; i < nblk; i += blockDim.x) v += partial[row * kRed + i];
     return bsum(v, sh);
 }
 
-// coefficient c_k = (z.Q_j) / (P_j.Q_j) of basis entry k (slot j = L.s[k]) from partial row k,
-// computed by the last block (warp k -> rows k, k + nwarps, ...; lane-strided sums, then the
-// shuffle tree); 0 for a degenerate or non-finite direction, which the combination then skips
-__device__ __forceinline__ void coef_rows(const double* partial, const SlotList& L, double* sc)
+// Step length alpha_dd = r.P / P.Q (0 if degenerate) of the last gather, in every thread; block 0
+// keeps it and P.Q (slot `slot`) for the kernels that follow.
+__device__ __forceinline__ double finish_gather(const double* partial, int nblk, double* sc, int slot, int dd,
+                                                double* sh)
+{
+    // warp 0 adds P.Q, warp 1 r.P (a block has at least 8 warps and nblk is at most kRed)
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (w < 2) {
+        const double* row = partial + (w == 0 ? ROW_PQ : ROW_RP) * kRed;
+        double v = 0.0;
+        for (int i = lane; i < nblk; i += 32) v += row[i];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) sh[w] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double pq = sh[0], rp = sh[1];
+        double a = (pq > 0.0 && isfinite(pq)) ? rp / pq : 0.0;
+        a = isfinite(a) ? a : 0.0;
+        if (blockIdx.x == 0) {
+            sc[F_PQ + slot] = pq;
+            sc[F_A0 + dd] = a;
+        }
+        sh[2] = a;
+    }
+    __syncthreads();
+    const double a = sh[2];
+    __syncthreads();
+    return a;
+}
+
+// coefficients c_k = (z.Q_j) / (P_j.Q_j) of the basis entries (slot j = L.s[k]) from partial rows k,
+// into c (shared): warp k -> rows k, k + nwarps, ...; lane-strided sums, then the shuffle tree; 0 for
+// a degenerate or non-finite direction, which the combination then skips
+__device__ __forceinline__ void coef_rows(const double* partial, int nblk, const SlotList& L, const double* sc,
+                                          double* c)
 {
     const int nw = blockDim.x >> 5, lane = threadIdx.x & 31;
     for (int k = threadIdx.x >> 5; k < L.n; k += nw) {
         double v = 0.0;
-        for (int i = lane; i < gridDim.x; i += 32) v += __ldcg(partial + k * kRed + i);
+        for (int i = lane; i < nblk; i += 32) v += partial[k * kRed + i];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
         if (lane == 0) {
-            double pq = sc[F_PQ + L.s[k]];
-            double c = (pq > 0.0 && isfinite(pq)) ? v / pq : 0.0;
-            sc[F_C + k] = isfinite(c) ? c : 0.0;
+            const double pq = sc[F_PQ + L.s[k]];
+            const double q = (pq > 0.0 && isfinite(pq)) ? v / pq : 0.0;
+            c[k] = isfinite(q) ? q : 0.0;
         }
     }
+    __syncthreads();
 }
 
 
@@ -1525,14 +1559,14 @@ __global__ void k_fkeep(const int32_t* __restrict__ part, int64_t nnu, const dou
     GF_FOR(t, n) o[t] = part[t] < nnu ? 0.0 : x[t];
 }
 
-// r = rhs_u - (A x)_u (0 on prescribed); partial r.r
-__global__ void __launch_bounds__(256)
+// r = rhs_u - (A x)_u (0 on prescribed); partial r.r (ROW_RR)
+__global__ void __launch_bounds__(kWide)
 k_fres(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
        const int32_t* __restrict__ part, int64_t nnu, const double* __restrict__ fe,
        const double* __restrict__ rhs, int64_t n, double* __restrict__ r, double* __restrict__ partial,
        RegGrid reg)
 {
-    __shared__ double sh[32];
+    __shared__ double sh[kWide];
     double rr = 0.0;
     GF_FOR(t, n)
     {
@@ -1545,18 +1579,17 @@ k_fres(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr, const 
         r[t] = rv;
     }
     double s = bsum(rr, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = s;
+    if (threadIdx.x == 0) partial[ROW_RR * kRed + blockIdx.x] = s;
 }
 
-// q = (A p)_u; partials p.q (row 0) and r.p (row 1)
-__global__ void __launch_bounds__(256)
+// q = (A p)_u; partials p.q (ROW_PQ) and r.p (ROW_RP)
+__global__ void __launch_bounds__(kWide)
 k_fgather(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr, const int32_t* __restrict__ idx,
           const int32_t* __restrict__ part, int64_t nnu, const double* __restrict__ fe,
           const double* __restrict__ p, const double* __restrict__ r, int64_t n, double* __restrict__ q,
-          double* __restrict__ partial, double* __restrict__ sc, int slot, int dd,
-          unsigned int* __restrict__ counter, RegGrid reg)
+          double* __restrict__ partial, RegGrid reg)
 {
-    __shared__ double sh[32];
+    __shared__ double sh[kWide];
     double pq = 0.0, rp = 0.0;
     GF_FOR(t, n)
     {
@@ -1571,28 +1604,19 @@ k_fgather(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr, con
     double s1 = bsum(pq, sh);
     double s2 = bsum(rp, sh);
     if (threadIdx.x == 0) {
-        partial[blockIdx.x] = s1;
-        partial[kRed + blockIdx.x] = s2;
-    }
-    if (last_block(counter)) { // P.Q and the step length alpha_dd = r.P / P.Q (0 if degenerate)
-        const double tpq = block_sum_partials(partial, sh);
-        const double trp = block_sum_partials(partial + kRed, sh);
-        if (threadIdx.x == 0) {
-            sc[F_PQ + slot] = tpq;
-            double a = (tpq > 0.0 && isfinite(tpq)) ? trp / tpq : 0.0;
-            sc[F_A0 + dd] = isfinite(a) ? a : 0.0;
-        }
+        partial[ROW_PQ * kRed + blockIdx.x] = s1;
+        partial[ROW_RP * kRed + blockIdx.x] = s2;
     }
 }
 
-// r1 = r - alpha_0 q0 (the residual after the step along the first direction of the iteration);
-// partial r1.r1
-__global__ void __launch_bounds__(256)
-k_resid1(const double* __restrict__ r, const double* __restrict__ q0, double* __restrict__ sc,
-         int64_t n, double* __restrict__ r1, double* __restrict__ partial, unsigned int* __restrict__ counter)
+// alpha_0 from the gather's partials; r1 = r - alpha_0 q0 (the residual after the step along the first
+// direction of the iteration, whose slot is `slot`); partial r1.r1 (ROW_R1)
+__global__ void __launch_bounds__(kWide)
+k_resid1(const double* __restrict__ r, const double* __restrict__ q0, double* __restrict__ sc, int slot,
+         int64_t n, double* __restrict__ r1, double* partial, int nblk)
 {
-    __shared__ double sh[32];
-    const double a0 = sc[F_A0];
+    __shared__ double sh[kWide];
+    const double a0 = finish_gather(partial, nblk, sc, slot, 0, sh);
     double rr = 0.0;
     GF_FOR(t, n)
     {
@@ -1601,35 +1625,31 @@ k_resid1(const double* __restrict__ r, const double* __restrict__ q0, double* __
         rr = fma(v, v, rr);
     }
     double s = bsum(rr, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = s;
-    if (last_block(counter)) {
-        const double t = block_sum_partials(partial, sh);
-        if (threadIdx.x == 0) sc[F_R1] = t;
-    }
+    if (threadIdx.x == 0) partial[ROW_R1 * kRed + blockIdx.x] = s;
 }
 
-// sc[dst.s[k]] = sum of the nblk partials of row k (fixed order)
-__global__ void k_fredv(const double* __restrict__ partial, int nblk, SlotList dst, double* __restrict__ sc)
+// sc[dst] = sum of the nblk partials of row `row` (fixed order)
+__global__ void k_fredv(const double* __restrict__ partial, int row, int nblk, int dst, double* __restrict__ sc)
 {
-    __shared__ double sh[32];
-    for (int p = 0; p < dst.n; ++p) {
-        double v = 0.0;
-        for (int i = threadIdx.x; i < nblk; i += blockDim.x) v += partial[p * kRed + i];
-        double t = bsum(v, sh);
-        if (threadIdx.x == 0) sc[dst.s[p]] = t;
-        __syncthreads();
-    }
+    __shared__ double sh[kWide];
+    const double t = sum_row(partial, row, nblk, sh);
+    if (threadIdx.x == 0) sc[dst] = t;
 }
+
+// threads of a block that keeps NS sums (and their pointers) per thread in registers
+constexpr int wide_ns(int ns) { return ns <= 4 ? kWide : 256; }
 
 // partial dots z.Q_j for the basis slots (z = minv * r when zin is null); NS >= L.n. Vectors
-// are read as double2 (n even, slots 256-byte aligned).
+// are read as double2 (n even, slots 256-byte aligned). fin_slot >= 0: the gather before this kernel
+// was the first direction's (slot fin_slot) and no kernel in between took its step length.
 template <int NS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(wide_ns(NS))
 k_mdot(const double* __restrict__ zin, const double* __restrict__ minv, const double* __restrict__ r,
-       const double* __restrict__ Q, int64_t ld, SlotList L, int64_t n, double* __restrict__ partial,
-       double* __restrict__ sc, unsigned int* __restrict__ counter)
+       const double* __restrict__ Q, int64_t ld, SlotList L, int64_t n, double* partial,
+       double* __restrict__ sc, int fin_slot, int fin_nblk)
 {
-    __shared__ double sh[32];
+    __shared__ double sh[wide_ns(NS)];
+    if (fin_slot >= 0 && blockIdx.x == 0) finish_gather(partial, fin_nblk, sc, fin_slot, 0, sh);
     double acc[NS];
     const double2* q[NS];
 #pragma unroll
@@ -1671,22 +1691,23 @@ k_mdot(const double* __restrict__ zin, const double* __restrict__ minv, const do
             if (threadIdx.x == 0) partial[j * kRed + blockIdx.x] = v;
         }
     }
-    if (last_block(counter)) coef_rows(partial, L, sc);
 }
 
-// P_new = z - sum_k c_k P_{L.s[k]} (A-orthogonalisation with the precomputed coefficients),
-// double2 access as in k_mdot
+// P_new = z - sum_k c_k P_{L.s[k]} (A-orthogonalisation, the coefficients from the dots' nblk
+// partials), double2 access as in k_mdot
 template <int NS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(wide_ns(NS))
 k_mcombine(const double* __restrict__ zin, const double* __restrict__ minv,
-           const double* __restrict__ r, const double* __restrict__ sc, double* P, int64_t ld,
-           SlotList L, int snew, int64_t n)
+           const double* __restrict__ r, const double* __restrict__ partial, int nblk,
+           const double* __restrict__ sc, double* P, int64_t ld, SlotList L, int snew, int64_t n)
 {
+    __shared__ double cs[NS];
+    coef_rows(partial, nblk, L, sc, cs);
     double c[NS];
     const double2* p[NS];
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
-        c[j] = j < L.n ? sc[F_C + j] : 0.0;
+        c[j] = j < L.n ? cs[j] : 0.0;
         p[j] = reinterpret_cast<const double2*>(P + (j < L.n ? L.s[j] : 0) * ld);
     }
     double2* out = reinterpret_cast<double2*>(P + snew * ld);
@@ -1722,15 +1743,17 @@ k_mcombine(const double* __restrict__ zin, const double* __restrict__ minv,
 }
 
 // x += sum_d alpha_d P_d, r -= sum_d alpha_d Q_d (the new directions are mutually
-// A-orthogonal, so every alpha is taken with the same r); partial r.r
-__global__ void __launch_bounds__(256)
+// A-orthogonal, so every alpha is taken with the same r; the last one's from the gather's nblk
+// partials); partial r.r (ROW_RR)
+__global__ void __launch_bounds__(kWide)
 k_mupdate(const int32_t* __restrict__ part, int64_t nnu, const double* __restrict__ P,
           const double* __restrict__ Q, int64_t ld, int s0, int s1, int ndir,
-          double* __restrict__ sc, int64_t n, double* __restrict__ x, double* __restrict__ r,
-          double* __restrict__ partial, unsigned int* __restrict__ counter)
+          double* sc, int64_t n, double* __restrict__ x, double* __restrict__ r,
+          double* partial, int nblk)
 {
-    __shared__ double sh[32];
-    double a0 = sc[F_A0], a1 = ndir > 1 ? sc[F_A1] : 0.0;
+    __shared__ double sh[kWide];
+    const double al = finish_gather(partial, nblk, sc, ndir > 1 ? s1 : s0, ndir - 1, sh);
+    const double a0 = ndir > 1 ? sc[F_A0] : al, a1 = ndir > 1 ? al : 0.0;
     const double* P0 = P + s0 * ld;
     const double* Q0 = Q + s0 * ld;
     const double* P1 = P + s1 * ld;
@@ -1754,11 +1777,7 @@ k_mupdate(const int32_t* __restrict__ part, int64_t nnu, const double* __restric
         }
     }
     double v = bsum(rr, sh);
-    if (threadIdx.x == 0) partial[blockIdx.x] = v;
-    if (last_block(counter)) {
-        const double t = block_sum_partials(partial, sh);
-        if (threadIdx.x == 0) sc[F_RR] = t;
-    }
+    if (threadIdx.x == 0) partial[ROW_RR * kRed + blockIdx.x] = v;
 }
 
 // launch k_mdot / k_mcombine with the smallest slot-count instantiation that holds L.n
@@ -1776,25 +1795,27 @@ inline void with_ns(int n, A&&... a)
 
 template <int NS>
 struct MdotL {
-    static void go(unsigned g, cudaStream_t st, const double* zin, const double* minv, const double* r,
-                   const double* Q, int64_t ld, const SlotList& L, int64_t n, double* partial, double* sc,
-                   unsigned int* counter)
+    static void go(cudaStream_t st, const double* zin, const double* minv, const double* r, const double* Q,
+                   int64_t ld, const SlotList& L, int64_t n, double* partial, double* sc, int fin_slot, int fin_nblk,
+                   int* nblk)
     {
-        k_mdot<NS><<<g, 256, 0, st>>>(zin, minv, r, Q, ld, L, n, partial, sc, counter);
+        const Shape g = red_shape(n / 2, wide_ns(NS));
+        *nblk = static_cast<int>(g.grid);
+        k_mdot<NS><<<g.grid, g.block, 0, st>>>(zin, minv, r, Q, ld, L, n, partial, sc, fin_slot, fin_nblk);
     }
 };
 
 template <int NS>
 struct McombineL {
-    static void go(unsigned g, cudaStream_t st, const double* zin, const double* minv, const double* r,
-                   const double* sc, double* P, int64_t ld, const SlotList& L, int snew, int64_t n)
+    static void go(cudaStream_t st, const double* zin, const double* minv, const double* r, const double* partial,
+                   int nblk, const double* sc, double* P, int64_t ld, const SlotList& L, int snew, int64_t n)
     {
-        k_mcombine<NS><<<g, 256, 0, st>>>(zin, minv, r, sc, P, ld, L, snew, n);
+        const Shape g = red_shape(n / 2, wide_ns(NS));
+        k_mcombine<NS><<<g.grid, g.block, 0, st>>>(zin, minv, r, partial, nblk, sc, P, ld, L, snew, n);
     }
 };
 
 struct FcgWs {
-    unsigned int* cnt; // last-block counters: [0] dots, [1] gather, [2] update, [3] resid1
     double *fe, *r, *z, *minv, *P, *Q, *partial, *sc;
     int64_t ld;
     __nv_bfloat16 *a1, *a2, *a3, *wt1, *wt2, *wt0, *wt3;
@@ -1851,11 +1872,9 @@ inline FcgWs carve_fcg(const gfgpu_verlet_desc* d, int64_t hw, int nslots, void*
     w.Q = reinterpret_cast<double*>(c);
     c += nslots * w.ld * 8;
     w.partial = reinterpret_cast<double*>(c);
-    c += a256(int64_t(kMaxSlots) * kRed * 8);
+    c += a256(int64_t(ROW_COUNT) * kRed * 8);
     w.sc = reinterpret_cast<double*>(c);
     c += a256(F_COUNT * 8);
-    w.cnt = reinterpret_cast<unsigned int*>(c);
-    c += 256;
     carve_nn(c, hw, &w.a1, &w.a2, &w.a3, &w.wt1, &w.wt2, &w.wt0, &w.wt3);
     return w;
 }
@@ -1864,7 +1883,7 @@ inline int64_t fcg_bytes(const gfgpu_verlet_desc* d, int64_t hw, int nslots)
 {
     int64_t n = d->nnode * d->ndim;
     return a256(d->nelem * d->nne * d->ndim * 8) + (3 + 2 * int64_t(nslots)) * a256(n * 8) +
-           a256(int64_t(kMaxSlots) * kRed * 8) + a256(F_COUNT * 8) + 256 + nn_bytes(hw);
+           a256(int64_t(ROW_COUNT) * kRed * 8) + a256(F_COUNT * 8) + nn_bytes(hw);
 }
 
 // the tensor-core layers' weights in their shared-memory layouts
@@ -1938,8 +1957,8 @@ inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t sm
 
 // the four layers on one H x W grid: input from the FP64 residual (r != null) or from X0,
 // output to the FP64 correction z (z != null) or to Y
-inline int nn_forward(const gfgpu_nn_desc* nn, const double* r, const float* X0, const double* sc,
-                      int rr_slot, double nfree, const int32_t* part, int64_t nnu,
+inline int nn_forward(const gfgpu_nn_desc* nn, const double* r, const float* X0, double* sc,
+                      int rr_slot, const double* rr_part, int rr_nblk, double nfree, const int32_t* part, int64_t nnu,
                       __nv_bfloat16* a1, __nv_bfloat16* a2, __nv_bfloat16* a3,
                       const __nv_bfloat16* wt1, const __nv_bfloat16* wt2, const __nv_bfloat16* wt0,
                       const __nv_bfloat16* wt3, double* z, float* Y, cudaStream_t s)
@@ -1948,11 +1967,11 @@ inline int nn_forward(const gfgpu_nn_desc* nn, const double* r, const float* X0,
     dim3 grid((W + kTileX - 1) / kTileX, (H + kTileY - 1) / kTileY);
     const bool planar = nn_tensor_path() >= 2; // paths 2, 3: channel-planar activations
     if (planar)
-        k_first_mma<true><<<grid, kMmaThreads, 0, s>>>(r, sc, rr_slot, nfree, nn->material, X0, wt0,
-                                                       nn->params_f32 + b_off(0), H, W, a1);
+        k_first_mma<true><<<grid, kMmaThreads, 0, s>>>(r, sc, rr_slot, rr_part, rr_nblk, nfree, nn->material, X0,
+                                                       wt0, nn->params_f32 + b_off(0), H, W, a1);
     else
-        k_first_mma<false><<<grid, kMmaThreads, 0, s>>>(r, sc, rr_slot, nfree, nn->material, X0, wt0,
-                                                        nn->params_f32 + b_off(0), H, W, a1);
+        k_first_mma<false><<<grid, kMmaThreads, 0, s>>>(r, sc, rr_slot, rr_part, rr_nblk, nfree, nn->material, X0,
+                                                        wt0, nn->params_f32 + b_off(0), H, W, a1);
     if (nn_tensor_path() >= 2) {
         static_assert(kPlanarPad >= 4, "dilations up to 4 fit the 17-group box");
         // path 2: one box per plane of a whole halo tile; path 3: one box per plane row
@@ -2013,10 +2032,10 @@ inline int nn_forward(const gfgpu_nn_desc* nn, const double* r, const float* X0,
 }
 
 // z = RMS(r) * net(r / RMS(r)) on the nodal grid (0 on prescribed dofs)
-inline int nn_apply(const gfgpu_nn_desc* nn, const double* r, const double* sc, int rr_slot,
-                    double nfree, const int32_t* part, int64_t nnu, FcgWs& w, double* z, cudaStream_t s)
+inline int nn_apply(const gfgpu_nn_desc* nn, const double* r, double* sc, int rr_slot, const double* rr_part,
+                    int rr_nblk, double nfree, const int32_t* part, int64_t nnu, FcgWs& w, double* z, cudaStream_t s)
 {
-    return nn_forward(nn, r, nullptr, sc, rr_slot, nfree, part, nnu, w.a1, w.a2, w.a3, w.wt1, w.wt2,
+    return nn_forward(nn, r, nullptr, sc, rr_slot, rr_part, rr_nblk, nfree, part, nnu, w.a1, w.a2, w.a3, w.wt1, w.wt2,
                       w.wt0, w.wt3, z, nullptr, s);
 }
 
@@ -2200,7 +2219,7 @@ int gfgpu_nn_infer(const gfgpu_nn_desc* nn, const float* X0, float* Y, void* wor
     __nv_bfloat16 *a1, *a2, *a3, *wt1, *wt2, *wt0, *wt3;
     carve_nn(static_cast<char*>(workspace), act_pixels(nn->H, nn->W), &a1, &a2, &a3, &wt1, &wt2, &wt0, &wt3);
     nn_prepare_weights(nn, wt1, wt2, wt0, wt3, s);
-    return nn_forward(nn, nullptr, X0, nullptr, 0, 1.0, nullptr, 0, a1, a2, a3, wt1, wt2, wt0, wt3,
+    return nn_forward(nn, nullptr, X0, nullptr, 0, nullptr, 0, 1.0, nullptr, 0, a1, a2, a3, wt1, wt2, wt0, wt3,
                       nullptr, Y, s);
 }
 
@@ -2237,24 +2256,19 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
         yc = reinterpret_cast<double*>(c + a256(n * 8) + a256(nc * 8));
     }
     const double nfree = static_cast<double>(d->nnu);
-    const unsigned gb = red_blocks(n);
+    const Shape rs = red_shape(n);
+    const int nr = static_cast<int>(rs.grid); // partials of a kernel over the dofs
     double h[F_COUNT];
     auto read_sc = [&]() -> int {
         GF_TRY(check_cuda(cudaMemcpyAsync(h, w.sc, F_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s),
                           "cudaMemcpyAsync"));
         return check_cuda(cudaStreamSynchronize(s), "cudaStreamSynchronize");
     };
-    auto one = [](int slot) {
-        SlotList l{};
-        l.n = 1;
-        l.s[0] = slot;
-        return l;
-    };
-
     // One iteration, direction counter `c0` on entry (slot of direction k: k mod nslots). New
     // direction d is A-orthogonalised against the last nkeep directions of earlier iterations
-    // and the earlier directions of this iteration.
-    auto iteration = [&](int64_t c0, cudaStream_t st) -> int {
+    // and the earlier directions of this iteration. read: r.r is formed as well (the host reads it
+    // next, or the network takes its scale from it).
+    auto iteration = [&](int64_t c0, bool read, cudaStream_t st) -> int {
         for (int dd = 0; dd < ndir; ++dd) {
             int64_t cur = c0 + dd;
             int snew = static_cast<int>(cur % nslots);
@@ -2262,6 +2276,8 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
             for (int64_t k = std::max<int64_t>(0, c0 - nkeep); k < cur; ++k)
                 L.s[L.n++] = static_cast<int>(k % nslots);
             const double* zin = nullptr;
+            int fin_slot = -1; // the first direction's slot, while its step length is still to be taken
+            if (dd == 1 && !post) fin_slot = static_cast<int>(c0 % nslots);
             if (dd == 0 && g) {
                 GF_TRY(gfgpu_internal_coarse_apply(g, d->part, d->nnu, w.minv, w.r, vc, yc, zc, st));
                 zin = zc;
@@ -2270,44 +2286,44 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
                 // the network sees the residual left after the step along the two-level direction
                 // (zc is free again: its direction is stored in slot c0 % nslots)
                 const double* q0 = w.Q + static_cast<int>(c0 % nslots) * w.ld;
-                k_resid1<<<gb, 256, 0, st>>>(w.r, q0, w.sc, n, zc, w.partial, w.cnt + 3);
-                GF_TRY(nn_apply(nn, zc, w.sc, F_R1, nfree, d->part, d->nnu, w, w.z, st));
+                k_resid1<<<rs.grid, rs.block, 0, st>>>(w.r, q0, w.sc, static_cast<int>(c0 % nslots), n, zc, w.partial, nr);
+                GF_TRY(nn_apply(nn, zc, w.sc, F_R1, w.partial + ROW_R1 * kRed, nr, nfree, d->part, d->nnu, w, w.z, st));
                 zin = w.z;
             }
             else if (dd == 1) {
-                GF_TRY(nn_apply(nn, w.r, w.sc, F_RR, nfree, d->part, d->nnu, w, w.z, st));
+                GF_TRY(nn_apply(nn, w.r, w.sc, F_RR, nullptr, 0, nfree, d->part, d->nnu, w, w.z, st));
                 zin = w.z;
             }
-            if (L.n > 0) {
-                with_ns<MdotL>(L.n, red_blocks(n / 2), st, zin, w.minv, w.r, w.Q, w.ld, L, n, w.partial, w.sc, w.cnt);
-            }
-            with_ns<McombineL>(L.n, grid_for(n / 2), st, zin, w.minv, w.r, w.sc, w.P, w.ld, L, snew, n);
+            int nd = 0; // partials of the dots
+            if (L.n > 0)
+                with_ns<MdotL>(L.n, st, zin, w.minv, w.r, w.Q, w.ld, L, n, w.partial, w.sc, fin_slot, nr, &nd);
+            with_ns<McombineL>(L.n, st, zin, w.minv, w.r, w.partial, nd, w.sc, w.P, w.ld, L, snew, n);
             double* Pn = w.P + snew * w.ld;
             double* Qn = w.Q + snew * w.ld;
             GF_TRY(gfgpu_internal_iteration_element_forces(d, Pn, w.fe, st));
-            k_fgather<<<gb, 256, 0, st>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, Pn,
-                                          w.r, n, Qn, w.partial, w.sc, snew, dd, w.cnt + 1, reg_grid(d));
+            k_fgather<<<rs.grid, rs.block, 0, st>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, Pn, w.r, n,
+                                                    Qn, w.partial, reg_grid(d));
         }
-        k_mupdate<<<gb, 256, 0, st>>>(d->part, d->nnu, w.P, w.Q, w.ld, static_cast<int>(c0 % nslots),
-                                      static_cast<int>((c0 + 1) % nslots), ndir, w.sc, n, x, w.r,
-                                      w.partial, w.cnt + 2);
+        k_mupdate<<<rs.grid, rs.block, 0, st>>>(d->part, d->nnu, w.P, w.Q, w.ld, static_cast<int>(c0 % nslots),
+                                                static_cast<int>((c0 + 1) % nslots), ndir, w.sc, n, x, w.r, w.partial,
+                                                nr);
+        if (read || (nn && !post)) k_fredv<<<1, kWide, 0, st>>>(w.partial, ROW_RR, nr, F_RR, w.sc);
         return check_launch("fcg iteration");
     };
 
     if (nn) nn_prepare_weights(nn, w.wt1, w.wt2, w.wt0, w.wt3, s);
-    GF_TRY(check_cuda(cudaMemsetAsync(w.cnt, 0, 256, s), "cudaMemsetAsync"));
     k_finv<<<grid_for(n), kBlock, 0, s>>>(d->part, d->nnu, diag, n, w.minv);
     // ||b||, b = -(A x_p)_u (P slot 0 as scratch)
     k_fkeep<<<grid_for(n), kBlock, 0, s>>>(d->part, d->nnu, x, n, w.P);
     GF_TRY(gfgpu_internal_element_forces(d, w.P, w.fe, s));
-    k_fres<<<gb, 256, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.z,
+    k_fres<<<rs.grid, rs.block, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.z,
                               w.partial, reg_grid(d));
-    k_fredv<<<1, 1024, 0, s>>>(w.partial, static_cast<int>(gb), one(F_BB), w.sc);
+    k_fredv<<<1, kWide, 0, s>>>(w.partial, ROW_RR, nr, F_BB, w.sc);
     // r = -(A x)_u
     GF_TRY(gfgpu_internal_element_forces(d, x, w.fe, s));
-    k_fres<<<gb, 256, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.r,
+    k_fres<<<rs.grid, rs.block, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.r,
                               w.partial, reg_grid(d));
-    k_fredv<<<1, 1024, 0, s>>>(w.partial, static_cast<int>(gb), one(F_RR), w.sc);
+    k_fredv<<<1, kWide, 0, s>>>(w.partial, ROW_RR, nr, F_RR, w.sc);
     GF_TRY(read_sc());
     double bnorm = std::sqrt(h[F_BB]);
     if (bnorm == 0.0) bnorm = 1.0;
@@ -2335,7 +2351,7 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
             rc = check_cuda(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "capture");
             if (rc != GFGPU_OK) break;
             int crc = GFGPU_OK;
-            for (int64_t k = 0; k < chunk && crc == GFGPU_OK; ++k) crc = iteration(c + k * ndir, cs);
+            for (int64_t k = 0; k < chunk && crc == GFGPU_OK; ++k) crc = iteration(c + k * ndir, k == chunk - 1, cs);
             cudaError_t e = cudaStreamEndCapture(cs, &graph);
             if (crc != GFGPU_OK) {
                 if (graph) cudaGraphDestroy(graph);
@@ -2356,7 +2372,7 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
         else {
             int64_t nb = exec ? maxiter - it : std::min<int64_t>(check_every, maxiter - it);
             for (int64_t k = 0; k < nb && rc == GFGPU_OK; ++k) {
-                rc = iteration(c, s);
+                rc = iteration(c, true, s);
                 ++it;
                 c += ndir;
                 if (!exec && c >= int64_t(nkeep) + ndir && c % nslots == 0 && maxiter - it >= chunk) break;
@@ -2377,9 +2393,9 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
     GF_TRY(rc);
     // true residual -(A x)_u
     GF_TRY(gfgpu_internal_element_forces(d, x, w.fe, s));
-    k_fres<<<gb, 256, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.r,
+    k_fres<<<rs.grid, rs.block, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.r,
                               w.partial, reg_grid(d));
-    k_fredv<<<1, 1024, 0, s>>>(w.partial, static_cast<int>(gb), one(F_RR), w.sc);
+    k_fredv<<<1, kWide, 0, s>>>(w.partial, ROW_RR, nr, F_RR, w.sc);
     GF_TRY(read_sc());
     *iters = it;
     *relres = std::sqrt(h[F_RR]) / bnorm;
