@@ -4,6 +4,7 @@
 // operators, one thread per element for the integrals that sum over the integration points, so
 // every output entry is summed in the reference's order.
 #include "common.cuh"
+#include "fixdot.cuh"
 
 namespace gfgpu {
 
@@ -486,7 +487,7 @@ __global__ void k_int_tensor4_strict(const double* __restrict__ dNx, const doubl
 // row (m, j) and the columns (n, k) of one k, so that its T never leaves registers; the NNE * ND^2
 // threads of an element read its tensors, gradients and v * gradients from shared memory, filled
 // (and the matrices written back) in address order. EPB elements per block make whole warps
-// (16 x 16 and 72 x 4 threads).
+// (16 x 16 and 72 x 4 threads). For rules other than the Gauss ones (k_int_tensor4_fix).
 template <int NNE, int ND>
 struct Tensor4Block {
     static constexpr int K = NNE * ND, C4 = ND * ND * ND * ND, G = NNE * ND;
@@ -566,16 +567,197 @@ k_int_tensor4(const double* __restrict__ dNx, const double* __restrict__ vol,
     }
 }
 
+// The same two contractions on the integer pipes (fixdot.cuh) for the Gauss rules (NNE points): FP64
+// issue bounds the kernel above at 200 and 2400 instructions per integration point. The tensors, the
+// gradients and the volume * gradients of an element are brought to one exponent each over all its
+// points, so that the entries of its matrix are integer sums until the end. A thread (m, j, k) loads
+// the (j, k) block of the tensor of point m and a few gradients of one direction, the largest exponents
+// per block and direction meet in shared memory, and the threads leave the limbs of what they loaded
+// there for all. An entry is judged by the largest terms that its block and directions can have: an
+// element whose blocks or directions differ by more than 2^24 in all (thin elements, tensors with one
+// weak block), or whose values leave the range, takes the FP64 form on operands in global memory.
+// 9177 Hex8 elements 326 -> 203 us against the FP64 form, 49k Quad4 80 -> 61 us, with a third of its
+// error; the integer multiply-add pipe is 59 % busy (half of it the multiply-adds, the rest the
+// conversions), 2 blocks per SM (registers).
+template <int NNE, int ND>
+struct Tensor4Fix {
+    static constexpr int K = NNE * ND, C4 = ND * ND * ND * ND, G = NNE * ND, JK = ND * ND;
+    static constexpr int TPE = NNE * ND * ND;
+    static constexpr int EPB = ND == 2 ? 16 : 4;
+    static constexpr int THREADS = TPE * EPB;
+    static constexpr int NE = JK + 2 * ND; // exponents per element: (j, k) blocks, gradients, v * gradients
+    static constexpr int NG = NNE * G;     // gradients per element
+    static constexpr int SL = NNE * (C4 + 2 * G) + 1; // limbs per element (+ 1: elements on other banks)
+    // the limbs, or the matrices that take their place, then the exponents
+    static constexpr size_t BODY = sizeof(int4) * EPB * SL > sizeof(double) * EPB * K * K ? sizeof(int4) * EPB * SL
+                                                                                         : sizeof(double) * EPB * K * K;
+    static constexpr size_t SMEM = BODY + sizeof(int) * EPB * NE;
+};
+
+template <int NNE, int ND, int TD>
+__global__ void __launch_bounds__(Tensor4Fix<NNE, ND>::THREADS, 2)
+k_int_tensor4_fix(const double* __restrict__ dNx, const double* __restrict__ vol, const double* __restrict__ C,
+                  int64_t nelem, double* __restrict__ elemmat)
+{
+    using B = Tensor4Fix<NNE, ND>;
+    constexpr int K = B::K, C4 = B::C4, G = B::G, JK = B::JK, T4 = TD * TD * TD * TD, NE = B::NE, SL = B::SL;
+    constexpr int TPE = B::TPE, NG = B::NG, GT = (NG + TPE - 1) / TPE; // gradients per thread
+    static_assert(3 * ND * NNE < 128, "ND * NNE products of limbs fit a 64-bit sum");
+    static_assert(TPE % ND == 0, "a thread's gradients are of one direction");
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int tid = threadIdx.x;
+    const int el = tid / TPE, r = tid - el * TPE;
+    const int m = r / (ND * ND), j = (r / ND) % ND, k = r % ND;
+    const int64_t e0 = static_cast<int64_t>(blockIdx.x) * B::EPB;
+    const int ne = static_cast<int>(nelem - e0 < B::EPB ? nelem - e0 : B::EPB);
+    const bool on = el < ne;
+    int4* lim = reinterpret_cast<int4*>(smem) + el * SL;
+    double* out = reinterpret_cast<double*>(smem);
+    int* ex = reinterpret_cast<int*>(smem + B::BODY) + el * NE;
+    if (r < NE) ex[r] = 0;
+    // this thread's values: point m's C[i, j, k, l], and gradients r, r + TPE, ... of the element
+    const double* Ce = C + (e0 + el) * NNE * T4;
+    const double* ge = dNx + (e0 + el) * NG;
+    double c[JK], g[GT], gv[GT];
+    int xc = 0, xg = 0, xv = 0;
+    if (on) {
+#pragma unroll
+        for (int t = 0; t < JK; ++t) {
+            c[t] = __ldg(Ce + m * T4 + (((t / ND) * TD + j) * TD + k) * TD + t % ND);
+            xc = max(xc, fx_exponent(c[t]));
+        }
+#pragma unroll
+        for (int t = 0; t < GT; ++t) {
+            const int y = r + t * TPE;
+            g[t] = gv[t] = 0.0;
+            if (y < NG) {
+                g[t] = __ldg(ge + y);
+                gv[t] = __ldg(vol + (e0 + el) * NNE + y / G) * g[t];
+            }
+            xg = max(xg, fx_exponent(g[t]));
+            xv = max(xv, fx_exponent(gv[t]));
+        }
+    }
+    __syncthreads();
+    if (on) {
+        atomicMax(ex + j * ND + k, xc);
+        atomicMax(ex + JK + r % ND, xg);
+        atomicMax(ex + JK + ND + r % ND, xv);
+    }
+    __syncthreads();
+    // the largest exponents, and how far the scales lie apart
+    int ec = 0, eg = 0, ev = 0;
+    bool fix = false;
+    if (on) {
+        int lc = 0x7ff, lg = 0x7ff, lv = 0x7ff;
+#pragma unroll
+        for (int b = 0; b < JK; ++b) {
+            ec = max(ec, ex[b]);
+            if (ex[b]) lc = min(lc, ex[b]); // a block of zeros is exact
+        }
+#pragma unroll
+        for (int i = 0; i < ND; ++i) {
+            eg = max(eg, ex[JK + i]);
+            lg = min(lg, ex[JK + i]);
+            ev = max(ev, ex[JK + ND + i]);
+            lv = min(lv, ex[JK + ND + i]);
+        }
+        const int sum = ec + eg + ev - 3 * 1022;
+        fix = ec > 100 && eg > 100 && ev > 100 && ec < 0x7ff && eg < 0x7ff && ev < 0x7ff && sum > -800 && sum < 900 &&
+              (ec - lc) + (eg - lg) + (ev - lv) <= 24;
+        if (fix) {
+#pragma unroll
+            for (int t = 0; t < JK; ++t) lim[m * C4 + ((t / ND * ND + j) * ND + k) * ND + t % ND] = fx_from_double(c[t], ec);
+#pragma unroll
+            for (int t = 0; t < GT; ++t) {
+                const int y = r + t * TPE;
+                if (y < NG) {
+                    lim[NNE * C4 + y] = fx_from_double(g[t], eg);
+                    lim[NNE * C4 + NG + y] = fx_from_double(gv[t], ev);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    double res[NNE];
+    if (fix) {
+        FxSum acc[NNE];
+#pragma unroll
+        for (int n = 0; n < NNE; ++n) fx_zero(acc[n]);
+        const int4* lc = lim + (j * ND + k) * ND;
+        const int4* lg = lim + NNE * C4;
+        const int4* lv = lg + NG + m * ND;
+#pragma unroll 1
+        for (int q = 0; q < NNE; ++q, lc += C4, lg += G, lv += G) {
+            int4 t[ND];
+#pragma unroll
+            for (int l = 0; l < ND; ++l) {
+                FxSum s;
+                fx_zero(s);
+#pragma unroll
+                for (int i = 0; i < ND; ++i) fx_mad(s, lv[i], lc[i * ND * ND * ND + l]);
+                t[l] = fx_limbs(s);
+            }
+#pragma unroll
+            for (int n = 0; n < NNE; ++n)
+#pragma unroll
+                for (int l = 0; l < ND; ++l) fx_mad(acc[n], t[l], lg[n * ND + l]);
+        }
+        const int scale = ec + ev + eg - 3 * 1022 + 2;
+#pragma unroll
+        for (int n = 0; n < NNE; ++n) res[n] = fx_to_double(acc[n], scale);
+    }
+    else if (on) {
+#pragma unroll
+        for (int n = 0; n < NNE; ++n) res[n] = 0.0;
+#pragma unroll 1
+        for (int q = 0; q < NNE; ++q) {
+            const double* cq = Ce + q * T4;
+            const double* gq = ge + q * G;
+            const double v = __ldg(vol + (e0 + el) * NNE + q);
+            double t[ND];
+#pragma unroll
+            for (int l = 0; l < ND; ++l) {
+                t[l] = 0.0;
+#pragma unroll
+                for (int i = 0; i < ND; ++i)
+                    t[l] = fma(v * __ldg(gq + m * ND + i), __ldg(cq + ((i * TD + j) * TD + k) * TD + l), t[l]);
+            }
+#pragma unroll
+            for (int n = 0; n < NNE; ++n)
+#pragma unroll
+                for (int l = 0; l < ND; ++l) res[n] = fma(t[l], __ldg(gq + n * ND + l), res[n]);
+        }
+    }
+    __syncthreads(); // the limbs are read: the matrices take their place
+    if (on)
+#pragma unroll
+        for (int n = 0; n < NNE; ++n) out[el * K * K + (m * ND + j) * K + n * ND + k] = res[n];
+    __syncthreads();
+    for (int i = tid; i < ne * K * K; i += B::THREADS) elemmat[e0 * K * K + i] = out[i];
+}
+
 template <int NNE, int ND, int TD = ND>
-static void launch_int_tensor4(const double* dNx, const double* vol, const double* C, int64_t nelem, int nip,
-                               double* elemmat, cudaStream_t s)
+static int launch_int_tensor4(const double* dNx, const double* vol, const double* C, int64_t nelem, int nip,
+                              double* elemmat, cudaStream_t s)
 {
     using B = Tensor4Block<NNE, ND>;
-    if (strict_mode())
+    using X = Tensor4Fix<NNE, ND>;
+    if (strict_mode()) {
         k_int_tensor4_strict<<<grid_for(nelem * B::K * B::K), kBlock, 0, s>>>(dNx, vol, C, nelem, NNE, nip, ND, TD,
                                                                              elemmat);
-    else
+    }
+    else if (nip == NNE) {
+        // 66 KB of limbs for 4 Hex8 elements
+        auto kernel = k_int_tensor4_fix<NNE, ND, TD>;
+        GF_TRY(check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(X::SMEM)),
+                          "cudaFuncSetAttribute"));
+        kernel<<<grid_for(nelem, X::EPB), X::THREADS, X::SMEM, s>>>(dNx, vol, C, nelem, elemmat);
+    }
+    else {
         k_int_tensor4<NNE, ND, TD><<<grid_for(nelem, B::EPB), B::THREADS, 0, s>>>(dNx, vol, C, nelem, nip, elemmat);
+    }
+    return GFGPU_OK;
 }
 
 // Linear elastic stress (plane strain for nd = 2), strict arithmetic: the oracle's operation order.
@@ -867,9 +1049,9 @@ int gfgpu_int_grad_n_dot_tensor4_dot_grad_nt_dv(const double* dNx, const double*
     GF_REQUIRE(!too_big(nelem * K * K), "too many elements");
     if (nelem == 0) return GFGPU_OK;
     if (ndim == 2)
-        launch_int_tensor4<4, 2>(dNx, vol, qtensor4, nelem, nip, elemmat, S(stream));
+        GF_TRY((launch_int_tensor4<4, 2>(dNx, vol, qtensor4, nelem, nip, elemmat, S(stream))));
     else
-        launch_int_tensor4<8, 3>(dNx, vol, qtensor4, nelem, nip, elemmat, S(stream));
+        GF_TRY((launch_int_tensor4<8, 3>(dNx, vol, qtensor4, nelem, nip, elemmat, S(stream))));
     return check_launch("int_grad_n_dot_tensor4_dot_grad_nt_dv");
 }
 
@@ -922,7 +1104,7 @@ int gfgpu_int_grad_n_dot_tensor4_dot_grad_nt_dv_planar(const double* dNx, const 
     GF_REQUIRE(dNx && vol && qtensor4 && elemmat && nip > 0, "bad argument");
     GF_REQUIRE(!too_big(nelem * 64) && !too_big(nelem * nip * 81), "too many elements");
     if (nelem == 0) return GFGPU_OK;
-    launch_int_tensor4<4, 2, 3>(dNx, vol, qtensor4, nelem, nip, elemmat, S(stream));
+    GF_TRY((launch_int_tensor4<4, 2, 3>(dNx, vol, qtensor4, nelem, nip, elemmat, S(stream))));
     return check_launch("int_grad_n_dot_tensor4_dot_grad_nt_dv_planar");
 }
 

@@ -135,3 +135,55 @@ def test_unaligned_vectors(gf):
             want = ue.clone(), sig.clone()
     assert torch.equal(ue, want[0]) and torch.equal(sig, want[1])
     assert torch.equal(ue.reshape(ne, 4, 2), u[conn.long()])
+
+
+def _stiffness_bound(dNx, vol, C):
+    """Sum of the magnitudes of an entry's terms: 2^-53 of it is one rounding."""
+    a = np.abs
+    t = np.einsum("eqmi,eqijkl->eqmjkl", a(dNx), a(C) * vol[..., None, None, None, None])
+    k = dNx.shape[2] * dNx.shape[3]
+    return np.einsum("eqmjkl,eqnl->emjnk", t, a(dNx)).reshape(-1, k, k)
+
+
+@pytest.mark.parametrize("nd", [2, 3])
+@pytest.mark.parametrize("stretch,scale", [(1.0, "one"), (40.0, "one"), (1e5, "one"), (1.0, "wide"), (1.0, "blocks"),
+                                           (1.0, "huge"), (1.0, "tiny"), (1e-3, "zero")])
+def test_stiffness_scales(gf, oracle, nd, stretch, scale):
+    """Thin elements and tensors whose entries or blocks lie far apart: every entry to within 64
+    roundings of its terms (the oracle's own sum of 64 to 72 terms takes up to as many; integer sums
+    and the FP64 form for what they do not cover)."""
+    R = oracle
+    x = _elements(37, nd, 5)
+    x[..., 0] *= stretch
+    quad = (gf.Element.Quad4 if nd == 2 else gf.Element.Hex8).Quadrature(x)
+    dNx, vol = R.compute_dN(x, *(R.quad4_gauss() if nd == 2 else R.hex8_gauss()))
+    C = seeded_field(vol.shape + (nd,) * 4, 6)
+    if scale == "wide":
+        C *= 10.0 ** (6.0 * seeded_field(C.shape, 7) - 6.0)
+    elif scale == "blocks":
+        C[:, :, :, 0, 1, :] *= 1e-14
+        C[:, :, :, 1, 0, :] = 0.0
+    elif scale in ("huge", "tiny"):
+        C *= 1e300 if scale == "huge" else 1e-300
+    elif scale == "zero":
+        C[::2] = 0.0
+    ref = R.int_grad_n_dot_tensor4_dot_grad_nt_dv(dNx, vol, C)
+    err = np.abs(to_np(quad.Int_gradN_dot_tensor4_dot_gradNT_dV(C)) - ref)
+    assert np.all(err <= 64 * 2.0 ** -53 * _stiffness_bound(dNx, vol, C))
+
+
+@pytest.mark.parametrize("nd", [2, 3])
+def test_stiffness_not_finite(gf, oracle, nd):
+    """An infinite and a NaN tensor entry reach the entries that they take part in, and no others."""
+    R = oracle
+    x = _elements(21, nd, 8)
+    quad = (gf.Element.Quad4 if nd == 2 else gf.Element.Hex8).Quadrature(x)
+    dNx, vol = R.compute_dN(x, *(R.quad4_gauss() if nd == 2 else R.hex8_gauss()))
+    C = seeded_field(vol.shape + (nd,) * 4, 9)
+    C[3, 1, 0, 1, 0, 1] = np.inf
+    C[17, 2, 1, 0, 0, 0] = np.nan
+    ref = R.int_grad_n_dot_tensor4_dot_grad_nt_dv(dNx, vol, C)
+    got = to_np(quad.Int_gradN_dot_tensor4_dot_gradNT_dV(C))
+    assert np.array_equal(np.isfinite(got), np.isfinite(ref)) and not np.isfinite(ref).all()
+    ok = np.isfinite(ref)
+    assert rel_err(got[ok], ref[ok]) <= RTOL
