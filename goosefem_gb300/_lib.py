@@ -38,6 +38,7 @@ class VerletDesc(C.Structure):
         ("reg_nx", C.c_int64), ("reg_ny", C.c_int64), ("reg_nz", C.c_int64),
         ("coef_pair", C.c_void_p), ("pair_mode", C.c_int32),
         ("pcg_pair", C.c_void_p), ("ell", C.c_void_p),
+        ("tiles", C.c_void_p), ("ntiles", C.c_int32), ("tile_edge", C.c_int32),
     ]
 
 

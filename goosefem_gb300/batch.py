@@ -86,6 +86,7 @@ class BatchedVerlet:
                                  dt=self.dt, eta=eta, iip=None)
         if not self.vv.uniform:
             raise RuntimeError("batched instances must be uniform Quad4 meshes")
+        self.vv._detect_blocks([(i.nx, i.ny) for i in instances])
         nbytes = int(_lib.lib().gfgpu_verlet_persistent_workspace_bytes(C.addressof(self.vv.desc)))
         self.pws = torch.empty(nbytes // 8 + 1, dtype=torch.float64, device=_dev.device())
         self.vv.use_mixed()  # pair element coefficients for mode 3 (FP64 state)

@@ -20,6 +20,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "quad4_square.cuh"
 
 #include <string>
 #include <vector>
@@ -302,21 +303,11 @@ __device__ __forceinline__ void quad4_square_elem(int64_t e, const int32_t* __re
             u3 = ld2<CG>(u2 + cn.w);
     double2 c01 = __ldg(reinterpret_cast<const double2*>(coef) + 2 * e);
     double2 c23 = __ldg(reinterpret_cast<const double2*>(coef) + 2 * e + 1);
-    double L = c01.x, M = c01.y, N = c23.x, kH = c23.y;
-    double px = u2v.x - u0.x, qx = u1.x - u3.x;
-    double py = u2v.y - u0.y, qy = u1.y - u3.y;
-    double A1x = px + qx, A2x = px - qx, A3x = (u0.x + u2v.x) - (u1.x + u3.x);
-    double A1y = py + qy, A2y = py - qy, A3y = (u0.y + u2v.y) - (u1.y + u3.y);
-    double Lt = L * (A1x + A2y);
-    double P0 = fma(M, A1x, Lt), Q1 = fma(M, A2y, Lt);
-    double P1 = N * (A1y + A2x); // = Q0
-    double H0 = kH * A3x, H1 = kH * A3y;
-    double Sx = P0 + P1, Dx = P0 - P1, Sy = P1 + Q1, Dy = P1 - Q1;
+    double2 f[4];
+    quad4_square_forces(u0, u1, u2v, u3, c01, c23, f);
     double2* fo = reinterpret_cast<double2*>(fe) + e * 4;
-    fo[0] = make_double2(H0 - Sx, H1 - Sy);
-    fo[1] = make_double2(Dx - H0, Dy - H1);
-    fo[2] = make_double2(Sx + H0, Sy + H1);
-    fo[3] = make_double2(-(Dx + H0), -(Dy + H1));
+#pragma unroll
+    for (int m = 0; m < 4; ++m) fo[m] = f[m];
 }
 
 __global__ void __launch_bounds__(256, 4)
@@ -645,17 +636,13 @@ k_elem_force_hex8_cube(const int32_t* __restrict__ conn, const double* u,
 
 // ------------------------------------------------------------------ node kernels
 
-struct VerletCoef {
-    double dt, h, c, eta; // h = 0.5 dt, c = 0.5 dt^2
-};
-
-// u = u + dt v + 0.5 dt^2 a (main.cpp:119), with the same arithmetic as the predictor that the
+// uout = u + dt v + 0.5 dt^2 a (main.cpp:119; uout may be u), with the same arithmetic as the predictor that the
 // node kernels fuse into the previous increment, so that split and single calls agree bit for bit.
 template <bool S>
-__global__ void k_predict(double* __restrict__ u, const double* __restrict__ v,
+__global__ void k_predict(const double* u, double* uout, const double* __restrict__ v,
                           const double* __restrict__ a, int64_t n, VerletCoef k)
 {
-    GF_FOR(t, n) u[t] = madd<S>(k.c, a[t], madd<S>(k.dt, v[t], u[t]));
+    GF_FOR(t, n) uout[t] = madd<S>(k.c, a[t], madd<S>(k.dt, v[t], u[t]));
 }
 
 // One node-dof t of the increment: fint by the CSR gather, three velocity estimates, predictor.
@@ -787,18 +774,6 @@ __global__ void k_build_ell(const int32_t* __restrict__ dofs, const int32_t* __r
     }
 }
 
-// Per-class coefficients of the three velocity estimates in closed form. With be = m^-1 eta,
-// h = dt/2 and mR = m^-1 (fext - f), the sequence v1 = v + dt a, a1 = mR - be v1, w = v + h a,
-// v2 = w + h a1, a2 = mR - be v2, v' = w + h a2, a' = mR - be v' is
-//   v' = c1 v + c2 a + c3 mR,  c1 = (1 - h be) + h^2 be^2,  c2 = h (1 - h be) + h^2 be^2 dt,
-//   c3 = h (1 - h be),  a' = mR - be v'
-// (10 FP64 instructions per free dof instead of 14).
-struct MassClassTab {
-    int n;
-    double mi[GFGPU_MASS_CLASSES], be[GFGPU_MASS_CLASSES], c1[GFGPU_MASS_CLASSES],
-        c2[GFGPU_MASS_CLASSES], c3[GFGPU_MASS_CLASSES];
-};
-
 __global__ void __launch_bounds__(256)
 k_verlet_node_cls(const int32_t* __restrict__ dofs, const int32_t* __restrict__ ptr,
                   const int32_t* __restrict__ idx, const int4* __restrict__ ell, const uint8_t* __restrict__ mclass,
@@ -806,15 +781,8 @@ k_verlet_node_cls(const int32_t* __restrict__ dofs, const int32_t* __restrict__ 
                   int64_t n, VerletCoef k, int advance, double* __restrict__ u,
                   double* __restrict__ v, double* __restrict__ a)
 {
-    __shared__ double sm[5][GFGPU_MASS_CLASSES];
-    if (threadIdx.x < GFGPU_MASS_CLASSES) {
-        int c = threadIdx.x;
-        sm[0][c] = tab.mi[c];
-        sm[1][c] = tab.be[c];
-        sm[2][c] = tab.c1[c];
-        sm[3][c] = tab.c2[c];
-        sm[4][c] = tab.c3[c];
-    }
+    __shared__ MassClassShared sm;
+    sm.load(tab);
     pdl_wait();
     __syncthreads();
     GF_FOR(t, n)
@@ -837,16 +805,7 @@ k_verlet_node_cls(const int32_t* __restrict__ dofs, const int32_t* __restrict__ 
         int c = __ldg(mclass + t);
         double vn = v[t], an = a[t];
         double vv, aa;
-        if (c < GFGPU_MASS_CLASSES) {
-            double mi = sm[0][c];
-            double mR = fext ? mi * (__ldg(fext + t) - fint) : -mi * fint;
-            vv = fma(sm[4][c], mR, fma(sm[3][c], an, sm[2][c] * vn));
-            aa = fma(-sm[1][c], vv, mR);
-        }
-        else {
-            aa = an;
-            vv = fma(k.h, an + an, vn);
-        }
+        sm.update(c, fint, fext != nullptr, fext ? __ldg(fext + t) : 0.0, vn, an, k.h, vv, aa);
         v[t] = vv;
         a[t] = aa;
         if (advance) u[t] = fma(k.c, aa, fma(k.dt, vv, u[t]));
@@ -863,15 +822,8 @@ k_verlet_node_cls_regular(int64_t nx, int64_t ny, const uint8_t* __restrict__ mc
                           const double* __restrict__ fext, VerletCoef k, int advance,
                           double* __restrict__ u, double* __restrict__ v, double* __restrict__ a)
 {
-    __shared__ double sm[5][GFGPU_MASS_CLASSES];
-    if (threadIdx.x < GFGPU_MASS_CLASSES) {
-        int c = threadIdx.x;
-        sm[0][c] = tab.mi[c];
-        sm[1][c] = tab.be[c];
-        sm[2][c] = tab.c1[c];
-        sm[3][c] = tab.c2[c];
-        sm[4][c] = tab.c3[c];
-    }
+    __shared__ MassClassShared sm;
+    sm.load(tab);
     pdl_wait();
     __syncthreads();
     const int64_t W = nx + 1, nnode = W * (ny + 1);
@@ -907,19 +859,7 @@ k_verlet_node_cls_regular(int64_t nx, int64_t ny, const uint8_t* __restrict__ mc
                      fxi[2] = {fx2.x, fx2.y};
         const int ci[2] = {cc.x, cc.y};
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            int c = ci[i];
-            if (c < GFGPU_MASS_CLASSES) {
-                double mi = sm[0][c];
-                double mR = fext ? mi * (fxi[i] - fi[i]) : -mi * fi[i];
-                vv[i] = fma(sm[4][c], mR, fma(sm[3][c], ai[i], sm[2][c] * vi[i]));
-                aa[i] = fma(-sm[1][c], vv[i], mR);
-            }
-            else {
-                aa[i] = ai[i];
-                vv[i] = fma(k.h, ai[i] + ai[i], vi[i]);
-            }
-        }
+        for (int i = 0; i < 2; ++i) sm.update(ci[i], fi[i], fext != nullptr, fxi[i], vi[i], ai[i], k.h, vv[i], aa[i]);
         reinterpret_cast<double2*>(v)[node] = make_double2(vv[0], vv[1]);
         reinterpret_cast<double2*>(a)[node] = make_double2(aa[0], aa[1]);
         if (advance) {
@@ -1203,6 +1143,13 @@ int gfgpu_internal_pair_element_forces_f64(const gfgpu_verlet_desc* d, const dou
 int gfgpu_internal_mixed_increment(const gfgpu_verlet_desc* d, double* fe, int advance, double* u, double* v,
                                    double* a, cudaStream_t s);
 
+// one increment by the tile kernel (verlet_pair.cu): its tile edge, 0 if it does not apply
+int gfgpu_internal_tile_edge(const gfgpu_verlet_desc* d, bool mixed, const double* u, const double* v,
+                             const double* a, const double* scratch);
+int gfgpu_internal_tile_increment(const gfgpu_verlet_desc* d, const MassClassTab& tab, const VerletCoef& k, int edge,
+                                  bool mixed, const double* uin, double* uout, int advance, double* v, double* a,
+                                  cudaStream_t s);
+
 // "Mixed" arithmetic: in fast mode with d->pcg_pair set on a uniform square Quad4 mesh, the FP64
 // state with the element forces of the pair closed form (on node differences formed in FP64).
 static bool mixed_arithmetic(const gfgpu_verlet_desc* d)
@@ -1305,16 +1252,26 @@ static int run_increments(const gfgpu_verlet_desc* d, double* u, double* v, doub
     const Shape l = spread(n);
     MassClassTab tab;
     GF_TRY(mass_class_tab(d, k, &tab));
-    if (strict_mode())
-        k_predict<true><<<l.grid, l.block, 0, s>>>(u, v, a, n, k);
-    else
-        k_predict<false><<<l.grid, l.block, 0, s>>>(u, v, a, n, k);
-    GF_TRY(check_launch("verlet predict"));
     // mixed arithmetic with lumped-mass classes: the element forces stay pairs and the node kernel
     // takes the velocity estimates on pairs (4 FP64 instructions per free dof instead of 10)
     const bool mixed_cls = mixed_arithmetic(d) && d->mclass && d->mclass_inv && d->ncls > 0;
+    // the tile kernel reads one displacement buffer and writes the other (fe, which it does not need for
+    // forces, holds at least as many values); the last increment has to read the caller's
+    const int edge = gfgpu_internal_tile_edge(d, mixed_cls, u, v, a, fe);
+    double* const ub[2] = {u, edge ? fe : u};
+    int64_t at = (nsteps - 1) & 1;
+    if (strict_mode())
+        k_predict<true><<<l.grid, l.block, 0, s>>>(u, u, v, a, n, k);
+    else
+        k_predict<false><<<l.grid, l.block, 0, s>>>(u, ub[at], v, a, n, k);
+    GF_TRY(check_launch("verlet predict"));
     for (int64_t it = 0; it < nsteps; ++it) {
         const int adv = it + 1 < nsteps ? 1 : 0;
+        if (edge) {
+            GF_TRY(gfgpu_internal_tile_increment(d, tab, k, edge, mixed_cls, ub[at], ub[at ^ 1], adv, v, a, s));
+            at ^= 1;
+            continue;
+        }
         if (mixed_cls) {
             GF_TRY(gfgpu_internal_mixed_increment(d, fe, adv, u, v, a, s));
             continue;

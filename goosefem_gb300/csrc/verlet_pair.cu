@@ -24,10 +24,13 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
+#include <vector>
 
 #include "common.cuh"
 #include "ffpair.cuh"
 #include "ffpair2.cuh"
+#include "quad4_square.cuh"
 
 namespace gfgpu {
 
@@ -655,6 +658,26 @@ k_pair_elem_square(const int32_t* __restrict__ conn, const float4* u, const floa
     }
 }
 
+// Pair forces {x, y} of nodes 0..3 of a square element from FP64 nodal displacements (coefficients
+// {L, N} and kH as pairs).
+__device__ __forceinline__ void pair_square_forces(double2 q0, double2 q1, double2 q2, double2 q3, float4 cln,
+                                                   float2 ch, ffv (&f)[8])
+{
+    float4 S, D, H;
+    pair_element_diff(ff_from_double(q2.x - q0.x), ff_from_double(q2.y - q0.y), ff_from_double(q1.x - q3.x),
+                      ff_from_double(q1.y - q3.y), ff_from_double(q0.x - q1.x), ff_from_double(q0.y - q1.y),
+                      ff_from_double(q2.x - q3.x), ff_from_double(q2.y - q3.y), lo2(cln), hi2(cln), pf(ch), S, D, H);
+    const ffv Sx = lo2(S), Sy = hi2(S), Dx = lo2(D), Dy = hi2(D), H0 = lo2(H), H1 = hi2(H);
+    f[0] = ff_sub(H0, Sx);
+    f[1] = ff_sub(H1, Sy);
+    f[2] = ff_sub(Dx, H0);
+    f[3] = ff_sub(Dy, H1);
+    f[4] = ff_add(Sx, H0);
+    f[5] = ff_add(Sy, H1);
+    f[6] = ff_neg(ff_add(Dx, H0));
+    f[7] = ff_neg(ff_add(Dy, H1));
+}
+
 // Element forces of uniform square Quad4 elements in pair arithmetic with FP64 input and output
 // (the static solvers' operator and the explicit step's element kernel in "mixed" arithmetic): the
 // node differences of the square closed form are formed in FP64 (8 subtractions), split into pairs
@@ -676,14 +699,8 @@ k_pair_elem_square_f64(const int32_t* __restrict__ conn, const double2* u,
         const int4 cn = __ldg(reinterpret_cast<const int4*>(conn) + e);
         const double2 q0 = u[cn.x], q1 = u[cn.y], q2 = u[cn.z], q3 = u[cn.w];
         const float4 cln = __ldg(cLN + e);
-        float4 S, D, H;
-        pair_element_diff(ff_from_double(q2.x - q0.x), ff_from_double(q2.y - q0.y), ff_from_double(q1.x - q3.x),
-                          ff_from_double(q1.y - q3.y), ff_from_double(q0.x - q1.x), ff_from_double(q0.y - q1.y),
-                          ff_from_double(q2.x - q3.x), ff_from_double(q2.y - q3.y), lo2(cln), hi2(cln),
-                          pf(__ldg(cH + e)), S, D, H);
-        const ffv Sx = lo2(S), Sy = hi2(S), Dx = lo2(D), Dy = hi2(D), H0 = lo2(H), H1 = hi2(H);
-        const ffv f[8] = {ff_sub(H0, Sx), ff_sub(H1, Sy), ff_sub(Dx, H0), ff_sub(Dy, H1),
-                          ff_add(Sx, H0), ff_add(Sy, H1), ff_neg(ff_add(Dx, H0)), ff_neg(ff_add(Dy, H1))};
+        ffv f[8];
+        pair_square_forces(q0, q1, q2, q3, cln, __ldg(cH + e), f);
         if constexpr (PAIR_OUT) {
             float4* o = reinterpret_cast<float4*>(fe) + e * 4;
 #pragma unroll
@@ -703,6 +720,41 @@ k_pair_elem_square_f64(const int32_t* __restrict__ conn, const double2* u,
 // estimates with the lumped-mass class's coefficients on pairs (v and a split from FP64 on the
 // integer pipe), v' and a' returned to FP64, and the predictor u + dt v' + c a' in FP64 as in
 // k_verlet_node_cls. 4 FP64 instructions per free dof instead of 10; prescribed dofs as there.
+struct PairClassShared {
+    float2 mi[GFGPU_MASS_CLASSES], be[GFGPU_MASS_CLASSES], c1[GFGPU_MASS_CLASSES], c2[GFGPU_MASS_CLASSES],
+        c3[GFGPU_MASS_CLASSES];
+    __device__ __forceinline__ void load(const PairClassTab& tab)
+    {
+        const int c = threadIdx.x;
+        if (c < GFGPU_MASS_CLASSES) {
+            mi[c] = tab.mi[c];
+            be[c] = tab.be[c];
+            c1[c] = tab.c1[c];
+            c2[c] = tab.c2[c];
+            c3[c] = tab.c3[c];
+        }
+    }
+    // mixed arithmetic: one component of class c, pair force f, FP64 state
+    __device__ __forceinline__ void update(int c, ffv f, bool has_fext, double fx, double vn, double an, double h,
+                                           double& vv, double& aa) const
+    {
+        if (c < GFGPU_MASS_CLASSES) {
+            const ffv R = has_fext ? ff_sub(ff_from_double(fx), f) : ff_neg(f);
+            const ffv mR = ff_mul(pf(mi[c]), R);
+            const ffv V = ff_add(ff_add(ff_mul(pf(c1[c]), ff_from_double(vn)), ff_mul(pf(c2[c]), ff_from_double(an))),
+                                 ff_mul(pf(c3[c]), mR));
+            const ffv Vn = ff_norm(V);
+            const ffv Ac = ff_sub(mR, ff_mul(pf(be[c]), Vn));
+            vv = ff_to_double(Vn);
+            aa = ff_to_double(Ac);
+        }
+        else {
+            aa = an;
+            vv = fma(h, an + an, vn);
+        }
+    }
+};
+
 struct MixedNodeStep {
     const int32_t *dofs, *ptr, *idx;
     const uint8_t* mclass;
@@ -718,16 +770,8 @@ struct MixedNodeStep {
 __global__ void __launch_bounds__(256)
 k_mixed_node(const MixedNodeStep p, const __grid_constant__ PairClassTab tab)
 {
-    __shared__ float2 smi[GFGPU_MASS_CLASSES], sbe[GFGPU_MASS_CLASSES], sc1[GFGPU_MASS_CLASSES],
-        sc2[GFGPU_MASS_CLASSES], sc3[GFGPU_MASS_CLASSES];
-    if (threadIdx.x < GFGPU_MASS_CLASSES) {
-        const int c = threadIdx.x;
-        smi[c] = tab.mi[c];
-        sbe[c] = tab.be[c];
-        sc1[c] = tab.c1[c];
-        sc2[c] = tab.c2[c];
-        sc3[c] = tab.c3[c];
-    }
+    __shared__ PairClassShared sm;
+    sm.load(tab);
     pdl_wait();
     __syncthreads();
     GF_FOR(t, p.n)
@@ -762,24 +806,171 @@ k_mixed_node(const MixedNodeStep p, const __grid_constant__ PairClassTab tab)
         const int c = __ldg(p.mclass + t);
         const double vn = p.v[t], an = p.a[t];
         double vv, aa;
-        if (c < GFGPU_MASS_CLASSES) {
-            const ffv R = p.fext ? ff_sub(ff_from_double(__ldg(p.fext + t)), f) : ff_neg(f);
-            const ffv mR = ff_mul(pf(smi[c]), R);
-            const ffv V = ff_add(ff_add(ff_mul(pf(sc1[c]), ff_from_double(vn)), ff_mul(pf(sc2[c]), ff_from_double(an))),
-                                 ff_mul(pf(sc3[c]), mR));
-            const ffv Vn = ff_norm(V);
-            const ffv Ac = ff_sub(mR, ff_mul(pf(sbe[c]), Vn));
-            vv = ff_to_double(Vn);
-            aa = ff_to_double(Ac);
-        }
-        else {
-            aa = an;
-            vv = fma(p.h, an + an, vn);
-        }
+        sm.update(c, f, p.fext != nullptr, p.fext ? __ldg(p.fext + t) : 0.0, vn, an, p.h, vv, aa);
         p.v[t] = vv;
         p.a[t] = aa;
         if (p.advance) p.u[t] = fma(p.c, aa, fma(p.dt, vv, p.u[t]));
     }
+}
+
+// One increment of a mesh of square Quad4 elements with a grid numbering in one kernel, FP64 (PAIR
+// false) or mixed arithmetic: a block of T x T threads takes the T x T elements around a tile of
+// (T - 1) x (T - 1) nodes (the elements on the rim are computed by both neighbours), keeps their forces
+// in shared memory and updates the nodes from there. The formulas and the order of the sums are those of
+// the two-kernel increment (quad4_square_forces / pair_square_forces, ascending element index,
+// MassClassShared / PairClassShared), the forces never reach memory and the displacement is
+// double-buffered: neighbours read it while a block updates its nodes.
+// The grid is Regular(nx, ny) (tiles null) or, per tile, the record {node0, elem0, nx, ny},
+// {x0, y0, periodic, 0} of one of many meshes; a periodic mesh takes the elements across its edges, and
+// the nodes of both copies of an edge compute the same sums.
+struct TileStep {
+    const double2* uin;
+    double2 *uout, *v, *a;
+    const double2* fext;
+    const uchar2* mclass;
+    const double2* coef;  // FP64: {L, M}, {N, kH} per element
+    const float4* cLN;    // mixed: {L, N}
+    const float2* cH;     // and kH
+    const int4* tiles;
+    int nx, ny, tiles_x;
+    double dt, h, c;
+    int advance;
+};
+
+template <bool PAIR, int T, class Tab>
+__global__ void __launch_bounds__(T * T)
+k_verlet_tile(const TileStep p, const __grid_constant__ Tab tab)
+{
+    using Classes = std::conditional_t<PAIR, PairClassShared, MassClassShared>;
+    using Force = std::conditional_t<PAIR, float4, double2>;
+    __shared__ Classes sm;
+    __shared__ Force sf[4][T * T];
+    sm.load(tab);
+    const int tid = threadIdx.x, lx = tid % T, ly = tid / T;
+    int4 g, q;
+    if (p.tiles) {
+        g = __ldg(p.tiles + 2 * static_cast<int64_t>(blockIdx.x));
+        q = __ldg(p.tiles + 2 * static_cast<int64_t>(blockIdx.x) + 1);
+    }
+    else {
+        const int ty = static_cast<int>(blockIdx.x) / p.tiles_x;
+        g = make_int4(0, 0, p.nx, p.ny);
+        q = make_int4((static_cast<int>(blockIdx.x) - ty * p.tiles_x) * (T - 1), ty * (T - 1), 0, 0);
+    }
+    const int nx = g.z, ny = g.w, W = nx + 1;
+    pdl_wait();
+    // this thread's node
+    const int ix = q.x + lx, iy = q.y + ly, node = g.x + iy * W + ix;
+    const bool own = lx < T - 1 && ly < T - 1 && ix <= nx && iy <= ny;
+    double2 vn, an, fx = make_double2(0.0, 0.0);
+    uchar2 cls;
+    if (own) {
+        vn = p.v[node];
+        an = p.a[node];
+        cls = __ldg(p.mclass + node);
+        if (p.fext) fx = __ldg(p.fext + node);
+    }
+    // this thread's element: the one whose upper right node is the tile's (lx, ly)
+    int ex = ix - 1, ey = iy - 1;
+    if (q.z) {
+        ex = ex < 0 ? nx - 1 : (ex == nx ? 0 : ex);
+        ey = ey < 0 ? ny - 1 : (ey == ny ? 0 : ey);
+    }
+    if (ex >= 0 && ex < nx && ey >= 0 && ey < ny) {
+        const int e = g.y + ey * nx + ex;
+        const double2* un = p.uin + g.x + ey * W + ex;
+        const double2 u0 = un[0], u1 = un[1], u3 = un[W], u2 = un[W + 1];
+        if constexpr (PAIR) {
+            ffv f[8];
+            pair_square_forces(u0, u1, u2, u3, __ldg(p.cLN + e), __ldg(p.cH + e), f);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) sf[m][tid] = pack(ff_norm(f[2 * m]), ff_norm(f[2 * m + 1]));
+        }
+        else {
+            double2 f[4];
+            quad4_square_forces(u0, u1, u2, u3, __ldg(p.coef + 2 * static_cast<int64_t>(e)),
+                                __ldg(p.coef + 2 * static_cast<int64_t>(e) + 1), f);
+#pragma unroll
+            for (int m = 0; m < 4; ++m) sf[m][tid] = f[m];
+        }
+    }
+    __syncthreads();
+    if (!own) return;
+    // the element forces of the node in ascending element index: local elements (dx, dy) = left / right,
+    // below / above; across a periodic edge the wrapped row or column changes places
+    const bool sx = q.z && (ix == 0 || ix == nx), sy = q.z && (iy == 0 || iy == ny);
+    [[maybe_unused]] ffv f0 = ff_make(0.f, 0.f), f1 = f0;
+    [[maybe_unused]] double d0 = 0.0, d1 = 0.0;
+    bool first = true;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int dy = (k >> 1) ^ (sy ? 1 : 0), dx = (k & 1) ^ (sx ? 1 : 0);
+        const bool there = q.z || (ix - 1 + dx >= 0 && ix - 1 + dx < nx && iy - 1 + dy >= 0 && iy - 1 + dy < ny);
+        if (!there) continue;
+        const int m = dy ? (dx ? 0 : 1) : (dx ? 3 : 2);
+        const Force t = sf[m][tid + dy * T + dx];
+        if constexpr (PAIR) {
+            f0 = first ? lo2(t) : ff_add(f0, lo2(t));
+            f1 = first ? hi2(t) : ff_add(f1, hi2(t));
+        }
+        else {
+            d0 = first ? t.x : d0 + t.x;
+            d1 = first ? t.y : d1 + t.y;
+        }
+        first = false;
+    }
+    double2 vv, aa;
+    if constexpr (PAIR) {
+        sm.update(cls.x, f0, p.fext != nullptr, fx.x, vn.x, an.x, p.h, vv.x, aa.x);
+        sm.update(cls.y, f1, p.fext != nullptr, fx.y, vn.y, an.y, p.h, vv.y, aa.y);
+    }
+    else {
+        sm.update(cls.x, d0, p.fext != nullptr, fx.x, vn.x, an.x, p.h, vv.x, aa.x);
+        sm.update(cls.y, d1, p.fext != nullptr, fx.y, vn.y, an.y, p.h, vv.y, aa.y);
+    }
+    p.v[node] = vv;
+    p.a[node] = aa;
+    if (p.advance) {
+        const double2 un = p.uin[node];
+        p.uout[node] = make_double2(fma(p.c, aa.x, fma(p.dt, vv.x, un.x)), fma(p.c, aa.y, fma(p.dt, vv.y, un.y)));
+    }
+}
+
+// flag = 1 if the tiles' meshes differ from conn or from the gather table
+template <int T>
+__global__ void __launch_bounds__(T * T)
+k_check_tiles(const int4* __restrict__ tiles, const int32_t* __restrict__ conn, const int32_t* __restrict__ ell,
+              int* __restrict__ flag)
+{
+    const int4 g = tiles[2 * blockIdx.x], q = tiles[2 * blockIdx.x + 1];
+    const int nx = g.z, ny = g.w, W = nx + 1;
+    const int lx = threadIdx.x % T, ly = threadIdx.x / T, ix = q.x + lx, iy = q.y + ly;
+    if (lx == T - 1 || ly == T - 1 || ix > nx || iy > ny) return;
+    const int node = g.x + iy * W + ix;
+    bool bad = false;
+    if (ix < nx && iy < ny) {
+        const int64_t e = g.y + iy * nx + ix;
+        bad = conn[4 * e] != node || conn[4 * e + 1] != node + 1 || conn[4 * e + 2] != node + W + 1 ||
+              conn[4 * e + 3] != node + W;
+    }
+    const bool sx = q.z && (ix == 0 || ix == nx), sy = q.z && (iy == 0 || iy == ny);
+    int n = 0;
+    const int32_t* list = ell + static_cast<int64_t>(node) * 8;
+    for (int k = 0; k < 4; ++k) {
+        const int dy = (k >> 1) ^ (sy ? 1 : 0), dx = (k & 1) ^ (sx ? 1 : 0);
+        int ex = ix - 1 + dx, ey = iy - 1 + dy;
+        if (q.z) {
+            ex = ex < 0 ? nx - 1 : (ex == nx ? 0 : ex);
+            ey = ey < 0 ? ny - 1 : (ey == ny ? 0 : ey);
+        }
+        if (ex < 0 || ex >= nx || ey < 0 || ey >= ny) continue;
+        const int m = dy ? (dx ? 0 : 1) : (dx ? 3 : 2);
+        const int32_t at = ((g.y + ey * nx + ex) * 4 + m) * 2;
+        bad = bad || list[n] != at || list[4 + n] != at + 1;
+        ++n;
+    }
+    for (; n < 4; ++n) bad = bad || list[n] >= 0 || list[4 + n] >= 0;
+    if (bad) *flag = 1;
 }
 
 __global__ void __launch_bounds__(128)
@@ -1359,6 +1550,89 @@ int gfgpu_internal_mixed_increment(const gfgpu_verlet_desc* d, double* fe, int a
     return launch_dependent(k_mixed_node, spread(q.n, 256), s, 0, q, pair_class_tab(d));
 }
 
+// k_verlet_tile, measured against the element and node kernels (us per increment; FP64: tiles of 8,
+// mixed: tiles of 8 / 16):
+//                 64^2   128^2   181^2   256^2   400^2   800^2   2048^2
+//   FP64     two  5.85   5.95    7.08    11.5    23.8    73.1    437
+//           tile  4.11   5.10    7.44    12.7    26.5    94.6    597   (16: 5.71 .. 499)
+//   mixed    two  5.02   5.30    6.04    8.14    13.4    37.9    235
+//           tile  3.60   4.16    5.01    6.89    12.2    37.0    223
+//                 4.12   4.20    5.62    7.16    11.0    33.5    204
+// Small meshes: one launch instead of two, and small blocks on as many SMs as there are. From three tiles
+// of 8 per SM on, FP64 issue bounds the FP64 increment and the elements computed twice on the rims cost
+// more than the launch: two kernels there. Mixed arithmetic has the room; tiles of 16 compute 1.14
+// elements per node instead of 1.31.
+constexpr int64_t kTilesFew = 3 * 152;
+
+static int tile_edge(int64_t tiles16)
+{
+    return tiles16 < kTilesFew ? 8 : 16;
+}
+
+static int64_t grid_tiles(int64_t nx, int64_t ny, int edge)
+{
+    const int64_t n = edge - 1;
+    return (nx + n) / n * ((ny + n) / n); // of (nx + 1) x (ny + 1) nodes
+}
+
+// 0 if k_verlet_tile does not take the descriptor's increments, else its tile edge: square elements with
+// coefficients, lumped-mass classes, and a grid numbering (Regular, or the verified table of
+// gfgpu_verlet_detect_blocks with its gather table still in use).
+int gfgpu_internal_tile_edge(const gfgpu_verlet_desc* d, bool mixed, const double* u, const double* v,
+                             const double* a, const double* scratch)
+{
+    if (strict_mode() || variant_elem() != 0 || !(d->uniform && d->nne == 4 && d->ndim == 2 && d->coef)) return 0;
+    if (!(d->mclass && d->mclass_inv && d->ncls > 0) || d->nelem == 0) return 0;
+    // pairs of values in 16-byte accesses
+    const uintptr_t at = reinterpret_cast<uintptr_t>(u) | reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(a) |
+                         reinterpret_cast<uintptr_t>(scratch) | reinterpret_cast<uintptr_t>(d->fext) |
+                         reinterpret_cast<uintptr_t>(d->coef);
+    if ((at & 15u) != 0 || (reinterpret_cast<uintptr_t>(d->mclass) & 1u) != 0) return 0;
+    int edge = 0;
+    int64_t n = 0;
+    if (d->reg_nx > 0 && d->reg_ny > 0 && d->reg_nz == 0) {
+        edge = tile_edge(grid_tiles(d->reg_nx, d->reg_ny, 16));
+        n = grid_tiles(d->reg_nx, d->reg_ny, edge);
+    }
+    else if (d->tiles && d->ntiles > 0 && d->ell) {
+        edge = d->tile_edge;
+        n = d->ntiles;
+    }
+    return mixed || (edge == 8 && n <= kTilesFew) ? edge : 0;
+}
+
+// One increment by k_verlet_tile: reads uin, writes uout if it advances.
+int gfgpu_internal_tile_increment(const gfgpu_verlet_desc* d, const MassClassTab& tab, const VerletCoef& k, int edge,
+                                  bool mixed, const double* uin, double* uout, int advance, double* v, double* a,
+                                  cudaStream_t s)
+{
+    TileStep p;
+    p.uin = reinterpret_cast<const double2*>(uin);
+    p.uout = reinterpret_cast<double2*>(uout);
+    p.v = reinterpret_cast<double2*>(v);
+    p.a = reinterpret_cast<double2*>(a);
+    p.fext = reinterpret_cast<const double2*>(d->fext);
+    p.mclass = reinterpret_cast<const uchar2*>(d->mclass);
+    p.coef = reinterpret_cast<const double2*>(d->coef);
+    p.cLN = reinterpret_cast<const float4*>(d->pcg_pair);
+    p.cH = mixed ? reinterpret_cast<const float2*>(d->pcg_pair + 4 * d->nelem) : nullptr;
+    const bool regular = d->reg_nx > 0;
+    p.tiles = regular ? nullptr : reinterpret_cast<const int4*>(d->tiles);
+    p.nx = static_cast<int>(d->reg_nx);
+    p.ny = static_cast<int>(d->reg_ny);
+    p.tiles_x = static_cast<int>((d->reg_nx + edge - 1) / (edge - 1));
+    p.dt = k.dt;
+    p.h = k.h;
+    p.c = k.c;
+    p.advance = advance;
+    const int64_t n = regular ? grid_tiles(d->reg_nx, d->reg_ny, edge) : d->ntiles;
+    const Shape shape{static_cast<unsigned>(n), edge * edge};
+    if (mixed)
+        return edge == 8 ? launch_dependent(k_verlet_tile<true, 8, PairClassTab>, shape, s, 0, p, pair_class_tab(d))
+                         : launch_dependent(k_verlet_tile<true, 16, PairClassTab>, shape, s, 0, p, pair_class_tab(d));
+    return launch_dependent(k_verlet_tile<false, 8, MassClassTab>, shape, s, 0, p, tab);
+}
+
 // {L, N} [nelem] interleaved pairs, then kH [nelem] (6 floats per element) of a uniform square Quad4
 // mesh, the layout k_pair_elem_square_f64 reads
 int gfgpu_internal_pair_coef_square(const gfgpu_verlet_desc* d, float* coef, cudaStream_t s)
@@ -1372,6 +1646,80 @@ int gfgpu_internal_pair_coef_square(const gfgpu_verlet_desc* d, float* coef, cud
 }
 
 extern "C" {
+
+int64_t gfgpu_verlet_tiles_ints(int64_t nblocks, const int64_t* nx, const int64_t* ny)
+{
+    int64_t n16 = 0, n8 = 0;
+    for (int64_t b = 0; nx && ny && b < nblocks; ++b) {
+        if (nx[b] < 1 || ny[b] < 1) return 0;
+        n16 += grid_tiles(nx[b], ny[b], 16);
+        n8 += grid_tiles(nx[b], ny[b], 8);
+    }
+    return 8 * (tile_edge(n16) == 8 ? n8 : n16);
+}
+
+int gfgpu_verlet_detect_blocks(gfgpu_verlet_desc* d, int64_t nblocks, const int64_t* nx, const int64_t* ny,
+                               int32_t* tiles, gfgpu_stream_t stream)
+{
+    GF_REQUIRE(d && nblocks > 0 && nx && ny && tiles && d->conn, "bad argument");
+    GF_REQUIRE((reinterpret_cast<uintptr_t>(tiles) & 15u) == 0, "tiles must be 16-byte aligned");
+    d->tiles = nullptr;
+    d->ntiles = 0;
+    d->tile_edge = 0;
+    if (!(d->nne == 4 && d->ndim == 2 && d->ell)) return GFGPU_OK;
+    int64_t nelem = 0, nnode = 0, n16 = 0;
+    bool wrap = true; // a mesh one element wide meets itself across its edge: left to the gather table
+    for (int64_t b = 0; b < nblocks; ++b) {
+        if (nx[b] < 1 || ny[b] < 1 || nx[b] > d->nelem || ny[b] > d->nelem) return GFGPU_OK;
+        nelem += nx[b] * ny[b];
+        nnode += (nx[b] + 1) * (ny[b] + 1);
+        n16 += grid_tiles(nx[b], ny[b], 16);
+        wrap = wrap && nx[b] > 1 && ny[b] > 1;
+        if (nelem > d->nelem || nnode > d->nnode) return GFGPU_OK;
+    }
+    if (nelem != d->nelem || nnode != d->nnode || too_big(8 * nelem)) return GFGPU_OK;
+    const int edge = tile_edge(n16);
+    cudaStream_t s = S(stream);
+    int* flag = nullptr;
+    for (int periodic = wrap ? 1 : 0; periodic >= 0; --periodic) {
+        std::vector<int32_t> t;
+        int64_t node0 = 0, elem0 = 0;
+        for (int64_t b = 0; b < nblocks; ++b) {
+            for (int64_t y = 0; y <= ny[b]; y += edge - 1)
+                for (int64_t x = 0; x <= nx[b]; x += edge - 1) {
+                    const int64_t r[8] = {node0, elem0, nx[b], ny[b], x, y, periodic, 0};
+                    for (int64_t v : r) t.push_back(static_cast<int32_t>(v));
+                }
+            node0 += (nx[b] + 1) * (ny[b] + 1);
+            elem0 += nx[b] * ny[b];
+        }
+        int h = 1;
+        GF_TRY(check_cuda(cudaMallocAsync(reinterpret_cast<void**>(&flag), sizeof(int), s), "cudaMallocAsync"));
+        int rc = check_cuda(cudaMemsetAsync(flag, 0, sizeof(int), s), "cudaMemsetAsync");
+        if (rc == GFGPU_OK)
+            rc = check_cuda(cudaMemcpyAsync(tiles, t.data(), t.size() * sizeof(int32_t), cudaMemcpyHostToDevice, s), "copy");
+        if (rc == GFGPU_OK) {
+            const unsigned n = static_cast<unsigned>(t.size() / 8);
+            const int4* q = reinterpret_cast<const int4*>(tiles);
+            if (edge == 8) k_check_tiles<8><<<n, 64, 0, s>>>(q, d->conn, d->ell, flag);
+            else k_check_tiles<16><<<n, 256, 0, s>>>(q, d->conn, d->ell, flag);
+            rc = check_launch("detect_blocks");
+        }
+        if (rc == GFGPU_OK) rc = check_cuda(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, s), "copy");
+        const int rc_free = check_cuda(cudaFreeAsync(flag, s), "cudaFreeAsync");
+        if (rc == GFGPU_OK) rc = rc_free;
+        const int rc_sync = check_cuda(cudaStreamSynchronize(s), "cudaStreamSynchronize");
+        if (rc == GFGPU_OK) rc = rc_sync;
+        GF_TRY(rc);
+        if (h == 0) {
+            d->tiles = tiles;
+            d->ntiles = static_cast<int32_t>(t.size() / 8);
+            d->tile_edge = edge;
+            return GFGPU_OK;
+        }
+    }
+    return GFGPU_OK;
+}
 
 int gfgpu_verlet_pair_begin(const gfgpu_verlet_desc* d, const double* u, const double* v, const double* a,
                             void* workspace, gfgpu_stream_t stream)

@@ -156,6 +156,9 @@ class VelocityVerlet:
         if nne == 4:
             if not self._detect_regular(conn_h):
                 self._build_ell()
+                nx = int(conn_h[0][3]) - 1
+                if nx > 0 and nelem % nx == 0:
+                    self._detect_blocks([(nx, nelem // nx)])
         self.coef_pair = None
         if arithmetic == "pair":
             self.use_pair()
@@ -247,6 +250,16 @@ class VelocityVerlet:
             self._ell = t
         except _lib.GFGPUError:
             self.desc.ell = None
+
+    def _detect_blocks(self, sizes):
+        """Grids of the given (nx, ny) one after the other (gfgpu_verlet_detect_blocks, checked on the
+        device): one kernel per increment for square elements with lumped-mass classes."""
+        nx, ny = (np.array([s[i] for s in sizes], dtype=np.int64) for i in (0, 1))
+        n = int(_lib.lib().gfgpu_verlet_tiles_ints(len(sizes), nx.ctypes.data, ny.ctypes.data))
+        t = torch.empty(max(n, 1), dtype=torch.int32, device=_dev.device())
+        _lib.call("gfgpu_verlet_detect_blocks", C.addressof(self.desc), len(sizes), nx.ctypes.data,
+                  ny.ctypes.data, t.data_ptr(), _dev.stream())
+        self._tiles = t
 
     def use_csr_gather(self):
         """Node kernel through the dof CSR even on a Regular mesh, without the gather table (FP64

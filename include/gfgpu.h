@@ -391,6 +391,13 @@ typedef struct {
      * instead of dofs / csr_ptr / csr_idx: one dependent load of 16 bytes instead of three
      * levels (same order, same bits). NULL = the CSR. */
     const int32_t* ell;
+    /* optional tile table (gfgpu_verlet_detect_blocks): the mesh is one or many grids numbered as
+     * Mesh::Quad4::Regular, all with periodic or all with open dofs; with square elements, lumped-mass
+     * classes and ell still set, gfgpu_verlet_step in fast mode runs one kernel per increment instead
+     * of an element and a node kernel (mixed arithmetic; FP64 on small meshes). NULL = two kernels (a
+     * mesh with reg_nx set needs no table). */
+    const int32_t* tiles;
+    int32_t ntiles, tile_edge;
 } gfgpu_verlet_desc;
 
 #define GFGPU_MASS_CLASSES 16
@@ -479,6 +486,14 @@ int gfgpu_verlet_detect_regular(gfgpu_verlet_desc* d, int64_t nx, int64_t ny, gf
  * when every dof has at most 4 element contributions; else leave d->ell unchanged and return
  * GFGPU_ERR_UNSUPPORTED. Synchronises. */
 int gfgpu_verlet_build_ell(gfgpu_verlet_desc* d, int32_t* ell, gfgpu_stream_t stream);
+/* Checks on the device that conn and ell (set before) are those of nblocks grids, one after the other
+ * in nodes, elements and dofs: grid b with the connectivity of Mesh::Quad4::Regular(nx[b], ny[b]) (host
+ * arrays) and dofs = node * 2 + i or, in all grids, RegularBase::dofsPeriodic (at least 2 x 2 elements
+ * then). tiles: gfgpu_verlet_tiles_ints(nblocks, nx, ny) device ints, 16-byte aligned. On success sets
+ * d->tiles, d->ntiles and d->tile_edge, else clears them. Returns GFGPU_OK either way. Synchronises. */
+int64_t gfgpu_verlet_tiles_ints(int64_t nblocks, const int64_t* nx, const int64_t* ny);
+int gfgpu_verlet_detect_blocks(gfgpu_verlet_desc* d, int64_t nblocks, const int64_t* nx, const int64_t* ny,
+                               int32_t* tiles, gfgpu_stream_t stream);
 /* The same for MeshHex8.h:77-130's Regular(nx, ny, nz) connectivity with dofs = arange(nnode * 3):
  * sets d->reg_nx, reg_ny, reg_nz on success (used by the static solvers' gather; the explicit
  * step's node kernels are Quad4 only). Returns GFGPU_OK either way. Synchronises. */
