@@ -127,6 +127,26 @@ __device__ __forceinline__ ffv ff_from_double(double x)
     return ff_make(__uint_as_float(hb), l);
 }
 
+// The same split for kernels whose issue slots it fills: h is x's significand rounded to 24 bits with
+// ties away from zero (one 64-bit addition of half a unit, which also rebiases the exponent), and the
+// remainder is what is left of the 29 bits below, so h + l has the error of ff_from_double (a tie gives
+// another pair of the same exact sum). Same domain: l = 0 below 2^-74, h = +-0 below 2^-126; l of an
+// exact h may be -0; |x| >= 2^128, infinities and NaN give NaN, which the pair sums make of them anyway.
+// 18 instructions instead of about 30.
+__device__ __forceinline__ ffv ff_split(double x)
+{
+    const uint32_t hi = static_cast<uint32_t>(__double2hiint(x)), a = hi & 0x7fffffffu, sign = hi & 0x80000000u;
+    const unsigned long long b =
+        static_cast<unsigned long long>(__double_as_longlong(x)) + ((1ull << 59) + (1ull << 28));
+    uint32_t hb = static_cast<uint32_t>(b >> 29) | sign;
+    const int d = static_cast<int>(static_cast<uint32_t>(b) & 0x1fffffffu) - (1 << 28);
+    float l = __fmul_rn(__int2float_rn(d), __uint_as_float((((hi << 3) - (948u << 23)) & 0x7f800000u) | sign));
+    if (a < (949u << 20)) l = 0.0f;
+    if (a < (897u << 20)) hb = sign;
+    if (a >= (1151u << 20)) hb = 0x7fffffffu;
+    return ff_make(__uint_as_float(hb), l);
+}
+
 // pair -> double: rn(h + l), one FP64 addition of the two exactly converted parts
 __device__ __forceinline__ double ff_to_double(ffv x)
 {

@@ -678,6 +678,31 @@ __device__ __forceinline__ void pair_square_forces(double2 q0, double2 q1, doubl
     f[7] = ff_neg(ff_add(Dy, H1));
 }
 
+// The same on packed pairs (lanes x, y), the forces normalised.
+__device__ __forceinline__ void pair_square_forces2(double2 q0, double2 q1, double2 q2, double2 q3, float4 cln,
+                                                    float2 ch, f2 nz, ff2 (&f)[4])
+{
+    auto diff = [](double2 a, double2 b) { return ff2_from(ff_split(a.x - b.x), ff_split(a.y - b.y)); };
+    const ff2 P = diff(q2, q0), Q = diff(q1, q3);
+    const ff2 A1 = ff2_add(P, Q), A2 = ff2_sub(P, Q);
+    const ff2 A3 = ff2_add(diff(q0, q1), diff(q2, q3));
+    // (t, s) = (A1x + A2y, A1y + A2x); (Lt, P1) = (L t, N s)
+    const ff2 A2s = ff2_make(f2_make(f2_hi(A2.h), f2_lo(A2.h)), f2_make(f2_hi(A2.l), f2_lo(A2.l)));
+    const ff2 LtP1 = ff2_mul(ff2_from(lo2(cln), hi2(cln)), ff2_add(A1, A2s), nz);
+    // (P0, Q1) = 2 N (A1x, A2y) + (Lt, Lt)
+    const ff2 dg = ff2_make(f2_make(f2_lo(A1.h), f2_hi(A2.h)), f2_make(f2_lo(A1.l), f2_hi(A2.l)));
+    const ff2 PQ = ff2_add(ff2_mul(ff2_bcast(ff_twice(hi2(cln))), dg, nz), ff2_bcast(ff2_lane0(LtP1)));
+    const ff2 H = ff2_norm(ff2_mul(ff2_bcast(pf(ch)), A3, nz));
+    // S = (P0 + P1, P1 + Q1), D = (P0 - P1, P1 - Q1)
+    const ff2 P1 = ff2_bcast(ff2_lane1(LtP1));
+    const ff2 S = ff2_norm(ff2_add(PQ, P1)), E = ff2_norm(ff2_sub(PQ, P1));
+    const ff2 D = ff2_make(f2_make(f2_lo(E.h), -f2_hi(E.h)), f2_make(f2_lo(E.l), -f2_hi(E.l)));
+    f[0] = ff2_norm(ff2_sub(H, S));
+    f[1] = ff2_norm(ff2_sub(D, H));
+    f[2] = ff2_norm(ff2_add(S, H));
+    f[3] = ff2_neg(ff2_norm(ff2_add(D, H)));
+}
+
 // Element forces of uniform square Quad4 elements in pair arithmetic with FP64 input and output
 // (the static solvers' operator and the explicit step's element kernel in "mixed" arithmetic): the
 // node differences of the square closed form are formed in FP64 (8 subtractions), split into pairs
@@ -753,6 +778,31 @@ struct PairClassShared {
             vv = fma(h, an + an, vn);
         }
     }
+    // both components of a node at once
+    __device__ __forceinline__ void update2(uchar2 c, ff2 f, bool has_fext, double2 fx, double2 vn, double2 an,
+                                            double h, f2 nz, double2& vv, double2& aa) const
+    {
+        if (c.x < GFGPU_MASS_CLASSES && c.y < GFGPU_MASS_CLASSES) {
+            const int cx = c.x, cy = c.y;
+            auto co = [&](const float2* t) {
+                const float2 x = t[cx], y = t[cy];
+                return ff2_make(f2_make(x.x, y.x), f2_make(x.y, y.y));
+            };
+            const ff2 R = has_fext ? ff2_sub(ff2_from(ff_split(fx.x), ff_split(fx.y)), f) : ff2_neg(f);
+            const ff2 mR = ff2_mul(co(mi), R, nz);
+            const ff2 V = ff2_add(ff2_add(ff2_mul(co(c1), ff2_from(ff_split(vn.x), ff_split(vn.y)), nz),
+                                          ff2_mul(co(c2), ff2_from(ff_split(an.x), ff_split(an.y)), nz)),
+                                  ff2_mul(co(c3), mR, nz));
+            const ff2 Vn = ff2_norm(V);
+            const ff2 Ac = ff2_sub(mR, ff2_mul(co(be), Vn, nz));
+            vv = make_double2(ff_to_double(ff2_lane0(Vn)), ff_to_double(ff2_lane1(Vn)));
+            aa = make_double2(ff_to_double(ff2_lane0(Ac)), ff_to_double(ff2_lane1(Ac)));
+        }
+        else {
+            update(c.x, ff2_lane0(f), has_fext, fx.x, vn.x, an.x, h, vv.x, aa.x);
+            update(c.y, ff2_lane1(f), has_fext, fx.y, vn.y, an.y, h, vv.y, aa.y);
+        }
+    }
 };
 
 struct MixedNodeStep {
@@ -823,6 +873,10 @@ k_mixed_node(const MixedNodeStep p, const __grid_constant__ PairClassTab tab)
 // The grid is Regular(nx, ny) (tiles null) or, per tile, the record {node0, elem0, nx, ny},
 // {x0, y0, periodic, 0} of one of many meshes; a periodic mesh takes the elements across its edges, and
 // the nodes of both copies of an edge compute the same sums.
+// Mixed arithmetic is bound by issue slots and the 16 FP64 instructions of a node (differences, joins,
+// predictor): both components of a node run as packed pairs and the splits are ff_split's, 1000 -> 760
+// instructions per node. 24 periodic meshes of 32 to 256 elements an edge (428k nodes): 25.2 -> 22.3 us
+// per increment.
 struct TileStep {
     const double2* uin;
     double2 *uout, *v, *a;
@@ -834,6 +888,7 @@ struct TileStep {
     const int4* tiles;
     int nx, ny, tiles_x;
     double dt, h, c;
+    f2 nz;                // kF2NegZero
     int advance;
 };
 
@@ -842,7 +897,7 @@ __global__ void __launch_bounds__(T * T)
 k_verlet_tile(const TileStep p, const __grid_constant__ Tab tab)
 {
     using Classes = std::conditional_t<PAIR, PairClassShared, MassClassShared>;
-    using Force = std::conditional_t<PAIR, float4, double2>;
+    using Force = std::conditional_t<PAIR, ulonglong2, double2>; // pairs: packed {h, l}
     __shared__ Classes sm;
     __shared__ Force sf[4][T * T];
     sm.load(tab);
@@ -881,10 +936,10 @@ k_verlet_tile(const TileStep p, const __grid_constant__ Tab tab)
         const double2* un = p.uin + g.x + ey * W + ex;
         const double2 u0 = un[0], u1 = un[1], u3 = un[W], u2 = un[W + 1];
         if constexpr (PAIR) {
-            ffv f[8];
-            pair_square_forces(u0, u1, u2, u3, __ldg(p.cLN + e), __ldg(p.cH + e), f);
+            ff2 f[4];
+            pair_square_forces2(u0, u1, u2, u3, __ldg(p.cLN + e), __ldg(p.cH + e), p.nz, f);
 #pragma unroll
-            for (int m = 0; m < 4; ++m) sf[m][tid] = pack(ff_norm(f[2 * m]), ff_norm(f[2 * m + 1]));
+            for (int m = 0; m < 4; ++m) sf[m][tid] = make_ulonglong2(f[m].h, f[m].l);
         }
         else {
             double2 f[4];
@@ -899,7 +954,7 @@ k_verlet_tile(const TileStep p, const __grid_constant__ Tab tab)
     // the element forces of the node in ascending element index: local elements (dx, dy) = left / right,
     // below / above; across a periodic edge the wrapped row or column changes places
     const bool sx = q.z && (ix == 0 || ix == nx), sy = q.z && (iy == 0 || iy == ny);
-    [[maybe_unused]] ffv f0 = ff_make(0.f, 0.f), f1 = f0;
+    [[maybe_unused]] ff2 fp = ff2_make(0ull, 0ull);
     [[maybe_unused]] double d0 = 0.0, d1 = 0.0;
     bool first = true;
 #pragma unroll
@@ -910,8 +965,8 @@ k_verlet_tile(const TileStep p, const __grid_constant__ Tab tab)
         const int m = dy ? (dx ? 0 : 1) : (dx ? 3 : 2);
         const Force t = sf[m][tid + dy * T + dx];
         if constexpr (PAIR) {
-            f0 = first ? lo2(t) : ff_add(f0, lo2(t));
-            f1 = first ? hi2(t) : ff_add(f1, hi2(t));
+            const ff2 tp = ff2_make(t.x, t.y);
+            fp = first ? tp : ff2_add(fp, tp);
         }
         else {
             d0 = first ? t.x : d0 + t.x;
@@ -921,8 +976,7 @@ k_verlet_tile(const TileStep p, const __grid_constant__ Tab tab)
     }
     double2 vv, aa;
     if constexpr (PAIR) {
-        sm.update(cls.x, f0, p.fext != nullptr, fx.x, vn.x, an.x, p.h, vv.x, aa.x);
-        sm.update(cls.y, f1, p.fext != nullptr, fx.y, vn.y, an.y, p.h, vv.y, aa.y);
+        sm.update2(cls, fp, p.fext != nullptr, fx, vn, an, p.h, p.nz, vv, aa);
     }
     else {
         sm.update(cls.x, d0, p.fext != nullptr, fx.x, vn.x, an.x, p.h, vv.x, aa.x);
@@ -1556,8 +1610,7 @@ int gfgpu_internal_mixed_increment(const gfgpu_verlet_desc* d, double* fe, int a
 //   FP64     two  5.85   5.95    7.08    11.5    23.8    73.1    437
 //           tile  4.11   5.10    7.44    12.7    26.5    94.6    597   (16: 5.71 .. 499)
 //   mixed    two  5.02   5.30    6.04    8.14    13.4    37.9    235
-//           tile  3.60   4.16    5.01    6.89    12.2    37.0    223
-//                 4.12   4.20    5.62    7.16    11.0    33.5    204
+//           tile  3.60   4.06    4.86    6.45    10.1    29.0    198   (8 to 181^2, 16 above)
 // Small meshes: one launch instead of two, and small blocks on as many SMs as there are. From three tiles
 // of 8 per SM on, FP64 issue bounds the FP64 increment and the elements computed twice on the rims cost
 // more than the launch: two kernels there. Mixed arithmetic has the room; tiles of 16 compute 1.14
@@ -1624,6 +1677,7 @@ int gfgpu_internal_tile_increment(const gfgpu_verlet_desc* d, const MassClassTab
     p.dt = k.dt;
     p.h = k.h;
     p.c = k.c;
+    p.nz = kF2NegZero;
     p.advance = advance;
     const int64_t n = regular ? grid_tiles(d->reg_nx, d->reg_ny, edge) : d->ntiles;
     const Shape shape{static_cast<unsigned>(n), edge * edge};
