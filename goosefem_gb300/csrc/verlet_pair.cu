@@ -107,26 +107,6 @@ __device__ __forceinline__ void pair_element(ffv u0x, ffv u0y, ffv u1x, ffv u1y,
     H = pack(ff_norm(H0), ff_norm(H1));
 }
 
-// The same closed form from the element's node differences P = u2 - u0, Q = u1 - u3 and
-// D = u0 - u1, E = u2 - u3 (A1 = P + Q, A2 = P - Q, A3 = D + E), given as pairs: a caller that
-// forms them in FP64 from an FP64 displacement keeps the pair rounding at the scale of the
-// differences, not of the displacement (an applied affine field cancels exactly as in FP64).
-__device__ __forceinline__ void pair_element_diff(ffv Px, ffv Py, ffv Qx, ffv Qy, ffv Dx, ffv Dy, ffv Ex,
-                                                  ffv Ey, ffv L, ffv N, ffv kH, float4& S, float4& D, float4& H)
-{
-    const ffv A1x = ff_add(Px, Qx), A2x = ff_sub(Px, Qx);
-    const ffv A1y = ff_add(Py, Qy), A2y = ff_sub(Py, Qy);
-    const ffv A3x = ff_add(Dx, Ex), A3y = ff_add(Dy, Ey);
-    const ffv Lt = ff_mul(L, ff_add(A1x, A2y));
-    const ffv P0 = ff_add(ff_twice(ff_mul(N, A1x)), Lt);
-    const ffv Q1 = ff_add(ff_twice(ff_mul(N, A2y)), Lt);
-    const ffv P1 = ff_mul(N, ff_add(A1y, A2x));
-    const ffv H0 = ff_mul(kH, A3x), H1 = ff_mul(kH, A3y);
-    S = pack(ff_norm(ff_add(P0, P1)), ff_norm(ff_add(P1, Q1)));
-    D = pack(ff_norm(ff_sub(P0, P1)), ff_norm(ff_sub(P1, Q1)));
-    H = pack(ff_norm(H0), ff_norm(H1));
-}
-
 // One velocity-Verlet component update (closed form per mass class, or a prescribed dof).
 __device__ __forceinline__ void pair_update(int c, ffv f, ffv fx, bool has_fext, ffv vn, ffv an,
                                             const float2* smi, const float2* sbe, const float2* sc1,
@@ -658,27 +638,11 @@ k_pair_elem_square(const int32_t* __restrict__ conn, const float4* u, const floa
     }
 }
 
-// Pair forces {x, y} of nodes 0..3 of a square element from FP64 nodal displacements (coefficients
-// {L, N} and kH as pairs).
-__device__ __forceinline__ void pair_square_forces(double2 q0, double2 q1, double2 q2, double2 q3, float4 cln,
-                                                   float2 ch, ffv (&f)[8])
-{
-    float4 S, D, H;
-    pair_element_diff(ff_from_double(q2.x - q0.x), ff_from_double(q2.y - q0.y), ff_from_double(q1.x - q3.x),
-                      ff_from_double(q1.y - q3.y), ff_from_double(q0.x - q1.x), ff_from_double(q0.y - q1.y),
-                      ff_from_double(q2.x - q3.x), ff_from_double(q2.y - q3.y), lo2(cln), hi2(cln), pf(ch), S, D, H);
-    const ffv Sx = lo2(S), Sy = hi2(S), Dx = lo2(D), Dy = hi2(D), H0 = lo2(H), H1 = hi2(H);
-    f[0] = ff_sub(H0, Sx);
-    f[1] = ff_sub(H1, Sy);
-    f[2] = ff_sub(Dx, H0);
-    f[3] = ff_sub(Dy, H1);
-    f[4] = ff_add(Sx, H0);
-    f[5] = ff_add(Sy, H1);
-    f[6] = ff_neg(ff_add(Dx, H0));
-    f[7] = ff_neg(ff_add(Dy, H1));
-}
-
-// The same on packed pairs (lanes x, y), the forces normalised.
+// Pair forces {x, y} of nodes 0..3 of a square element (lanes x, y; normalised) from FP64 nodal
+// displacements and its coefficients {L, N} and kH: k_elem_force_quad4_square's formulas from the node
+// differences P = u2 - u0, Q = u1 - u3, u0 - u1 and u2 - u3 (A1 = P + Q, A2 = P - Q, A3 the sum of the
+// others). Formed in FP64 and then split, they keep the pair rounding at the scale of the differences,
+// not of the displacement (an applied affine field cancels as in FP64).
 __device__ __forceinline__ void pair_square_forces2(double2 q0, double2 q1, double2 q2, double2 q3, float4 cln,
                                                     float2 ch, f2 nz, ff2 (&f)[4])
 {
@@ -706,7 +670,7 @@ __device__ __forceinline__ void pair_square_forces2(double2 q0, double2 q1, doub
 // Element forces of uniform square Quad4 elements in pair arithmetic with FP64 input and output
 // (the static solvers' operator and the explicit step's element kernel in "mixed" arithmetic): the
 // node differences of the square closed form are formed in FP64 (8 subtractions), split into pairs
-// on the integer pipe, the closed form runs on pairs (pair_element_diff) and the forces are joined
+// on the integer pipe, the closed form runs on packed pairs (pair_square_forces2) and the forces are joined
 // to FP64 into fe [nelem, 4, 2] (the layout of k_elem_force_quad4_square that the FP64 gathers and
 // node kernels read): 16 FP64 instructions per element instead of 34. Forming the differences in
 // FP64 keeps the pair rounding relative to them: an applied affine displacement cancels as in FP64.
@@ -716,7 +680,7 @@ template <bool PAIR_OUT>
 __global__ void __launch_bounds__(256)
 k_pair_elem_square_f64(const int32_t* __restrict__ conn, const double2* u,
                        const float4* __restrict__ cLN, const float2* __restrict__ cH, int64_t nelem,
-                       double2* __restrict__ fe)
+                       double2* __restrict__ fe, f2 nz)
 {
     pdl_wait();
     GF_FOR(e, nelem)
@@ -724,17 +688,17 @@ k_pair_elem_square_f64(const int32_t* __restrict__ conn, const double2* u,
         const int4 cn = __ldg(reinterpret_cast<const int4*>(conn) + e);
         const double2 q0 = u[cn.x], q1 = u[cn.y], q2 = u[cn.z], q3 = u[cn.w];
         const float4 cln = __ldg(cLN + e);
-        ffv f[8];
-        pair_square_forces(q0, q1, q2, q3, cln, __ldg(cH + e), f);
+        ff2 f[4];
+        pair_square_forces2(q0, q1, q2, q3, cln, __ldg(cH + e), nz, f);
         if constexpr (PAIR_OUT) {
             float4* o = reinterpret_cast<float4*>(fe) + e * 4;
 #pragma unroll
-            for (int m = 0; m < 4; ++m) o[m] = pack(ff_norm(f[2 * m]), ff_norm(f[2 * m + 1]));
+            for (int m = 0; m < 4; ++m) o[m] = pack(ff2_lane0(f[m]), ff2_lane1(f[m]));
         }
         else {
             double2* o = fe + e * 4;
 #pragma unroll
-            for (int m = 0; m < 4; ++m) o[m] = make_double2(ff_to_double(f[2 * m]), ff_to_double(f[2 * m + 1]));
+            for (int m = 0; m < 4; ++m) o[m] = make_double2(ff_to_double(ff2_lane0(f[m])), ff_to_double(ff2_lane1(f[m])));
         }
     }
 }
@@ -764,9 +728,9 @@ struct PairClassShared {
                                            double& vv, double& aa) const
     {
         if (c < GFGPU_MASS_CLASSES) {
-            const ffv R = has_fext ? ff_sub(ff_from_double(fx), f) : ff_neg(f);
+            const ffv R = has_fext ? ff_sub(ff_split(fx), f) : ff_neg(f);
             const ffv mR = ff_mul(pf(mi[c]), R);
-            const ffv V = ff_add(ff_add(ff_mul(pf(c1[c]), ff_from_double(vn)), ff_mul(pf(c2[c]), ff_from_double(an))),
+            const ffv V = ff_add(ff_add(ff_mul(pf(c1[c]), ff_split(vn)), ff_mul(pf(c2[c]), ff_split(an))),
                                  ff_mul(pf(c3[c]), mR));
             const ffv Vn = ff_norm(V);
             const ffv Ac = ff_sub(mR, ff_mul(pf(be[c]), Vn));
@@ -867,7 +831,7 @@ k_mixed_node(const MixedNodeStep p, const __grid_constant__ PairClassTab tab)
 // false) or mixed arithmetic: a block of T x T threads takes the T x T elements around a tile of
 // (T - 1) x (T - 1) nodes (the elements on the rim are computed by both neighbours), keeps their forces
 // in shared memory and updates the nodes from there. The formulas and the order of the sums are those of
-// the two-kernel increment (quad4_square_forces / pair_square_forces, ascending element index,
+// the two-kernel increment (quad4_square_forces / pair_square_forces2, ascending element index,
 // MassClassShared / PairClassShared), the forces never reach memory and the displacement is
 // double-buffered: neighbours read it while a block updates its nodes.
 // The grid is Regular(nx, ny) (tiles null) or, per tile, the record {node0, elem0, nx, ny},
@@ -1569,7 +1533,8 @@ int gfgpu_internal_pair_element_forces_f64(const gfgpu_verlet_desc* d, const dou
     const Shape l = spread(d->nelem, 256);
     k_pair_elem_square_f64<false><<<l.grid, l.block, 0, s>>>(
         d->conn, reinterpret_cast<const double2*>(u), reinterpret_cast<const float4*>(c),
-        reinterpret_cast<const float2*>(c + 4 * d->nelem), d->nelem, reinterpret_cast<double2*>(fe));
+        reinterpret_cast<const float2*>(c + 4 * d->nelem), d->nelem, reinterpret_cast<double2*>(fe),
+        kF2NegZero);
     return check_launch("pair element kernel (static operator)");
 }
 
@@ -1582,7 +1547,7 @@ int gfgpu_internal_mixed_increment(const gfgpu_verlet_desc* d, double* fe, int a
     GF_TRY(launch_dependent(k_pair_elem_square_f64<true>, spread(d->nelem, 256), s, 0, d->conn,
                             reinterpret_cast<const double2*>(u), reinterpret_cast<const float4*>(c),
                             reinterpret_cast<const float2*>(c + 4 * d->nelem), d->nelem,
-                            reinterpret_cast<double2*>(fe)));
+                            reinterpret_cast<double2*>(fe), static_cast<f2>(kF2NegZero)));
     MixedNodeStep q;
     q.dofs = d->dofs;
     q.ptr = d->csr_ptr;
