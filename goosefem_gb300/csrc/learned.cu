@@ -1259,6 +1259,9 @@ int gfgpu_internal_element_forces(const gfgpu_verlet_desc* d, const double* u, d
                                   cudaStream_t s);
 int gfgpu_internal_iteration_element_forces(const gfgpu_verlet_desc* d, const double* u, double* fe,
                                             cudaStream_t s);
+bool gfgpu_internal_pair_operator(const gfgpu_verlet_desc* d);
+int gfgpu_internal_tile_apply(const gfgpu_verlet_desc* d, const double* pv, const double* r, double* q, double* pq,
+                              double* rp, double* keep, const double* kept, int* nblk, cudaStream_t s);
 // two-level correction z = P ainv P^T r + minv r (coarse.cu)
 int gfgpu_internal_coarse_apply(const gfgpu_coarse_desc* g, const int32_t* part, int64_t nnu,
                                 const double* minv, const double* r, double* vc, double* yc,
@@ -2269,6 +2272,7 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
     // and the earlier directions of this iteration. read: r.r is formed as well (the host reads it
     // next, or the network takes its scale from it).
     auto iteration = [&](int64_t c0, bool read, cudaStream_t st) -> int {
+        int ng = nr; // partials of the last gather
         for (int dd = 0; dd < ndir; ++dd) {
             int64_t cur = c0 + dd;
             int snew = static_cast<int>(cur % nslots);
@@ -2286,7 +2290,7 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
                 // the network sees the residual left after the step along the two-level direction
                 // (zc is free again: its direction is stored in slot c0 % nslots)
                 const double* q0 = w.Q + static_cast<int>(c0 % nslots) * w.ld;
-                k_resid1<<<rs.grid, rs.block, 0, st>>>(w.r, q0, w.sc, static_cast<int>(c0 % nslots), n, zc, w.partial, nr);
+                k_resid1<<<rs.grid, rs.block, 0, st>>>(w.r, q0, w.sc, static_cast<int>(c0 % nslots), n, zc, w.partial, ng);
                 GF_TRY(nn_apply(nn, zc, w.sc, F_R1, w.partial + ROW_R1 * kRed, nr, nfree, d->part, d->nnu, w, w.z, st));
                 zin = w.z;
             }
@@ -2296,17 +2300,24 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
             }
             int nd = 0; // partials of the dots
             if (L.n > 0)
-                with_ns<MdotL>(L.n, st, zin, w.minv, w.r, w.Q, w.ld, L, n, w.partial, w.sc, fin_slot, nr, &nd);
+                with_ns<MdotL>(L.n, st, zin, w.minv, w.r, w.Q, w.ld, L, n, w.partial, w.sc, fin_slot, ng, &nd);
             with_ns<McombineL>(L.n, st, zin, w.minv, w.r, w.partial, nd, w.sc, w.P, w.ld, L, snew, n);
             double* Pn = w.P + snew * w.ld;
             double* Qn = w.Q + snew * w.ld;
-            GF_TRY(gfgpu_internal_iteration_element_forces(d, Pn, w.fe, st));
-            k_fgather<<<rs.grid, rs.block, 0, st>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, Pn, w.r, n,
-                                                    Qn, w.partial, reg_grid(d));
+            ng = 0;
+            if (gfgpu_internal_pair_operator(d))
+                GF_TRY(gfgpu_internal_tile_apply(d, Pn, w.r, Qn, w.partial + ROW_PQ * kRed, w.partial + ROW_RP * kRed,
+                                                 nullptr, nullptr, &ng, st));
+            if (ng == 0) {
+                ng = nr;
+                GF_TRY(gfgpu_internal_iteration_element_forces(d, Pn, w.fe, st));
+                k_fgather<<<rs.grid, rs.block, 0, st>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, Pn, w.r,
+                                                        n, Qn, w.partial, reg_grid(d));
+            }
         }
         k_mupdate<<<rs.grid, rs.block, 0, st>>>(d->part, d->nnu, w.P, w.Q, w.ld, static_cast<int>(c0 % nslots),
                                                 static_cast<int>((c0 + 1) % nslots), ndir, w.sc, n, x, w.r, w.partial,
-                                                nr);
+                                                ng);
         if (read || (nn && !post)) k_fredv<<<1, kWide, 0, st>>>(w.partial, ROW_RR, nr, F_RR, w.sc);
         return check_launch("fcg iteration");
     };

@@ -551,6 +551,10 @@ static int64_t pcg_bytes(const gfgpu_verlet_desc* d)
 
 using namespace gfgpu;
 
+// the operator on a Regular square Quad4 mesh in one kernel (verlet_pair.cu)
+int gfgpu_internal_tile_apply(const gfgpu_verlet_desc* d, const double* pv, const double* r, double* q, double* pq,
+                              double* rp, double* keep, const double* kept, int* nblk, cudaStream_t s);
+
 // element kernel launch shared with the explicit step (dynamics.cu)
 int gfgpu_internal_element_forces(const gfgpu_verlet_desc* d, const double* u, double* fe,
                                   cudaStream_t s);
@@ -560,12 +564,18 @@ int gfgpu_internal_pair_element_forces_f64(const gfgpu_verlet_desc* d, const dou
                                            cudaStream_t s);
 int gfgpu_internal_pair_coef_square(const gfgpu_verlet_desc* d, float* coef, cudaStream_t s);
 
+// whether the iterations apply the Quad4 pair operator (also asked by the flexible CG, learned.cu)
+bool gfgpu_internal_pair_operator(const gfgpu_verlet_desc* d)
+{
+    return d->pcg_pair && pcg_pair_kind(d) == 2;
+}
+
 // Element forces of an iteration's search direction: the Quad4 pair operator when d->pcg_pair is set
 // on a square Quad4 mesh, else the FP64 element kernel (also used by the flexible CG, learned.cu).
 int gfgpu_internal_iteration_element_forces(const gfgpu_verlet_desc* d, const double* u, double* fe,
                                             cudaStream_t s)
 {
-    if (d->pcg_pair && pcg_pair_kind(d) == 2) return gfgpu_internal_pair_element_forces_f64(d, u, fe, s);
+    if (gfgpu_internal_pair_operator(d)) return gfgpu_internal_pair_element_forces_f64(d, u, fe, s);
     return gfgpu_internal_element_forces(d, u, fe, s);
 }
 
@@ -659,10 +669,17 @@ static int pcg_iteration(const gfgpu_verlet_desc* d, const PcgWs& w, double* x, 
                                                       w.p, d->nnode, w.q, w.partial, w.sc, reg_grid(d));
     }
     else {
-        GF_TRY(gfgpu_internal_iteration_element_forces(d, w.p, w.fe, s));
-        gg = red_blocks(n);
-        k_pcg_gather<<<gg, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
-                                                 w.p, n, w.q, w.partial, w.sc, reg_grid(d));
+        int nblk = 0;
+        if (gfgpu_internal_pair_operator(d))
+            GF_TRY(gfgpu_internal_tile_apply(d, w.p, nullptr, w.q, w.partial, nullptr, w.sc + SC_RZ, w.sc + SC_RZ_NEW,
+                                             &nblk, s));
+        gg = static_cast<unsigned>(nblk);
+        if (nblk == 0) {
+            GF_TRY(gfgpu_internal_iteration_element_forces(d, w.p, w.fe, s));
+            gg = red_blocks(n);
+            k_pcg_gather<<<gg, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
+                                                     w.p, n, w.q, w.partial, w.sc, reg_grid(d));
+        }
     }
     // two wide blocks per SM, less where the dofs are fewer
     const unsigned gu = std::min<unsigned>(2 * 152, grid_for(n, kWideThreads));

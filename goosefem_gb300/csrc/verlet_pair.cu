@@ -954,6 +954,107 @@ k_verlet_tile(const TileStep p, const __grid_constant__ Tab tab)
     }
 }
 
+// The pair operator of the static solvers' iterations on a Regular mesh of square Quad4 elements in one
+// kernel: q = (A p)_u (0 on prescribed dofs) and a block's partials of p.q and, with r, r.p. Tiles as in
+// k_verlet_tile, one per block; the element forces and the order of the sums are those of
+// k_pair_elem_square_f64 and the gather, so q has their bits (the dots add up over tiles).
+// Below two tiles per SM the two kernels and the forces' way through memory are latency: an iteration of
+// the Jacobi flexible CG on 193 x 161 elements 20.3 -> 17.2 us, of the Jacobi-PCG on 160 x 170 20.6 ->
+// 18.7 us. At 256^2 (324 tiles) 22.7 -> 23.0, at 900^2 87.6 -> 96.5: the elements computed twice cost
+// more there.
+struct TileApply {
+    const double2 *p, *r;
+    double2* q;
+    const int2* part;
+    int64_t nnu;
+    const float4* cLN;
+    const float2* cH;
+    int nx, ny, tiles_x;
+    f2 nz;
+    double *pq, *rp;            // [blocks] partials; rp may be null
+    double* keep;               // block 0: keep[0] = kept[0] (may be null)
+    const double* kept;
+};
+
+template <int T>
+__global__ void __launch_bounds__(T * T)
+k_tile_apply(const TileApply p)
+{
+    __shared__ double2 sf[4][T * T];
+    __shared__ double sred[2][T * T / 32];
+    const int tid = threadIdx.x, lx = tid % T, ly = tid / T, nx = p.nx, ny = p.ny, W = nx + 1;
+    const int by = static_cast<int>(blockIdx.x) / p.tiles_x, bx = static_cast<int>(blockIdx.x) - by * p.tiles_x;
+    const int ix = bx * (T - 1) + lx, iy = by * (T - 1) + ly, node = iy * W + ix;
+    const bool own = lx < T - 1 && ly < T - 1 && ix <= nx && iy <= ny;
+    if (p.keep && blockIdx.x == 0 && tid == 0) p.keep[0] = p.kept[0];
+    double2 pn = make_double2(0.0, 0.0), rn = pn;
+    int2 pt = make_int2(0, 0);
+    if (own) {
+        pn = p.p[node];
+        pt = __ldg(p.part + node);
+        if (p.r) rn = p.r[node];
+    }
+    const int ex = ix - 1, ey = iy - 1;
+    if (ex >= 0 && ex < nx && ey >= 0 && ey < ny) {
+        const int64_t e = static_cast<int64_t>(ey) * nx + ex;
+        const double2* un = p.p + ey * W + ex;
+        const double2 u0 = un[0], u1 = un[1], u3 = un[W], u2 = un[W + 1];
+        ff2 g[4];
+        pair_square_forces2(u0, u1, u2, u3, __ldg(p.cLN + e), __ldg(p.cH + e), p.nz, g);
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+            sf[m][tid] = make_double2(ff_to_double(ff2_lane0(g[m])), ff_to_double(ff2_lane1(g[m])));
+    }
+    __syncthreads();
+    double pq = 0.0, rp = 0.0;
+    if (own) {
+        double2 f = make_double2(0.0, 0.0);
+        bool first = true;
+        auto take = [&](int m, int at, bool in) {
+            if (!in) return;
+            const double2 t = sf[m][at];
+            f.x = first ? t.x : f.x + t.x;
+            f.y = first ? t.y : f.y + t.y;
+            first = false;
+        };
+        take(2, tid, ix > 0 && iy > 0);
+        take(3, tid + 1, ix < nx && iy > 0);
+        take(1, tid + T, ix > 0 && iy < ny);
+        take(0, tid + T + 1, ix < nx && iy < ny);
+        if (pt.x < p.nnu) {
+            pq = fma(pn.x, f.x, pq);
+            rp = fma(rn.x, pn.x, rp);
+        }
+        else {
+            f.x = 0.0;
+        }
+        if (pt.y < p.nnu) {
+            pq = fma(pn.y, f.y, pq);
+            rp = fma(rn.y, pn.y, rp);
+        }
+        else {
+            f.y = 0.0;
+        }
+        p.q[node] = f;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        pq += __shfl_down_sync(0xffffffffu, pq, o);
+        if (p.rp) rp += __shfl_down_sync(0xffffffffu, rp, o);
+    }
+    if ((tid & 31) == 0) {
+        sred[0][tid >> 5] = pq;
+        sred[1][tid >> 5] = rp;
+    }
+    __syncthreads();
+    if (tid < 2 && (tid == 0 || p.rp)) {
+        double v = sred[tid][0];
+#pragma unroll
+        for (int w = 1; w < T * T / 32; ++w) v += sred[tid][w];
+        (tid == 0 ? p.pq : p.rp)[blockIdx.x] = v;
+    }
+}
+
 // flag = 1 if the tiles' meshes differ from conn or from the gather table
 template <int T>
 __global__ void __launch_bounds__(T * T)
@@ -1650,6 +1751,41 @@ int gfgpu_internal_tile_increment(const gfgpu_verlet_desc* d, const MassClassTab
         return edge == 8 ? launch_dependent(k_verlet_tile<true, 8, PairClassTab>, shape, s, 0, p, pair_class_tab(d))
                          : launch_dependent(k_verlet_tile<true, 16, PairClassTab>, shape, s, 0, p, pair_class_tab(d));
     return launch_dependent(k_verlet_tile<false, 8, MassClassTab>, shape, s, 0, p, tab);
+}
+
+// The static solvers' pair operator by k_tile_apply: *nblk = blocks (partials), 0 if it does not apply (then
+// nothing is launched).
+int gfgpu_internal_tile_apply(const gfgpu_verlet_desc* d, const double* pv, const double* r, double* q,
+                              double* pq, double* rp, double* keep, const double* kept, int* nblk, cudaStream_t s)
+{
+    *nblk = 0;
+    if (!d->pcg_pair) return GFGPU_OK;
+    if (!(d->reg_nx > 0 && d->reg_ny > 0 && d->reg_nz == 0 && d->reg_nx * d->reg_ny == d->nelem &&
+          (d->reg_nx + 1) * (d->reg_ny + 1) == d->nnode))
+        return GFGPU_OK;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(pv) | reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(q);
+    if ((at & 15u) != 0 || (reinterpret_cast<uintptr_t>(d->part) & 7u) != 0) return GFGPU_OK;
+    const int64_t n = grid_tiles(d->reg_nx, d->reg_ny, 16);
+    if (n > 2 * 152) return GFGPU_OK;
+    TileApply p;
+    p.p = reinterpret_cast<const double2*>(pv);
+    p.r = reinterpret_cast<const double2*>(r);
+    p.q = reinterpret_cast<double2*>(q);
+    p.part = reinterpret_cast<const int2*>(d->part);
+    p.nnu = d->nnu;
+    p.cLN = reinterpret_cast<const float4*>(d->pcg_pair);
+    p.cH = reinterpret_cast<const float2*>(d->pcg_pair + 4 * d->nelem);
+    p.nx = static_cast<int>(d->reg_nx);
+    p.ny = static_cast<int>(d->reg_ny);
+    p.tiles_x = static_cast<int>((d->reg_nx + 15) / 15);
+    p.nz = kF2NegZero;
+    p.pq = pq;
+    p.rp = rp;
+    p.keep = keep;
+    p.kept = kept;
+    *nblk = static_cast<int>(n);
+    k_tile_apply<16><<<static_cast<unsigned>(n), 256, 0, s>>>(p);
+    return check_launch("tile operator");
 }
 
 // {L, N} [nelem] interleaved pairs, then kH [nelem] (6 floats per element) of a uniform square Quad4

@@ -354,8 +354,9 @@ typedef struct {
     /* Quad4 Mesh::Quad4::Regular(reg_nx, reg_ny) numbering with dofs = node * 2 + i, verified
      * on the device by gfgpu_verlet_detect_regular: the node kernel and the static solvers'
      * operator (gfgpu_pcg_*, gfgpu_fcg_*, gfgpu_coarse_setup) then find the <= 4 element forces of
-     * a node by index arithmetic instead of the CSR (same summation order, same bits).
-     * 0 = use the CSR. */
+     * a node by index arithmetic instead of the CSR (same summation order, same bits; with pcg_pair
+     * the iterations on at most 304 tiles of 15 x 15 nodes apply the operator in one kernel, whose dot
+     * products add up over the tiles). 0 = use the CSR. */
     int64_t reg_nx, reg_ny;
     /* Hex8 Mesh::Hex8::Regular(reg_nx, reg_ny, reg_nz) numbering with dofs = node * 3 + i,
      * verified by gfgpu_verlet_detect_regular_hex8: the static solvers' operator gathers a node's
