@@ -4,10 +4,10 @@ Every instance has its own size, per-element moduli, fully periodic dofs
 (RegularBase::dofsPeriodic, Mesh.h:291-306) and an applied mean shear (the affine displacement
 of docs/examples/dynamics/Elastic-VelocityVerlet/main.cpp:88-98). The instances are concatenated
 into one block-diagonal mesh (node and dof numbers offset per instance), so one launch covers
-all of them: either a CUDA graph of the two kernels per increment (FP64, mode 0; float-float
+all of them: either a CUDA graph of the kernels of each increment (FP64, mode 0; float-float
 pairs, mode 2: square closed form + dof-CSR node kernel, gfgpu_verlet_precompute_pair path 2;
-mixed, mode 3: the pair element kernel on node differences formed in FP64 + the FP64 node
-kernel), or one persistent cooperative kernel for all increments (FP64, mode 1). `autotune` times
+mixed, mode 3: one kernel per increment, pair element forces on node differences formed in FP64 and
+the node update), or one persistent cooperative kernel for all increments (FP64, mode 1). `autotune` times
 them (and the persistent block shapes) on a few increments and keeps the fastest.
 """
 
