@@ -783,70 +783,101 @@ __global__ void k_stress_strict(const double* __restrict__ eps, const double* __
 }
 
 // The same, fast arithmetic: sigma = lam tr I + 2 G eps with lam = K - 2 G / 3, which needs no
-// division (an FP64 division is a dozen instructions at 2 per SM and clock): 64 us for 4.1 M 2-d
-// points (4.3 TB/s) against 192 us in the form above; 40 against 96 us for 1.2 M 3-d points. For a symmetric strain, as SymGradN gives it, the products
-// below the diagonal are copies of those above; the others are formed when a lane of the warp needs
-// one. A thread per point; its ND^2 values go through shared memory where they are not two aligned
-// double2 (VEC), so that global memory is read and written in address order.
-template <int ND, bool VEC>
+// division (an FP64 division is a dozen instructions at 2 per SM and clock): 57 us for 4.1 M 2-d
+// points (4.6 TB/s) against 192 us in the form above; 40 against 96 us for 1.2 M 3-d points. For a
+// symmetric strain, as SymGradN gives it, the products below the diagonal are copies of those above;
+// the others are formed when a lane of the warp needs one.
+template <int ND>
+__device__ __forceinline__ void stress_point(double (&s)[ND * ND], double lam, double g2, bool all)
+{
+    double tr = s[0];
+#pragma unroll
+    for (int i = 1; i < ND; ++i) tr += s[i * ND + i];
+    const double lt = lam * tr;
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+        s[i * ND + i] = fma(g2, s[i * ND + i], lt);
+#pragma unroll
+        for (int j = 0; j < i; ++j) {
+            s[j * ND + i] *= g2;
+            if (all) s[i * ND + j] = s[j * ND + i];
+            else s[i * ND + j] *= g2;
+        }
+    }
+}
+
+template <int ND>
+__device__ __forceinline__ bool stress_symmetric(const double (&s)[ND * ND])
+{
+    bool sym = true;
+#pragma unroll
+    for (int i = 0; i < ND; ++i)
+#pragma unroll
+        for (int j = 0; j < i; ++j)
+            sym = sym && __double_as_longlong(s[i * ND + j]) == __double_as_longlong(s[j * ND + i]);
+    return sym;
+}
+
+// A thread per point; its ND^2 values go through shared memory, so that global memory is read and
+// written in address order.
+template <int ND>
 __global__ void __launch_bounds__(kBlock)
 k_stress(const double* __restrict__ eps, const double* __restrict__ K, const double* __restrict__ G,
          int64_t npoint, uint32_t nip, double* __restrict__ sig)
 {
     constexpr int T = ND * ND;
-    __shared__ double sm[VEC ? 1 : kBlock * T];
+    __shared__ double sm[kBlock * T];
     const int64_t t0 = static_cast<int64_t>(blockIdx.x) * kBlock, t = t0 + threadIdx.x;
     const int n = static_cast<int>(npoint - t0 < kBlock ? npoint - t0 : kBlock);
     const bool on = static_cast<int>(threadIdx.x) < n;
     double s[T];
-    if constexpr (VEC) {
-        if (on) load<T>(eps + t * T, s);
-    }
-    else {
-        for (int i = threadIdx.x; i < n * T; i += kBlock) sm[i] = __ldg(eps + t0 * T + i);
-        __syncthreads();
-        if (on)
-#pragma unroll
-            for (int k = 0; k < T; ++k) s[k] = sm[threadIdx.x * T + k];
-    }
+    for (int i = threadIdx.x; i < n * T; i += kBlock) sm[i] = __ldg(eps + t0 * T + i);
+    __syncthreads();
     if (on) {
-        const uint32_t e = static_cast<uint32_t>(t) / nip;
-        const double Ge = __ldg(G + e), g2 = Ge + Ge, lam = fma(-2.0 / 3.0, Ge, __ldg(K + e));
-        double tr = s[0];
 #pragma unroll
-        for (int i = 1; i < ND; ++i) tr += s[i * ND + i];
-        const double lt = lam * tr;
+        for (int k = 0; k < T; ++k) s[k] = sm[threadIdx.x * T + k];
+        const uint32_t e = static_cast<uint32_t>(t) / nip;
+        const double Ge = __ldg(G + e), lam = fma(-2.0 / 3.0, Ge, __ldg(K + e));
+        const bool all = __all_sync(__activemask(), stress_symmetric<ND>(s));
+        stress_point<ND>(s, lam, Ge + Ge, all);
+#pragma unroll
+        for (int k = 0; k < T; ++k) sm[threadIdx.x * T + k] = s[k];
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n * T; i += kBlock) sig[t0 * T + i] = sm[i];
+}
+
+// 2-d tensors as two aligned double2 a point, P points of one element per thread (`groups` of them per
+// element): the element's moduli once, and P times the loads in flight. 4.1 M points: one 64 us, two
+// 57 us, four 66 us (a quarter of each 128-byte line per load).
+template <int P>
+__global__ void __launch_bounds__(kBlock)
+k_stress_2d(const double2* __restrict__ eps, const double* __restrict__ K, const double* __restrict__ G,
+            int64_t n, uint32_t groups, double2* __restrict__ sig)
+{
+    GF_FOR(t, n)
+    {
+        double s[P][4];
         bool sym = true;
 #pragma unroll
-        for (int i = 0; i < ND; ++i)
+        for (int p = 0; p < P; ++p) {
+            const double2 x = __ldg(eps + 2 * (P * t + p)), y = __ldg(eps + 2 * (P * t + p) + 1);
+            s[p][0] = x.x;
+            s[p][1] = x.y;
+            s[p][2] = y.x;
+            s[p][3] = y.y;
+        }
+        const uint32_t e = static_cast<uint32_t>(t) / groups;
+        const double Ge = __ldg(G + e), lam = fma(-2.0 / 3.0, Ge, __ldg(K + e));
 #pragma unroll
-            for (int j = 0; j < i; ++j)
-                sym = sym && __double_as_longlong(s[i * ND + j]) == __double_as_longlong(s[j * ND + i]);
+        for (int p = 0; p < P; ++p) sym = sym && stress_symmetric<2>(s[p]);
         const bool all = __all_sync(__activemask(), sym);
 #pragma unroll
-        for (int i = 0; i < ND; ++i) {
-            s[i * ND + i] = fma(g2, s[i * ND + i], lt);
-#pragma unroll
-            for (int j = 0; j < i; ++j) {
-                s[j * ND + i] *= g2;
-                if (all) s[i * ND + j] = s[j * ND + i];
-                else s[i * ND + j] *= g2;
-            }
+        for (int p = 0; p < P; ++p) {
+            stress_point<2>(s[p], lam, Ge + Ge, all);
+            sig[2 * (P * t + p)] = make_double2(s[p][0], s[p][1]);
+            sig[2 * (P * t + p) + 1] = make_double2(s[p][2], s[p][3]);
         }
-    }
-    if constexpr (VEC) {
-        if (on) {
-            double2* o = reinterpret_cast<double2*>(sig + t * T);
-#pragma unroll
-            for (int k = 0; k < T / 2; ++k) o[k] = make_double2(s[2 * k], s[2 * k + 1]);
-        }
-    }
-    else {
-        if (on)
-#pragma unroll
-            for (int k = 0; k < T; ++k) sm[threadIdx.x * T + k] = s[k];
-        __syncthreads();
-        for (int i = threadIdx.x; i < n * T; i += kBlock) sig[t0 * T + i] = sm[i];
     }
 }
 
@@ -1119,11 +1150,18 @@ int gfgpu_elastic_stress(const double* eps, const double* K, const double* G, in
     if (strict_mode())
         k_stress_strict<<<g, kBlock, 0, s>>>(eps, K, G, nelem, nip, ndim, sig);
     else if (ndim == 3)
-        k_stress<3, false><<<g, kBlock, 0, s>>>(eps, K, G, nelem * nip, nip, sig);
-    else if (aligned16(eps) && aligned16(sig))
-        k_stress<2, true><<<g, kBlock, 0, s>>>(eps, K, G, nelem * nip, nip, sig);
+        k_stress<3><<<g, kBlock, 0, s>>>(eps, K, G, nelem * nip, nip, sig);
+    else if (aligned16(eps) && aligned16(sig)) {
+        auto run = [&](auto kernel, int p) {
+            kernel<<<grid_for(nelem * nip / p), kBlock, 0, s>>>(reinterpret_cast<const double2*>(eps), K, G,
+                                                                nelem * nip / p, static_cast<uint32_t>(nip / p),
+                                                                reinterpret_cast<double2*>(sig));
+        };
+        if (nip % 2 == 0) run(k_stress_2d<2>, 2);
+        else run(k_stress_2d<1>, 1);
+    }
     else
-        k_stress<2, false><<<g, kBlock, 0, s>>>(eps, K, G, nelem * nip, nip, sig);
+        k_stress<2><<<g, kBlock, 0, s>>>(eps, K, G, nelem * nip, nip, sig);
     return check_launch("elastic_stress");
 }
 
