@@ -1412,13 +1412,13 @@ inline int forward_f32(const void* wbf, const float* pf, const float* X, int B, 
 {
     GF_TRY(prepare_train());
     const TrainGrid g = train_grid(B, H, W);
-    k_conv_tile<4, false><<<tile_blocks(g, 4), 256, conv_smem(4, dil_of(0)), s>>>(X, wb(wbf, 0), pf + b_off(0), dil_of(0), g, nullptr,
+    k_conv_tile<4, false><<<tile_blocks(g, 3), 256, conv_smem(4, dil_of(0)), s>>>(X, wb(wbf, 0), pf + b_off(0), dil_of(0), g, nullptr,
                                                                    is_aligned16(X), w.a1);
     k_conv_tile<32, false><<<tile_blocks(g, 2), 256, conv_smem(32, dil_of(1)), s>>>(w.a1, wb(wbf, 1), pf + b_off(1), dil_of(1), g,
                                                                      nullptr, true, w.a2);
     k_conv_tile<32, false><<<tile_blocks(g, 2), 256, conv_smem(32, dil_of(2)), s>>>(w.a2, wb(wbf, 2), pf + b_off(2), dil_of(2), g,
                                                                      nullptr, true, w.a3);
-    k_conv_out<<<tile_blocks(g, 4), 256, conv_out_smem(dil_of(3)), s>>>(w.a3, wb(wbf, 3), pf + b_off(3), dil_of(3), g, w.y);
+    k_conv_out<<<tile_blocks(g, 5), kOutThreads, conv_out_smem(dil_of(3)), s>>>(w.a3, wb(wbf, 3), pf + b_off(3), dil_of(3), g, w.y);
     return check_launch("nn training forward");
 }
 
@@ -1438,7 +1438,7 @@ inline void data_grad(const float* dY, const void* wbf, int layer, const TrainGr
                       cudaStream_t s)
 {
     const int dil = dil_of(layer);
-    k_conv_tile<CO, true><<<tile_blocks(g, CO == 2 ? 4 : 2), 256, conv_smem(CO, dil), s>>>(dY, wb(wbf, layer), nullptr, dil, g, act,
+    k_conv_tile<CO, true><<<tile_blocks(g, CO == 2 ? 3 : 2), 256, conv_smem(CO, dil), s>>>(dY, wb(wbf, layer), nullptr, dil, g, act,
                                                                           true, dX);
 }
 

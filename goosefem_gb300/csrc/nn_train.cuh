@@ -120,15 +120,19 @@ inline size_t conv_smem(int CI, int dil)
 //   BWD = false: Y = relu(b + sum_t sum_ci X[p + dil off_t, ci] W[t, ci, co]), W [9][CI][32];
 //   BWD = true:  Y = (sum_t sum_co X[p - dil off_t, co] W[t, ci, co]) where act > 0, else 0:
 //                the gradient for the input of a layer 32 -> CI, W [9][32][CI].
-// 256 threads, 256 pixels x 32 channels: lane & 3 selects 8 output channels, the rest 4 pixels
-// (columns gl and gl + 8 of two rows). Per 4 input channels a thread issues 4 + 8 16-byte shared
+// 256 threads, 256 pixels x 32 channels: a thread has 8 output channels (cg) of 4 pixels (columns gl
+// and gl + 8 of two rows). Per 4 input channels a thread issues 4 + 8 16-byte shared
 // loads for 64 packed FMAs. Two blocks per SM (111 KB each at dilation 4, 128 registers): one
 // computes while the other copies its tile, and four warps per scheduler cover the shared loads.
-// 32 -> 32 at 32 x 96 x 96: 111 us forward, 124 us for the data gradient (72 us at the FMA rate);
+// 32 -> 32 at 32 x 96 x 96: 108 us forward, 122 us for the data gradient (72 us at the FMA rate);
 // one block with two tiles in shared memory 118 / 141 us (two warps per scheduler); a pixel per
-// thread, each weight read from shared memory for one FMA, 477 / 519 us.
+// thread, each weight read from shared memory for one FMA, 477 / 519 us. Shared-memory reads bound
+// it: with 4 channel groups and 2 pixels in a quarter-warp 111 / 124 us. The gradient's ReLU mask is
+// read as bits before the products (a step of 32 crops 861 -> 854 us against reads in the epilogue,
+// one after the other). With 2 or 4 input channels there is little to compute per staged byte: three
+// blocks per SM.
 template <int CI, bool BWD>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, CI == 32 ? 2 : 3)
 k_conv_tile(const float* __restrict__ X, const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
             int dil, TrainGrid g, const float* __restrict__ act, bool vec, float* __restrict__ Y)
 {
@@ -149,7 +153,11 @@ k_conv_tile(const float* __restrict__ X, const __nv_bfloat16* __restrict__ W, co
         }
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int cg = (lane & 3) * 8, gl = lane >> 2;
+    // a quarter-warp's 16-byte shared loads take 2 clocks for up to two different chunks, else 4: with 32
+    // input channels it holds 2 groups of output channels and 4 pixels (the 8 weight loads are the cheap
+    // ones), else 4 groups and 2 pixels
+    const int cg = (SWZ ? (lane & 1) | ((lane >> 2) & 2) : lane & 3) * 8;
+    const int gl = SWZ ? ((lane >> 1) & 3) | ((lane >> 2) & 4) : lane >> 2;
     const int sgn = BWD ? -dil : dil;
     f2 b0[4];
 #pragma unroll
@@ -161,6 +169,20 @@ k_conv_tile(const float* __restrict__ X, const __nv_bfloat16* __restrict__ W, co
         tile_origin(g, tile, b, y0, x0);
         stage_tile<CI, SWZ>(X, g, b, y0, x0, dil, vec, xs);
         cp_async_commit();
+        // bit 8 j + k: the activation of pixel j and channel cg + k is positive, read while the copies land
+        [[maybe_unused]] uint32_t pos = 0;
+        if constexpr (BWD) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int yy = y0 + 2 * warp + (j >> 1), xx = x0 + gl + 8 * (j & 1);
+                if (yy >= g.H || xx >= g.W) continue;
+                const float* a = act + ((b * g.H + yy) * g.W + xx) * 32 + cg;
+                const float4 m0 = *reinterpret_cast<const float4*>(a), m1 = *reinterpret_cast<const float4*>(a + 4);
+                const float m[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+#pragma unroll
+                for (int k = 0; k < 8; ++k) pos |= (m[k] > 0.0f ? 1u : 0u) << (8 * j + k);
+            }
+        }
         cp_async_wait<0>();
         __syncthreads();
         f2 acc[4][4];
@@ -221,11 +243,8 @@ k_conv_tile(const float* __restrict__ X, const __nv_bfloat16* __restrict__ W, co
                 v[2 * k + 1] = f2_hi(acc[j][k]);
             }
             if constexpr (BWD) {
-                const float4 m0 = *reinterpret_cast<const float4*>(act + o);
-                const float4 m1 = *reinterpret_cast<const float4*>(act + o + 4);
-                const float m[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
 #pragma unroll
-                for (int k = 0; k < 8; ++k) v[k] = m[k] > 0.0f ? v[k] : 0.0f;
+                for (int k = 0; k < 8; ++k) v[k] = (pos >> (8 * j + k)) & 1u ? v[k] : 0.0f;
             }
             else {
 #pragma unroll
@@ -243,12 +262,14 @@ inline size_t conv_out_smem(int dil)
     return (static_cast<size_t>(9 * 32 * 2) + tile_floats(32, dil)) * sizeof(float);
 }
 
-// Output layer 32 -> 2: Y = b + sum_t sum_ci X[p + dil off_t, ci] W[t, ci, co]. A thread per pixel
-// of the staged tile, its two outputs the lanes of one packed accumulator; 16-byte shared loads
-// bound it (one of the pixel and two of the weights per 4 packed FMAs), and four blocks per SM
-// overlap their copies. 26 us at 32 x 96 x 96 (300 us with a thread's pixel read from global memory
-// one float at a time).
-__global__ void __launch_bounds__(256)
+// Output layer 32 -> 2: Y = b + sum_t sum_ci X[p + dil off_t, ci] W[t, ci, co]. Two pixels (of rows ly
+// and ly + 8) of the staged tile per thread, a pixel's two outputs the lanes of one packed accumulator;
+// 16-byte shared loads bound it (4 clocks for the pixels of a warp, 2 for each of two weights), so the
+// weights serve two pixels. Five blocks per SM overlap their copies. 24 us at 32 x 96 x 96 (27 us with a
+// pixel per thread; 300 us with a thread's pixel read from global memory one float at a time).
+constexpr int kOutThreads = kTrainTile * kTrainTile / 2;
+
+__global__ void __launch_bounds__(kOutThreads)
 k_conv_out(const float* __restrict__ X, const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
            int dil, TrainGrid g, float* __restrict__ Y)
 {
@@ -256,7 +277,7 @@ k_conv_out(const float* __restrict__ X, const __nv_bfloat16* __restrict__ W, con
     const int hw = kTrainTile + 2 * dil;
     float* ws = sm;              // [9][32][2]
     float* xs = sm + 9 * 32 * 2; // [hw][hw][32]
-    for (int i = threadIdx.x; i < 9 * 32 * 2; i += 256) ws[i] = __bfloat162float(W[i]);
+    for (int i = threadIdx.x; i < 9 * 32 * 2; i += kOutThreads) ws[i] = __bfloat162float(W[i]);
     const int ly = threadIdx.x / kTrainTile, lx = threadIdx.x % kTrainTile;
     for (int64_t tile = blockIdx.x; tile < g.tiles; tile += gridDim.x) {
         int64_t b;
@@ -266,25 +287,33 @@ k_conv_out(const float* __restrict__ X, const __nv_bfloat16* __restrict__ W, con
         cp_async_commit();
         cp_async_wait<0>();
         __syncthreads();
-        f2 acc = f2_make(__ldg(bias), __ldg(bias + 1));
+        f2 acc[2];
+        acc[0] = acc[1] = f2_make(__ldg(bias), __ldg(bias + 1));
 #pragma unroll
         for (int t = 0; t < 9; ++t) {
             const int col = lx + dil + dil * (t % 3 - 1), key = (col & 7) * 4;
             const float* p = xs + ((ly + dil + dil * (t / 3 - 1)) * hw + col) * 32;
 #pragma unroll
             for (int c = 0; c < 32; c += 4) {
-                const float4 q = *reinterpret_cast<const float4*>(p + (c ^ key));
                 const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(ws + (t * 32 + c) * 2);
                 const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(ws + (t * 32 + c) * 2 + 4);
-                acc = f2_fma_acc(f2_make(q.x, q.x), w0.x, acc);
-                acc = f2_fma_acc(f2_make(q.y, q.y), w0.y, acc);
-                acc = f2_fma_acc(f2_make(q.z, q.z), w1.x, acc);
-                acc = f2_fma_acc(f2_make(q.w, q.w), w1.y, acc);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const float4 q = *reinterpret_cast<const float4*>(p + j * (kTrainTile / 2) * hw * 32 + (c ^ key));
+                    acc[j] = f2_fma_acc(f2_make(q.x, q.x), w0.x, acc[j]);
+                    acc[j] = f2_fma_acc(f2_make(q.y, q.y), w0.y, acc[j]);
+                    acc[j] = f2_fma_acc(f2_make(q.z, q.z), w1.x, acc[j]);
+                    acc[j] = f2_fma_acc(f2_make(q.w, q.w), w1.y, acc[j]);
+                }
             }
         }
-        if (y0 + ly < g.H && x0 + lx < g.W) {
-            const int64_t o = (b * g.H + y0 + ly) * g.W + x0 + lx;
-            *reinterpret_cast<float2*>(Y + o * 2) = make_float2(f2_lo(acc), f2_hi(acc));
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int yy = y0 + ly + j * (kTrainTile / 2);
+            if (yy < g.H && x0 + lx < g.W) {
+                const int64_t o = (b * g.H + yy) * g.W + x0 + lx;
+                *reinterpret_cast<float2*>(Y + o * 2) = make_float2(f2_lo(acc[j]), f2_hi(acc[j]));
+            }
         }
         __syncthreads();
     }
