@@ -404,8 +404,9 @@ typedef struct {
 #define GFGPU_MASS_CLASSES 16
 #define GFGPU_PRESCRIBED_CLASS 255
 
-/* Bytes of scratch the step needs (the element-force buffer, or the pair state when
- * d->coef_pair is set), 256-byte aligned size. */
+/* Bytes of scratch the step needs (the element-force buffer, which the one-kernel increment of grid
+ * meshes uses as its second displacement buffer, or the pair state when d->coef_pair is set), 256-byte
+ * aligned size. */
 int64_t gfgpu_verlet_workspace_bytes(const gfgpu_verlet_desc* d);
 /* Checks that dNx/vol describe congruent axis-aligned boxes with the Gauss rule, within `rtol`
  * relative to the largest |dNx| (vol: relative to the box volume): first on the host for the first
