@@ -6,6 +6,8 @@
 #include "common.cuh"
 #include "fixdot.cuh"
 
+#include <climits>
+
 namespace gfgpu {
 
 // ---------------------------------------------------------------- loads
@@ -567,25 +569,31 @@ k_int_tensor4(const double* __restrict__ dNx, const double* __restrict__ vol,
     }
 }
 
-// The same two contractions on the integer pipes (fixdot.cuh) for the Gauss rules (NNE points): FP64
-// issue bounds the kernel above at 200 and 2400 instructions per integration point. The tensors, the
-// gradients and the volume * gradients of an element are brought to one exponent each over all its
-// points, so that the entries of its matrix are integer sums until the end. A thread (m, j, k) loads
-// the (j, k) block of the tensor of point m and a few gradients of one direction, the largest exponents
-// per block and direction meet in shared memory, and the threads leave the limbs of what they loaded
-// there for all. An entry is judged by the largest terms that its block and directions can have: an
-// element whose blocks or directions differ by more than 2^24 in all (thin elements, tensors with one
-// weak block), or whose values leave the range, takes the FP64 form on operands in global memory.
-// 9177 Hex8 elements 326 -> 203 us against the FP64 form, 49k Quad4 80 -> 61 us, with a third of its
+// The same two contractions on the integer pipes (fixdot.cuh) for rules of NNE points (the Gauss and the
+// nodal rule, or any other): FP64 issue bounds the kernel above at 200 and 2400 instructions per
+// integration point. The tensors, the gradients and the volume * gradients of an element are brought to
+// one exponent each over all its points, so that the entries of its matrix are integer sums until the
+// end. A thread (m, j, k) loads the (j, k) block of the tensor of point m and a few gradients, the largest
+// exponents meet in shared memory, and the threads leave the limbs of what they loaded there for all,
+// with the exponents. What the limbs cut off is judged entry by entry: after the products a thread takes
+// the largest exponent of any term v g[m,i] C[i,j,k,l] g[n,l] of each of its entries, and if one lies more
+// than kSpread below that of the largest values (points of very different scale, a weak tensor block), or
+// a value leaves the range, the thread takes the FP64 form on operands in global memory.
+// 9177 Hex8 elements 326 -> 200 us against the FP64 form, 49k Quad4 80 -> 62 us, with a third of its
 // error; the integer multiply-add pipe is 59 % busy (half of it the multiply-adds, the rest the
-// conversions), 2 blocks per SM (registers).
+// conversions), 2 blocks per SM (registers; Quad4 3, with 2 of them 66 us). Looking at point m first saves
+// forming the exponents of all terms beside the products (Hex8 224 us). The nodal rule, whose gradients
+// hold zeros, looks at all points: 217 us.
 template <int NNE, int ND>
 struct Tensor4Fix {
     static constexpr int K = NNE * ND, C4 = ND * ND * ND * ND, G = NNE * ND, JK = ND * ND;
     static constexpr int TPE = NNE * ND * ND;
     static constexpr int EPB = ND == 2 ? 16 : 4;
     static constexpr int THREADS = TPE * EPB;
-    static constexpr int NE = JK + 2 * ND; // exponents per element: (j, k) blocks, gradients, v * gradients
+    static constexpr int NE = 3;           // exponents per element: tensors, gradients, v * gradients
+    // An entry's error is at most NNE * ND * (ND + 4) * 2^-82 (2^-74.6 for Hex8) of the product of the three
+    // scales, its largest term at least 2^-(kSpread + 3): an error below 2^-53 of that term.
+    static constexpr int kSpread = 18;
     static constexpr int NG = NNE * G;     // gradients per element
     static constexpr int SL = NNE * (C4 + 2 * G) + 1; // limbs per element (+ 1: elements on other banks)
     // the limbs, or the matrices that take their place, then the exponents
@@ -594,8 +602,26 @@ struct Tensor4Fix {
     static constexpr size_t SMEM = BODY + sizeof(int) * EPB * NE;
 };
 
+// top[n] = max(top[n], exponents of the terms of entry (m, j), (n, k) at point q)
+template <int NNE, int ND>
+__device__ __forceinline__ void tensor4_top(const int4* lim, int m, int j, int k, int q, int (&top)[NNE])
+{
+    using B = Tensor4Fix<NNE, ND>;
+    const int4* lc = lim + q * B::C4 + (j * ND + k) * ND;
+    const int4* lg = lim + NNE * B::C4 + q * B::G;
+    const int4* lv = lg + B::NG + m * ND;
+#pragma unroll
+    for (int l = 0; l < ND; ++l) {
+        int w = kFxNone;
+#pragma unroll
+        for (int i = 0; i < ND; ++i) w = max(w, lv[i].w + lc[i * ND * ND * ND + l].w);
+#pragma unroll
+        for (int n = 0; n < NNE; ++n) top[n] = max(top[n], w + lg[n * ND + l].w);
+    }
+}
+
 template <int NNE, int ND, int TD>
-__global__ void __launch_bounds__(Tensor4Fix<NNE, ND>::THREADS, 2)
+__global__ void __launch_bounds__(Tensor4Fix<NNE, ND>::THREADS, ND == 2 ? 3 : 2)
 k_int_tensor4_fix(const double* __restrict__ dNx, const double* __restrict__ vol, const double* __restrict__ C,
                   int64_t nelem, double* __restrict__ elemmat)
 {
@@ -603,7 +629,6 @@ k_int_tensor4_fix(const double* __restrict__ dNx, const double* __restrict__ vol
     constexpr int K = B::K, C4 = B::C4, G = B::G, JK = B::JK, T4 = TD * TD * TD * TD, NE = B::NE, SL = B::SL;
     constexpr int TPE = B::TPE, NG = B::NG, GT = (NG + TPE - 1) / TPE; // gradients per thread
     static_assert(3 * ND * NNE < 128, "ND * NNE products of limbs fit a 64-bit sum");
-    static_assert(TPE % ND == 0, "a thread's gradients are of one direction");
     extern __shared__ __align__(16) unsigned char smem[];
     const int tid = threadIdx.x;
     const int el = tid / TPE, r = tid - el * TPE;
@@ -640,31 +665,19 @@ k_int_tensor4_fix(const double* __restrict__ dNx, const double* __restrict__ vol
     }
     __syncthreads();
     if (on) {
-        atomicMax(ex + j * ND + k, xc);
-        atomicMax(ex + JK + r % ND, xg);
-        atomicMax(ex + JK + ND + r % ND, xv);
+        atomicMax(ex, xc);
+        atomicMax(ex + 1, xg);
+        atomicMax(ex + 2, xv);
     }
     __syncthreads();
-    // the largest exponents, and how far the scales lie apart
     int ec = 0, eg = 0, ev = 0;
     bool fix = false;
     if (on) {
-        int lc = 0x7ff, lg = 0x7ff, lv = 0x7ff;
-#pragma unroll
-        for (int b = 0; b < JK; ++b) {
-            ec = max(ec, ex[b]);
-            if (ex[b]) lc = min(lc, ex[b]); // a block of zeros is exact
-        }
-#pragma unroll
-        for (int i = 0; i < ND; ++i) {
-            eg = max(eg, ex[JK + i]);
-            lg = min(lg, ex[JK + i]);
-            ev = max(ev, ex[JK + ND + i]);
-            lv = min(lv, ex[JK + ND + i]);
-        }
+        ec = ex[0];
+        eg = ex[1];
+        ev = ex[2];
         const int sum = ec + eg + ev - 3 * 1022;
-        fix = ec > 100 && eg > 100 && ev > 100 && ec < 0x7ff && eg < 0x7ff && ev < 0x7ff && sum > -800 && sum < 900 &&
-              (ec - lc) + (eg - lg) + (ev - lv) <= 24;
+        fix = ec > 100 && eg > 100 && ev > 100 && ec < 0x7ff && eg < 0x7ff && ev < 0x7ff && sum > -800 && sum < 900;
         if (fix) {
 #pragma unroll
             for (int t = 0; t < JK; ++t) lim[m * C4 + ((t / ND * ND + j) * ND + k) * ND + t % ND] = fx_from_double(c[t], ec);
@@ -706,8 +719,23 @@ k_int_tensor4_fix(const double* __restrict__ dNx, const double* __restrict__ vol
         const int scale = ec + ev + eg - 3 * 1022 + 2;
 #pragma unroll
         for (int n = 0; n < NNE; ++n) res[n] = fx_to_double(acc[n], scale);
+        // the largest exponents of the entries' terms at point m, where they are nearly always enough, else
+        // at all points; an entry of zeros alone (below 0) is exact
+        int top[NNE], low = INT_MAX;
+#pragma unroll
+        for (int n = 0; n < NNE; ++n) top[n] = kFxNone;
+        tensor4_top<NNE, ND>(lim, m, j, k, m, top);
+#pragma unroll
+        for (int n = 0; n < NNE; ++n) low = min(low, top[n]);
+        const int need = ec + ev + eg - B::kSpread;
+        if (low < need) {
+#pragma unroll 1
+            for (int q = 0; q < NNE; ++q) tensor4_top<NNE, ND>(lim, m, j, k, q, top);
+#pragma unroll
+            for (int n = 0; n < NNE; ++n) fix = fix && (top[n] < 0 || top[n] >= need);
+        }
     }
-    else if (on) {
+    if (on && !fix) {
 #pragma unroll
         for (int n = 0; n < NNE; ++n) res[n] = 0.0;
 #pragma unroll 1

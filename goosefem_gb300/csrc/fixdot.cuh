@@ -7,12 +7,13 @@
 // products fit without a carry. So a dot product costs a fifth of an FP64 one in issue time, and
 // nothing is rounded until its end.
 //
-// Accuracy. An entry is cut at 2^-84 of its vector's largest (a double has 53 bits, so entries within
-// 2^31 of the largest are held exactly), and a product at 2^-82 of the largest times the largest. The
-// caller checks how far the scales within its vectors lie apart: with at most 2^24 between the largest
-// product and the scale that a result is judged by, the error is 2^-54 of that scale, below the
-// rounding of one FP64 operation. Where that does not hold, or a value is infinite, NaN or near the
-// ends of the exponent range, the caller takes its FP64 path.
+// Accuracy. With S = 2^(emax - 1022) of each vector, an entry is cut at 2^-84 S (a double has 53 bits, so
+// entries within 2^31 of the largest are held exactly) and a product at 2^-82 of the two vectors' S. That
+// says nothing about a result whose terms are all far below the product of the largest entries (a large
+// entry may meet only small ones), so limbs carry their entry's exponent and the caller forms the largest
+// exponent of the terms that a result does have. Where it lies too far below the vectors' (the caller
+// states the bound), or a value is infinite, NaN or near the ends of the exponent range, the caller takes
+// its FP64 path.
 #pragma once
 
 #include <cstdint>
@@ -29,8 +30,12 @@ __device__ __forceinline__ int fx_exponent(double d)
     return (__double2hiint(d) >> 20) & 0x7ff;
 }
 
-// d / 2^(emax - 1022) as limbs {x, y, z}: x 2^-28 + y 2^-56 + z 2^-84, emax >= the exponent of d;
-// subnormals count as zero (they lie below the cut of any vector the caller may pass)
+// what a zero has in the place of an exponent: below 0 with any two exponents added
+constexpr int kFxNone = -(1 << 14);
+
+// d / 2^(emax - 1022) as limbs {x, y, z}: x 2^-28 + y 2^-56 + z 2^-84, emax >= the exponent of d, and in w
+// the exponent (1 for a subnormal, kFxNone for a zero); subnormals count as zero (they lie below the cut
+// of any vector the caller may pass)
 __device__ __forceinline__ int4 fx_from_double(double d, int emax)
 {
     const uint32_t hi = static_cast<uint32_t>(__double2hiint(d)), lo = static_cast<uint32_t>(__double2loint(d));
@@ -55,7 +60,8 @@ __device__ __forceinline__ int4 fx_from_double(double d, int emax)
     const uint32_t r2 = s < 32u ? w2 >> s : 0u;
     const int sg = static_cast<int>(hi) >> 31 | 1; // +-1
     return make_int4(static_cast<int>(__funnelshift_l(r1, r2, 8)) * sg,
-                     static_cast<int>(__funnelshift_l(r0, r1, 4) & kFxMask) * sg, static_cast<int>(r0 & kFxMask) * sg, 0);
+                     static_cast<int>(__funnelshift_l(r0, r1, 4) & kFxMask) * sg, static_cast<int>(r0 & kFxMask) * sg,
+                     e ? e : (((hi << 1) | lo) ? 1 : kFxNone));
 }
 
 // sum of products: a 2^-56 + b 2^-84 + c 2^-112 (times the scales of the two vectors)
