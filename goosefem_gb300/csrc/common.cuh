@@ -66,7 +66,8 @@ inline Shape spread(int64_t n, int block = kBlock)
 // reads what a predecessor writes and before it writes anything, and what predecessors write is read
 // with plain loads (read-only loads, __ldg or a const __restrict__ parameter, may be moved ahead of
 // the wait and promise data that no one writes while the kernel runs). pdl_wait returns at once in a
-// kernel launched without the attribute.
+// kernel launched without the attribute. What such a chain takes as constant (tables, coefficients) may
+// have been written by the kernel just before the call, so a call's first kernel is launched plainly.
 __device__ __forceinline__ void pdl_wait()
 {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -79,7 +80,8 @@ __device__ __forceinline__ void pdl_launch_dependents()
 }
 
 template <class... P, class... A>
-inline int launch_dependent(void (*kernel)(P...), Shape shape, cudaStream_t s, size_t smem, const A&... args)
+inline int launch_chained(bool dependent, void (*kernel)(P...), Shape shape, cudaStream_t s, size_t smem,
+                          const A&... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(shape.grid);
@@ -90,8 +92,14 @@ inline int launch_dependent(void (*kernel)(P...), Shape shape, cudaStream_t s, s
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = dependent ? 1 : 0;
     return check_cuda(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...), "cudaLaunchKernelEx");
+}
+
+template <class... P, class... A>
+inline int launch_dependent(void (*kernel)(P...), Shape shape, cudaStream_t s, size_t smem, const A&... args)
+{
+    return launch_chained(true, kernel, shape, s, smem, args...);
 }
 
 // Strict arithmetic: every product and sum rounded on its own (no FMA contraction), which

@@ -1418,7 +1418,7 @@ static int nxp_of(int64_t nx)
 template <int TY>
 static int launch_tma(PairTmaStep p, const CUtensorMap* mu, const CUtensorMap& mv, const CUtensorMap& ma,
                       const CUtensorMap& ml, const CUtensorMap& mh, const PairClassTab& tab, int64_t first,
-                      int64_t count, int advance_last, float4* const* ub, int sms, cudaStream_t s)
+                      int64_t count, int advance_last, bool chained, float4* const* ub, int sms, cudaStream_t s)
 {
     using Gm = TmaGeom<TY>;
     static bool attr = false;
@@ -1440,8 +1440,8 @@ static int launch_tma(PairTmaStep p, const CUtensorMap* mu, const CUtensorMap& m
     for (int64_t it = first; it < first + count; ++it) {
         p.uout = ub[(it + 1) & 1];
         p.advance = (it + 1 < first + count || advance_last) ? 1 : 0;
-        GF_TRY(launch_dependent(k_verlet_pair_tma<TY>, Shape{static_cast<unsigned>(grid), Gm::threads}, s, Gm::Smem,
-                                mu[it & 1], mv, ma, ml, mh, p, tab));
+        GF_TRY(launch_chained(chained || it > first, k_verlet_pair_tma<TY>, Shape{static_cast<unsigned>(grid), Gm::threads},
+                              s, Gm::Smem, mu[it & 1], mv, ma, ml, mh, p, tab));
     }
     return GFGPU_OK;
 }
@@ -1495,8 +1495,9 @@ static int pair_begin(const gfgpu_verlet_desc* d, const double* u, const double*
     return check_launch("pair begin");
 }
 
+// chained: a kernel of the same call goes before
 static int pair_increments(const gfgpu_verlet_desc* d, int64_t first, int64_t count, int advance_last,
-                           void* workspace, cudaStream_t s)
+                           bool chained, void* workspace, cudaStream_t s)
 {
     if (count <= 0) return GFGPU_OK;
     const PairState ps = pair_state(d, workspace);
@@ -1532,12 +1533,12 @@ static int pair_increments(const gfgpu_verlet_desc* d, int64_t first, int64_t co
         const Shape l = spread(d->nelem, 256), h = spread(d->nelem, 128), r = spread(q.n, 256);
         for (int64_t it = first; it < first + count; ++it) {
             if (d->pair_mode == 2)
-                GF_TRY(launch_dependent(k_pair_elem_square, l, s, 0, d->conn, ub[0],
-                                        reinterpret_cast<const float4*>(d->coef_pair),
-                                        reinterpret_cast<const float2*>(d->coef_pair + 4 * d->nelem), d->nelem, fe));
+                GF_TRY(launch_chained(chained || it > first, k_pair_elem_square, l, s, 0, d->conn, ub[0],
+                                      reinterpret_cast<const float4*>(d->coef_pair),
+                                      reinterpret_cast<const float2*>(d->coef_pair + 4 * d->nelem), d->nelem, fe));
             else
-                GF_TRY(launch_dependent(k_pair_elem_stiff, h, s, 0, d->conn, ub[0],
-                                        reinterpret_cast<const float2*>(d->coef_pair), d->nelem, fe));
+                GF_TRY(launch_chained(chained || it > first, k_pair_elem_stiff, h, s, 0, d->conn, ub[0],
+                                      reinterpret_cast<const float2*>(d->coef_pair), d->nelem, fe));
             q.advance = (it + 1 < first + count || advance_last) ? 1 : 0;
             GF_TRY(launch_dependent(k_pair_node_csr, r, s, 0, q, tab));
         }
@@ -1597,8 +1598,8 @@ static int pair_increments(const gfgpu_verlet_desc* d, int64_t first, int64_t co
     p.dt = split_host(dt);
     p.cc = split_host(c);
     p.nz = kF2NegZero;
-    if (TY == 15) return launch_tma<15>(p, mu, mv, ma, ml, mh, tab, first, count, advance_last, ub, sms, s);
-    return launch_tma<7>(p, mu, mv, ma, ml, mh, tab, first, count, advance_last, ub, sms, s);
+    if (TY == 15) return launch_tma<15>(p, mu, mv, ma, ml, mh, tab, first, count, advance_last, chained, ub, sms, s);
+    return launch_tma<7>(p, mu, mv, ma, ml, mh, tab, first, count, advance_last, chained, ub, sms, s);
 }
 
 static int pair_end(const gfgpu_verlet_desc* d, int64_t last, double* u, double* v, double* a, void* workspace,
@@ -1618,7 +1619,7 @@ int gfgpu_internal_verlet_pair(const gfgpu_verlet_desc* d, double* u, double* v,
 {
     GF_TRY(pair_check(d, workspace));
     GF_TRY(pair_begin(d, u, v, a, workspace, s));
-    GF_TRY(pair_increments(d, 0, nsteps, 0, workspace, s));
+    GF_TRY(pair_increments(d, 0, nsteps, 0, true, workspace, s));
     // the last increment does not advance: its displacement is the one it read
     return pair_end(d, nsteps - 1, u, v, a, workspace, s);
 }
@@ -1889,7 +1890,7 @@ int gfgpu_verlet_pair_increments(const gfgpu_verlet_desc* d, int64_t first, int6
 {
     GF_REQUIRE(d && first >= 0 && count >= 0, "bad argument");
     GF_TRY(pair_check(d, workspace));
-    return pair_increments(d, first, count, advance_last ? 1 : 0, workspace, S(stream));
+    return pair_increments(d, first, count, advance_last ? 1 : 0, false, workspace, S(stream));
 }
 
 int gfgpu_verlet_pair_end(const gfgpu_verlet_desc* d, int64_t last, double* u, double* v, double* a,
