@@ -29,6 +29,7 @@ inline cudaStream_t S(gfgpu_stream_t s)
 }
 
 constexpr int kBlock = 256;
+constexpr int kSMs = 152; // of a GB300
 
 inline unsigned grid_for(int64_t n, int block = kBlock)
 {
@@ -38,7 +39,7 @@ inline unsigned grid_for(int64_t n, int block = kBlock)
 }
 
 // Launch shape of n independent entries, `block` threads at most: below one full block per SM the
-// blocks shrink to what puts one on each of the 152 SMs. An FP64 instruction of a warp takes 16 clocks
+// blocks shrink to what puts one on each SM. An FP64 instruction of a warp takes 16 clocks
 // of its SM, so eight warps on one SM of an otherwise idle chip take eight times as long as one warp on
 // each of eight (an increment of 1920 Quad4 elements 12.6 -> 10.5 us, of 576 distorted Hex8 74 -> 58 us).
 struct Shape {
@@ -48,11 +49,14 @@ struct Shape {
 
 inline Shape spread(int64_t n, int block = kBlock)
 {
-    constexpr int64_t kSMs = 152;
     const int64_t b = ((n + kSMs - 1) / kSMs + 31) / 32 * 32;
     if (b < block) block = static_cast<int>(b < 32 ? 32 : b);
     return Shape{grid_for(n, block), block};
 }
+
+// Most tiles that the static solvers' one-kernel operator takes (k_tile_apply, verlet_pair.cu), one block and
+// one partial of its dot products each: the solvers' rows of partials have to hold as many.
+constexpr int kApplyTiles = 2 * kSMs;
 
 // Grid-stride loop bound used by elementwise kernels.
 #define GF_FOR(i, n)                                                                            \

@@ -1270,8 +1270,9 @@ int gfgpu_internal_coarse_apply(const gfgpu_coarse_desc* g, const int32_t* part,
 namespace gfgpu {
 namespace nn {
 
-constexpr int kWgtBlocks = 152; // weight-gradient partials: a block on each of the 152 SMs
-constexpr int kRed = 304; // most blocks (and partials per row) of the FCG reductions: two per SM
+constexpr int kWgtBlocks = kSMs; // weight-gradient partials: a block on each SM
+constexpr int kRed = 2 * kSMs; // most blocks (and partials per row) of the FCG reductions: two per SM
+static_assert(kApplyTiles <= kRed, "the one-kernel operator's partials fit a row");
 
 inline int64_t a256(int64_t b)
 {
@@ -1380,12 +1381,12 @@ inline bool is_aligned16(const void* p)
     return (reinterpret_cast<uintptr_t>(p) & 15u) == 0;
 }
 
-// Blocks of a tile kernel: one wave of `per_sm` blocks on each of the 152 SMs (what its shared
+// Blocks of a tile kernel: one wave of `per_sm` blocks on each SM (what its shared
 // memory allows) walks the tiles when there are more, so that the weights are staged once per
 // block, else one block per tile.
 inline unsigned tile_blocks(const TrainGrid& g, int per_sm)
 {
-    return static_cast<unsigned>(std::min<int64_t>(g.tiles, int64_t(152) * per_sm));
+    return static_cast<unsigned>(std::min<int64_t>(g.tiles, int64_t(kSMs) * per_sm));
 }
 
 // dynamic shared memory above 48 KB, granted per device and kernel
@@ -1426,7 +1427,7 @@ template <int CI, int CO>
 inline void weight_grad(const float* X, const float* dY, int dil, const TrainGrid& g, float* partial, float* grad,
                         cudaStream_t s)
 {
-    const unsigned nb = tile_blocks(g, kWgtBlocks / 152);
+    const unsigned nb = tile_blocks(g, kWgtBlocks / kSMs);
     k_wgrad_tile<CI, CO><<<nb, kWgradThreads, wgrad_smem(CI, CO, dil), s>>>(X, dY, dil, g, is_aligned16(X), partial);
     const int n = 9 * CI * CO + CO;
     k_sum_partials<<<(n + 31) / 32, 256, 0, s>>>(partial, static_cast<int>(nb), n, grad);

@@ -21,6 +21,7 @@ constexpr int kRedBlocks = 4096; // most blocks (and partials per row) of a redu
 constexpr int kRedThreads = 256;
 constexpr int kReduceThreads = 1024; // the one-block kernels that add the partials (set-up, residual)
 constexpr int kWideThreads = 1024;   // update and direction
+static_assert(kApplyTiles <= kRedBlocks && 2 * kSMs <= kRedBlocks, "partials fit a row");
 
 // Blocks of a reduction kernel over n entries: one entry per thread up to kRedBlocks blocks. Fixed by
 // n: the same sums on every run.
@@ -682,7 +683,7 @@ static int pcg_iteration(const gfgpu_verlet_desc* d, const PcgWs& w, double* x, 
         }
     }
     // two wide blocks per SM, less where the dofs are fewer
-    const unsigned gu = std::min<unsigned>(2 * 152, grid_for(n, kWideThreads));
+    const unsigned gu = std::min<unsigned>(2 * kSMs, grid_for(n, kWideThreads));
     if (rr)
         k_pcg_update<true><<<gu, kWideThreads, 0, s>>>(d->part, d->nnu, w.minv, w.p, w.q, n, w.sc, x, w.r, w.z,
                                                        w.partial, static_cast<int>(gg), w.partial);

@@ -1682,7 +1682,7 @@ int gfgpu_internal_mixed_increment(const gfgpu_verlet_desc* d, double* fe, int a
 // of 8 per SM on, FP64 issue bounds the FP64 increment and the elements computed twice on the rims cost
 // more than the launch: two kernels there. Mixed arithmetic has the room; tiles of 16 compute 1.14
 // elements per node instead of 1.31.
-constexpr int64_t kTilesFew = 3 * 152;
+constexpr int64_t kTilesFew = 3 * kSMs;
 
 static int tile_edge(int64_t tiles16)
 {
@@ -1767,7 +1767,7 @@ int gfgpu_internal_tile_apply(const gfgpu_verlet_desc* d, const double* pv, cons
     const uintptr_t at = reinterpret_cast<uintptr_t>(pv) | reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(q);
     if ((at & 15u) != 0 || (reinterpret_cast<uintptr_t>(d->part) & 7u) != 0) return GFGPU_OK;
     const int64_t n = grid_tiles(d->reg_nx, d->reg_ny, 16);
-    if (n > 2 * 152) return GFGPU_OK;
+    if (n > kApplyTiles) return GFGPU_OK;
     TileApply p;
     p.p = reinterpret_cast<const double2*>(pv);
     p.r = reinterpret_cast<const double2*>(r);
