@@ -32,7 +32,7 @@ inline unsigned red_blocks(int64_t n)
 
 // scalar slots
 // SC_RZ: r.z of the current direction; SC_RZ_NEW: of the last update (copied by the next gather)
-enum { SC_RZ = 0, SC_RZ_NEW, SC_PQ, SC_RR, SC_BB, SC_ALPHA, SC_BETA, SC_COUNT };
+enum { SC_RZ = 0, SC_RZ_NEW, SC_RR, SC_BB, SC_COUNT };
 
 // Sum over the block's threads, a fixed order, valid in thread 0 (sh: blockDim doubles). An FP64
 // instruction of a warp takes 16 clocks of the SM's pipe, so the sum is left to one warp: 8 + 5 of
@@ -51,18 +51,14 @@ __device__ __forceinline__ double block_sum(double v, double* sh)
     return r;
 }
 
-// Final fixed-order reduction of `nparts` partial rows (nblk partials each) into scalars.
-__global__ void k_reduce(const double* __restrict__ partials, int nblk, int nparts, double* __restrict__ sc,
-                         int slot0)
+// Final fixed-order reduction of a row of nblk partials into a scalar.
+__global__ void k_reduce(const double* __restrict__ partials, int nblk, double* __restrict__ sc, int slot)
 {
     __shared__ double sh[kReduceThreads];
-    for (int p = 0; p < nparts; ++p) {
-        double v = 0.0;
-        for (int i = threadIdx.x; i < nblk; i += blockDim.x) v += partials[p * kRedBlocks + i];
-        double s = block_sum(v, sh);
-        if (threadIdx.x == 0) sc[slot0 + p] = s;
-        __syncthreads();
-    }
+    double v = 0.0;
+    for (int i = threadIdx.x; i < nblk; i += blockDim.x) v += partials[i];
+    double s = block_sum(v, sh);
+    if (threadIdx.x == 0) sc[slot] = s;
 }
 
 // q = A p on free dofs (gather of the element forces), 0 on prescribed dofs; partial p.q.
@@ -118,16 +114,12 @@ template <bool RR>
 __global__ void __launch_bounds__(kWideThreads, 2)
 k_pcg_update(const int32_t* __restrict__ part, int64_t nnu, const double* __restrict__ minv,
              const double* __restrict__ p, const double* __restrict__ q, int64_t n,
-             double* __restrict__ sc, double* __restrict__ x, double* __restrict__ r,
+             const double* __restrict__ sc, double* __restrict__ x, double* __restrict__ r,
              double* __restrict__ z, const double* __restrict__ pq_part, int nblk, double* __restrict__ partial)
 {
     __shared__ double sh[kWideThreads];
     const double pq = sum_partials(pq_part, nblk, sh);
     const double alpha = from_thread0(threadIdx.x == 0 ? sc[SC_RZ] / pq : 0.0, sh);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        sc[SC_PQ] = pq;
-        sc[SC_ALPHA] = alpha;
-    }
     double rz = 0.0, rr = 0.0;
     GF_FOR(t, n)
     {
@@ -161,7 +153,6 @@ __device__ __forceinline__ double direction_beta(const double* __restrict__ part
         if (threadIdx.x == 0) {
             sc[SC_RZ_NEW] = rz;
             if (with_rr) sc[SC_RR] = rr;
-            sc[SC_BETA] = beta;
         }
     }
     return beta;
@@ -733,13 +724,13 @@ int gfgpu_pcg_solve(const gfgpu_verlet_desc* d, const double* diag, double* x, d
     if ((rc = gfgpu_internal_element_forces(d, w.p, w.fe, s)) != GFGPU_OK) return fail_out(rc);
     k_pcg_residual<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
                                                nullptr, w.minv, n, w.bvec, w.z, nullptr, w.partial, reg_grid(d));
-    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), 1, w.sc, SC_BB);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), w.sc, SC_BB);
     // r = b - A x, z = M^-1 r, p = z
     if ((rc = gfgpu_internal_element_forces(d, x, w.fe, s)) != GFGPU_OK) return fail_out(rc);
     k_pcg_residual<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
                                                nullptr, w.minv, n, w.r, w.z, w.p, w.partial, reg_grid(d));
-    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial, static_cast<int>(gb), 1, w.sc, SC_RZ_NEW);
-    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), 1, w.sc, SC_RR);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial, static_cast<int>(gb), w.sc, SC_RZ_NEW);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), w.sc, SC_RR);
     if (d->pcg_pair && d->nne == 8) k_pcg_split<<<grid_for(n), kBlock, 0, s>>>(w.p, n, w.pp);
     if ((rc = check_launch("pcg set-up")) != GFGPU_OK) return fail_out(rc);
     cudaMemcpyAsync(hsc, w.sc, SC_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -815,7 +806,7 @@ int gfgpu_pcg_solve(const gfgpu_verlet_desc* d, const double* diag, double* x, d
     if ((rc = gfgpu_internal_element_forces(d, x, w.fe, s)) != GFGPU_OK) return fail_out(rc);
     k_pcg_residual<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
                                                nullptr, w.minv, n, w.r, w.z, nullptr, w.partial, reg_grid(d));
-    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), 1, w.sc, SC_RR);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), w.sc, SC_RR);
     cudaMemcpyAsync(hsc, w.sc, SC_COUNT * sizeof(double), cudaMemcpyDeviceToHost, s);
     if ((rc = check_cuda(cudaStreamSynchronize(s), "pcg final residual")) != GFGPU_OK)
         return fail_out(rc);
@@ -843,13 +834,13 @@ int gfgpu_pcg_begin(const gfgpu_verlet_desc* d, const double* diag, const double
     GF_TRY(gfgpu_internal_element_forces(d, w.p, w.fe, s));
     k_pcg_residual<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
                                                rhs, w.minv, n, w.bvec, w.z, nullptr, w.partial, reg_grid(d));
-    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), 1, w.sc, SC_BB);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), w.sc, SC_BB);
     // r = rhs_u - (A x)_u, z = M^-1 r, p = z
     GF_TRY(gfgpu_internal_element_forces(d, x, w.fe, s));
     k_pcg_residual<<<gb, kRedThreads, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe,
                                                rhs, w.minv, n, w.r, w.z, w.p, w.partial, reg_grid(d));
-    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial, static_cast<int>(gb), 1, w.sc, SC_RZ_NEW);
-    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), 1, w.sc, SC_RR);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial, static_cast<int>(gb), w.sc, SC_RZ_NEW);
+    k_reduce<<<1, kReduceThreads, 0, s>>>(w.partial + kRedBlocks, static_cast<int>(gb), w.sc, SC_RR);
     if (d->pcg_pair && d->nne == 8) k_pcg_split<<<grid_for(n), kBlock, 0, s>>>(w.p, n, w.pp);
     return check_launch("pcg_begin");
 }
