@@ -1,0 +1,65 @@
+"""A solve whose recursive residual meets the tolerance while the true one lies a rounding above it goes on
+instead of giving up: the tolerance is set just below the true residual at which a solve has stopped. The
+recursion then stops at the same iteration in about half of the cases, with a true residual above tol."""
+
+import numpy as np
+import pytest
+import torch
+
+import goosefem_gb300 as gf
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(elem, n, seed):
+    gf.set_strict(False)
+    rng = np.random.default_rng(seed)
+    m = gf.Mesh.Quad4.Regular(n, n + 3) if elem == "quad4" else gf.Mesh.Hex8.Regular(n, n + 1, n)
+    coor, conn, dofs = m.coor(), m.conn(), m.dofs()
+    nd = coor.shape[1]
+    K, G = rng.uniform(0.5, 1.5, m.nelem()), rng.uniform(0.25, 0.75, m.nelem())
+    top = coor[:, nd - 1].max()
+    lo, hi = np.flatnonzero(coor[:, nd - 1] == 0), np.flatnonzero(coor[:, nd - 1] == top)
+    x = np.zeros(coor.shape)
+    x[hi, nd - 1] = -1e-2 * rng.uniform(0.9, 1.1, hi.size)
+    iip = np.unique(np.concatenate([(lo[:, None] * nd + np.arange(nd)).ravel(), hi * nd + nd - 1]))
+    return m, coor, conn, dofs, K, G, iip, torch.tensor(x, device="cuda")
+
+
+def _stops(solve, x0, tol):
+    """(iterations, true residual) of solve to tol, then to just below that residual."""
+    out = []
+    for _ in range(2):
+        x = x0.clone()
+        it, rel = solve(x, tol)
+        assert rel <= tol and torch.isfinite(x).all()
+        out.append(it)
+        tol = float(np.nextafter(rel, 0.0))
+    assert out[0] <= out[1] <= out[0] + 200
+
+
+@pytest.mark.parametrize("arithmetic", ["fp64", "pair"])
+@pytest.mark.parametrize("elem,n", [("quad4", 30), ("hex8", 12)])
+def test_jacobi_pcg(elem, n, arithmetic):
+    for seed in range(6):
+        _, coor, conn, dofs, K, G, iip, x0 = _problem(elem, n, seed)
+        st = gf.ElasticStatic(coor, conn, dofs, K, G, iip, arithmetic=arithmetic)
+        for tol, every in ((1e-8, 16), (1e-10, 1), (1e-12, 16)):
+            _stops(lambda x, t: st.solve(x, tol=t, check_every=every), x0, tol)
+
+
+def test_out_of_reach_is_refused():
+    """A tolerance below the arithmetic's own: an error, and a finite solution."""
+    from goosefem_gb300 import _lib
+
+    _, coor, conn, dofs, K, G, iip, x0 = _problem("quad4", 20, 0)
+    st = gf.ElasticStatic(coor, conn, dofs, K, G, iip)
+    for tol in (1e-18, 1e-60):
+        x = x0.clone()
+        with pytest.raises(_lib.GFGPUError) as e:
+            st.solve(x, tol=tol)
+        assert e.value.code == -8 and torch.isfinite(x).all()
+    x = x0.clone()
+    with pytest.raises(_lib.GFGPUError) as e:
+        st.solve(x, tol=1e-8, maxiter=20)
+    assert e.value.code == -8
