@@ -20,6 +20,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <limits>
 #include <numeric>
 
 #include "common.cuh"
@@ -2354,63 +2355,75 @@ static int fcg_core(const gfgpu_verlet_desc* d, const double* diag, const gfgpu_
         if (exec) cudaGraphExecDestroy(exec);
         if (cs) cudaStreamDestroy(cs);
     };
-    while (rel > tol && it < maxiter) {
-        bool steady = c >= int64_t(nkeep) + ndir && c % nslots == 0;
-        if (steady && !exec && maxiter - it >= chunk) {
-            rc = check_cuda(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "cudaStreamCreate");
-            if (rc != GFGPU_OK) break;
-            cudaGraph_t graph = nullptr;
-            rc = check_cuda(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "capture");
-            if (rc != GFGPU_OK) break;
-            int crc = GFGPU_OK;
-            for (int64_t k = 0; k < chunk && crc == GFGPU_OK; ++k) crc = iteration(c + k * ndir, k == chunk - 1, cs);
-            cudaError_t e = cudaStreamEndCapture(cs, &graph);
-            if (crc != GFGPU_OK) {
+    // as in gfgpu_pcg_solve: the true residual -(A x)_u decides, and one a little above tol (rounding) takes
+    // the iterations further, from that residual
+    double goal = tol, truth = 0.0, before = std::numeric_limits<double>::infinity();
+    for (;;) {
+        while (rel > goal && it < maxiter) {
+            bool steady = c >= int64_t(nkeep) + ndir && c % nslots == 0;
+            if (steady && !exec && maxiter - it >= chunk) {
+                rc = check_cuda(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking), "cudaStreamCreate");
+                if (rc != GFGPU_OK) break;
+                cudaGraph_t graph = nullptr;
+                rc = check_cuda(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal), "capture");
+                if (rc != GFGPU_OK) break;
+                int crc = GFGPU_OK;
+                for (int64_t k = 0; k < chunk && crc == GFGPU_OK; ++k) crc = iteration(c + k * ndir, k == chunk - 1, cs);
+                cudaError_t e = cudaStreamEndCapture(cs, &graph);
+                if (crc != GFGPU_OK) {
+                    if (graph) cudaGraphDestroy(graph);
+                    rc = crc;
+                    break;
+                }
+                rc = check_cuda(e, "cudaStreamEndCapture");
+                if (rc == GFGPU_OK) rc = check_cuda(cudaGraphInstantiate(&exec, graph, 0), "cudaGraphInstantiate");
                 if (graph) cudaGraphDestroy(graph);
-                rc = crc;
-                break;
+                if (rc != GFGPU_OK) break;
             }
-            rc = check_cuda(e, "cudaStreamEndCapture");
-            if (rc == GFGPU_OK) rc = check_cuda(cudaGraphInstantiate(&exec, graph, 0), "cudaGraphInstantiate");
-            if (graph) cudaGraphDestroy(graph);
-            if (rc != GFGPU_OK) break;
-        }
-        if (exec && maxiter - it >= chunk) {
-            rc = check_cuda(cudaGraphLaunch(exec, s), "cudaGraphLaunch");
-            if (rc != GFGPU_OK) break;
-            it += chunk;
-            c += chunk * ndir;
-        }
-        else {
-            int64_t nb = exec ? maxiter - it : std::min<int64_t>(check_every, maxiter - it);
-            for (int64_t k = 0; k < nb && rc == GFGPU_OK; ++k) {
-                rc = iteration(c, true, s);
-                ++it;
-                c += ndir;
-                if (!exec && c >= int64_t(nkeep) + ndir && c % nslots == 0 && maxiter - it >= chunk) break;
+            if (exec && maxiter - it >= chunk) {
+                rc = check_cuda(cudaGraphLaunch(exec, s), "cudaGraphLaunch");
+                if (rc != GFGPU_OK) break;
+                it += chunk;
+                c += chunk * ndir;
             }
+            else {
+                int64_t nb = exec ? maxiter - it : std::min<int64_t>(check_every, maxiter - it);
+                for (int64_t k = 0; k < nb && rc == GFGPU_OK; ++k) {
+                    rc = iteration(c, true, s);
+                    ++it;
+                    c += ndir;
+                    if (!exec && c >= int64_t(nkeep) + ndir && c % nslots == 0 && maxiter - it >= chunk) break;
+                }
+                if (rc != GFGPU_OK) break;
+            }
+            rc = read_sc();
             if (rc != GFGPU_OK) break;
+            if (!std::isfinite(h[F_RR])) {
+                cleanup();
+                *iters = it;
+                *relres = h[F_RR];
+                return fail(GFGPU_ERR_NAN, "gfgpu_fcg_solve: non-finite residual");
+            }
+            rel = std::sqrt(h[F_RR]) / bnorm;
         }
-        rc = read_sc();
+        if (rc == GFGPU_OK) rc = gfgpu_internal_element_forces(d, x, w.fe, s);
+        if (rc == GFGPU_OK) {
+            k_fres<<<rs.grid, rs.block, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.r,
+                                                w.partial, reg_grid(d));
+            k_fredv<<<1, kWide, 0, s>>>(w.partial, ROW_RR, nr, F_RR, w.sc);
+            rc = read_sc();
+        }
         if (rc != GFGPU_OK) break;
-        if (!std::isfinite(h[F_RR])) {
-            cleanup();
-            *iters = it;
-            *relres = h[F_RR];
-            return fail(GFGPU_ERR_NAN, "gfgpu_fcg_solve: non-finite residual");
-        }
-        rel = std::sqrt(h[F_RR]) / bnorm;
+        truth = std::sqrt(h[F_RR]) / bnorm;
+        if (truth <= tol || it >= maxiter || !(truth < 2.0 * tol && truth < 0.97 * before)) break;
+        before = truth;
+        goal = 0.9 * tol * (rel / truth);
+        rel = truth;
     }
     cleanup();
     GF_TRY(rc);
-    // true residual -(A x)_u
-    GF_TRY(gfgpu_internal_element_forces(d, x, w.fe, s));
-    k_fres<<<rs.grid, rs.block, 0, s>>>(d->dofs, d->csr_ptr, d->csr_idx, d->part, d->nnu, w.fe, rhs, n, w.r,
-                              w.partial, reg_grid(d));
-    k_fredv<<<1, kWide, 0, s>>>(w.partial, ROW_RR, nr, F_RR, w.sc);
-    GF_TRY(read_sc());
     *iters = it;
-    *relres = std::sqrt(h[F_RR]) / bnorm;
+    *relres = truth;
     if (*relres > tol) return fail(GFGPU_ERR_DIVERGED, "gfgpu_fcg_solve: tolerance not reached");
     return GFGPU_OK;
 }

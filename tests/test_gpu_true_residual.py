@@ -63,3 +63,26 @@ def test_out_of_reach_is_refused():
     with pytest.raises(_lib.GFGPUError) as e:
         st.solve(x, tol=1e-8, maxiter=20)
     assert e.value.code == -8
+
+
+@pytest.mark.parametrize("arithmetic", ["fp64", "pair"])
+@pytest.mark.parametrize("coarse", [False, True])
+def test_flexible_cg(coarse, arithmetic):
+    from goosefem_gb300 import learned
+
+    gf.set_strict(False)
+    nx, ny = 60, 50
+    for seed in range(6):
+        rng = np.random.default_rng(seed)
+        K, G = rng.uniform(0.5, 5.0, nx * ny), rng.uniform(0.25, 2.5, nx * ny)
+        bot = np.arange(nx + 1)
+        top = bot + ny * (nx + 1)
+        iip = np.unique(np.concatenate([(bot[:, None] * 2 + np.arange(2)).ravel(), top * 2 + 1]))
+        x = np.zeros((nx + 1) * (ny + 1) * 2)
+        x[top * 2 + 1] = -1e-2
+        lp = learned.LearnedPreconditioner(nx, ny, K, G, iip, seed=seed, arithmetic=arithmetic)
+        if coarse:
+            lp.coarse_setup(12)
+        for tol, nkeep, every in ((1e-8, 1, 8), (1e-11, 2, 4), (1e-11, 1, 1)):
+            _stops(lambda x, t: lp.fcg(x, tol=t, use_nn=False, nkeep=nkeep, coarse=coarse, check_every=every),
+                   torch.tensor(x, device="cuda"), tol)
