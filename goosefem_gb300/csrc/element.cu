@@ -581,9 +581,9 @@ k_int_tensor4(const double* __restrict__ dNx, const double* __restrict__ vol,
 // a value leaves the range, the thread takes the FP64 form on operands in global memory.
 // 9177 Hex8 elements 326 -> 200 us against the FP64 form, 49k Quad4 80 -> 62 us, with a third of its
 // error; the integer multiply-add pipe is 59 % busy (half of it the multiply-adds, the rest the
-// conversions), 2 blocks per SM (registers; Quad4 3, with 2 of them 66 us). Looking at point m first saves
-// forming the exponents of all terms beside the products (Hex8 224 us). The nodal rule, whose gradients
-// hold zeros, looks at all points: 217 us.
+// conversions), 2 blocks per SM (registers; Quad4 3). Looking at point m first saves forming the exponents
+// of all terms beside the products (a call on the Hex8 mesh 208 us, 237 with them). The nodal rule, whose
+// gradients hold zeros, looks at all points: 225 us.
 template <int NNE, int ND>
 struct Tensor4Fix {
     static constexpr int K = NNE * ND, C4 = ND * ND * ND * ND, G = NNE * ND, JK = ND * ND;

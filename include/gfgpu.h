@@ -597,9 +597,10 @@ int gfgpu_elastic_diagonal(const gfgpu_verlet_desc* d, double* diag, void* works
                            gfgpu_stream_t stream);
 /* Solve for the unknown dofs of the nodevec x (prescribed dofs hold the prescribed values and the
  * unknown dofs the initial guess on entry). Stops when ||r|| / ||b|| <= tol (checked every
- * `check_every` iterations on the host), then verifies the true residual b - A x. Synchronises.
- * Returns GFGPU_ERR_DIVERGED when maxiter is reached first. Deterministic: fixed-grid
- * reductions in a fixed order. */
+ * `check_every` iterations on the host), then verifies the true residual b - A x: one that rounding
+ * leaves above tol, but within twice of it, takes the iterations further. Synchronises. Returns
+ * GFGPU_ERR_DIVERGED when maxiter is reached first or tol is below what the arithmetic reaches.
+ * Deterministic: fixed-grid reductions in a fixed order. */
 int gfgpu_pcg_solve(const gfgpu_verlet_desc* d, const double* diag, double* x, double tol,
                     int64_t maxiter, int32_t check_every, void* workspace, gfgpu_stream_t stream,
                     int64_t* iters, double* relres);
