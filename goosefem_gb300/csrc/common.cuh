@@ -207,6 +207,15 @@ __device__ __forceinline__ double gather_dof(int64_t t, const int32_t* __restric
     return f;
 }
 
+// The trace's part lam tr of sigma = lam tr I + 2 G eps, NaN where the trace is infinite, as the form with
+// the deviator has it (an infinite strain less a third of an infinite trace). Tested on the integer pipe.
+__device__ __forceinline__ double trace_stress(double lam, double tr)
+{
+    const double lt = lam * tr;
+    const bool finite = (__double2hiint(tr) & 0x7ff00000) != 0x7ff00000;
+    return __hiloint2double(finite ? __double2hiint(lt) : 0x7ff80000, __double2loint(lt));
+}
+
 inline bool too_big(int64_t n)
 {
     return n < 0 || n > INT32_MAX;

@@ -177,7 +177,7 @@ k_elem_force_general(const int32_t* __restrict__ conn, const double* u,
             double tr = h[0][0];
 #pragma unroll
             for (int i = 1; i < ND; ++i) tr += h[i][i];
-            const double lt = lam * tr;
+            const double lt = trace_stress(lam, tr);
             double s[ND][ND];
 #pragma unroll
             for (int i = 0; i < ND; ++i) {

@@ -821,7 +821,7 @@ __device__ __forceinline__ void stress_point(double (&s)[ND * ND], double lam, d
     double tr = s[0];
 #pragma unroll
     for (int i = 1; i < ND; ++i) tr += s[i * ND + i];
-    const double lt = lam * tr;
+    const double lt = trace_stress(lam, tr);
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
         s[i * ND + i] = fma(g2, s[i * ND + i], lt);
