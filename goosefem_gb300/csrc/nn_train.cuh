@@ -383,32 +383,41 @@ k_wgrad_tile(const float* __restrict__ X, const float* __restrict__ dY, int dil,
         const int rows = min(4, g.H - y0 - 4 * rg);
         const float* xr = xs + cur * xsz + ((4 * rg + dil + dil * (tr - 1)) * hw + pl) * CI + ig;
         const float* gr = gs + cur * gsz + (4 * rg * kTrainTile + pl) * CO + cg;
+        auto pixel = [&](int x) {
+            f2 d[CW / 2];
+            if constexpr (CW == 8) {
+                const ulonglong2 d0 = *reinterpret_cast<const ulonglong2*>(gr + x * CO);
+                const ulonglong2 d1 = *reinterpret_cast<const ulonglong2*>(gr + x * CO + 4);
+                d[0] = d0.x;
+                d[1] = d0.y;
+                d[2] = d1.x;
+                d[3] = d1.y;
+            }
+            else {
+                d[0] = *reinterpret_cast<const f2*>(gr + x * CO);
+            }
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                const float4 q = *reinterpret_cast<const float4*>(xr + (x + dil * t) * CI);
+                const float qa[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const f2 x2 = f2_make(qa[i], qa[i]);
+#pragma unroll
+                    for (int k = 0; k < CW / 2; ++k) acc[t][i][k] = f2_fma_acc(x2, d[k], acc[t][i][k]);
+                }
+            }
+        };
+        // pixels inside the image only: a zero of dY outside times an infinite or NaN neighbour would be NaN
+        const int cols = g.W - x0;
         for (int y = 0; y < rows; ++y, xr += hw * CI, gr += kTrainTile * CO) {
+            if (cols >= kTrainTile) {
 #pragma unroll(PL == 1 ? 16 : 2)
-            for (int x = 0; x < kTrainTile; x += PL) {
-                f2 d[CW / 2];
-                if constexpr (CW == 8) {
-                    const ulonglong2 d0 = *reinterpret_cast<const ulonglong2*>(gr + x * CO);
-                    const ulonglong2 d1 = *reinterpret_cast<const ulonglong2*>(gr + x * CO + 4);
-                    d[0] = d0.x;
-                    d[1] = d0.y;
-                    d[2] = d1.x;
-                    d[3] = d1.y;
-                }
-                else {
-                    d[0] = *reinterpret_cast<const f2*>(gr + x * CO);
-                }
-#pragma unroll
-                for (int t = 0; t < 3; ++t) {
-                    const float4 q = *reinterpret_cast<const float4*>(xr + (x + dil * t) * CI);
-                    const float qa[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const f2 x2 = f2_make(qa[i], qa[i]);
-#pragma unroll
-                        for (int k = 0; k < CW / 2; ++k) acc[t][i][k] = f2_fma_acc(x2, d[k], acc[t][i][k]);
-                    }
-                }
+                for (int x = 0; x < kTrainTile; x += PL) pixel(x);
+            }
+            else {
+#pragma unroll 1
+                for (int x = 0; x < cols - pl; x += PL) pixel(x);
             }
         }
         __syncthreads();

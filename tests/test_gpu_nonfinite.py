@@ -66,3 +66,33 @@ def test_general_element_forces(gf, oracle, nd, dims):
             ref = R.assemble_node(conn, dofs, R.int_grad_n_dot_tensor2_dv(dNx, vol, sig))
         got = to_np(st.force(u))
         assert np.array_equal(np.isnan(got), np.isnan(ref)) and not np.isinf(got).any()
+
+
+@pytest.mark.parametrize("where", [(0, 0, 34), (1, 34, 0), (0, 20, 17), (1, 34, 34), (0, 16, 15), (0, 31, 31)])
+def test_network_gradients(gf, where):
+    """A NaN in a crop whose edge is no multiple of the tiles' 16 pixels. The ReLU after the first layer (a
+    maximum with 0) turns what it makes of it into 0, so NaN is left in the first layer's weight gradient,
+    for the channel and the taps that bring a pixel of the image to it, and nowhere else."""
+    import torch
+    from goosefem_gb300 import _lib
+
+    layers = ((4, 32), (32, 32), (32, 32), (32, 2))
+    rng = np.random.default_rng(1)
+    flat = np.concatenate([a for ci, co in layers for a in (rng.normal(0.0, np.sqrt(2.0 / (9 * ci)), 9 * ci * co),
+                                                           rng.normal(0.0, 0.1, co))]).astype(np.float32)
+    B, S, ch = 2, 35, 1
+    X = rng.normal(size=(B, S, S, 4)).astype(np.float32)
+    T = rng.normal(size=(B, S, S, 2)).astype(np.float32)
+    X[where + (ch,)] = np.nan
+    flat, Xd, Td = (torch.tensor(a, device="cuda") for a in (flat, X, T))
+    ws = torch.empty(int(_lib.lib().gfgpu_nn_train_workspace_bytes(B, S, S)) // 4 + 1, dtype=torch.float32, device="cuda")
+    g, loss = torch.empty_like(flat), torch.empty(1, dtype=torch.float32, device="cuda")
+    wb = flat.to(torch.bfloat16)
+    _lib.call("gfgpu_nn_train_step", wb.data_ptr(), flat.data_ptr(), Xd.data_ptr(), Td.data_ptr(), None, None, B, S,
+              4, g.data_ptr(), loss.data_ptr(), ws.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    want = np.zeros(flat.numel(), dtype=bool)
+    first = want[:9 * 4 * 32].reshape(9, 4, 32)
+    for t in range(9):
+        y, x = where[1] - (t // 3 - 1), where[2] - (t % 3 - 1)
+        first[t, ch] = 0 <= y < S and 0 <= x < S
+    assert np.array_equal(np.isnan(g.cpu().numpy()), want) and bool(torch.isfinite(g[~g.isnan()]).all())
